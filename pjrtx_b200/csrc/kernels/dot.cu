@@ -22,6 +22,7 @@
 #include <cuda_fp16.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstdlib>
 #include <type_traits>
 
@@ -528,7 +529,7 @@ int launch_typed(const DotShape& s, const DotScratch& plan, const void* lhs, con
 
 namespace {
 int umma_eligible(const DotShape& s);
-DotScratch umma_plan(const DotShape* shapes, int count, int sm_count, bool k_major);
+DotScratch umma_plan(const DotShape* shapes, int count, int sm_count, int kind);
 }  // namespace
 
 namespace {
@@ -574,7 +575,7 @@ DotScratch dot_group_plan(const DotShape* shapes, int count, int sm_count, bool 
   if (batch == 1 && allow_tensor) {
     bool all_umma = true;
     for (int g = 0; g < count; g++) all_umma &= umma_eligible(shapes[g]) == 1;
-    if (all_umma) return umma_plan(shapes, count, sm_count, false);
+    if (all_umma) return umma_plan(shapes, count, sm_count, 1);
   }
   if (batch == 1) {
     // Persistent TMA kernel: equal shares of (column tile, row chunk) units per CTA, two CTAs per SM with a ring of
@@ -772,90 +773,128 @@ int umma_eligible(const DotShape& s) {
   return 0;
 }
 
-DotScratch umma_plan(const DotShape* shapes, int count, int sm_count, bool k_major) {
+int umma_source(const DotShape& s) { return s.rhs_s8 ? umma::kBytes : umma::kTile; }
+
+// Clusters of `size` CTAs, `per_sm` CTAs on an SM, that fit the chip at once. A cluster stays inside a GPC, so SMs are left
+// over; the table is what cudaOccupancyMaxActiveClusters answers for one CTA per SM on a B200 (148 SMs).
+int64_t clusters_that_fit(int sm_count, int size, int per_sm) {
+  static const int on_b200[umma::kSplitMax + 1] = {0, 148, 74, 45, 33, 26, 22, 15, 15};
+  return std::max<int64_t>(1, (int64_t)on_b200[size] * per_sm * sm_count / 148);
+}
+
+// CTAs of one launch that share an SM: two with int8 weights, whose units are a chain of copy, conversion and MMA that one
+// CTA cannot keep full. The 16-bit stream runs one (two: twice the partial sums), but in half the shared memory, so that
+// the next launch's CTA moves in, sets up and requests its first weights while this one streams.
+int umma_per_sm(int m_tile, int src) { return src == umma::kBytes && umma::tmem_columns(m_tile, 2, src) <= 256 ? 2 : 1; }
+
+// Shared memory of a CTA: half where the tensor memory of two CTAs fits and the ring still holds four stages or more.
+bool umma_half_possible(int m_tile, int ksplit, bool several_tiles, int src) {
+  const int sub = src == umma::kTile ? 1 : 2, rows = (m_tile + 4 * ksplit - 1) / (4 * ksplit) * 4;
+  return umma::tmem_columns(m_tile, sub, src) <= 256 &&
+         umma::sum_bytes(ksplit, rows, several_tiles ? 2 : 1) + 4 * umma::stage_bytes(m_tile, sub, src) + umma::kBarrierBytes + 1024 <=
+             umma::kSharedSmem;
+}
+
+// Tile height, split of k and ring size with the least modelled time, in nanoseconds. The weights arrive at the HBM rate or
+// at the rate of one CTA, 16 KiB per 250 ns with the whole ring and per 305 ns with half of it (32 x 14336 x 4096 by 32 CTAs:
+// 64 and 79 us, the same for 16 to 128 rows); near the crossing the two add up softly. Tall tiles are bound by shared memory
+// (copies in and the tensor core's reads out, 128 bytes per cycle) or by the MMAs. The half ring saves about 1.5 us of
+// start-up, the cluster's sum costs about 0.6 us. Measured, us per launch in a chain at 32 rows, best against the others:
+// 4096 x 4096 4 CTAs per tile, half ring 15.5 (whole 17.6; 2 CTAs 16.8, 1 CTA 24.0); 14336 x 4096 4, whole 28.6 (half 30.8;
+// 2 CTAs 37.5); 4096 x 28672 1, whole 49.5 (half 53.5; 2 CTAs 52.4); 8192 x 57344 3 155 (2 160, 1 170).
+struct UmmaChoice {
+  double ns = 0;
+  int m_tile = 0, ksplit = 1;
+  bool half = false;
+};
+UmmaChoice umma_choose(const DotShape* shapes, int count, int sm_count, int src) {
+  const DotShape& s = shapes[0];
+  const double weight_unit = umma::weight_stage_bytes(src, 1);
+  const int64_t kblocks = (s.k + 127) / 128 * 2;
+  UmmaChoice best;
+  int64_t n_tiles = 0;
+  for (int g = 0; g < count; g++) n_tiles += (shapes[g].n + 127) / 128;
+  static const int64_t caps[] = {256, 192, 128, 96, 64};
+  for (int64_t cap : caps) {
+    if (src != umma::kTile && cap > 128) continue;
+    const int64_t m_tiles = (s.m + cap - 1) / cap;
+    const int64_t mt = ((s.m + m_tiles - 1) / m_tiles + 15) / 16 * 16;
+    const int64_t tiles = n_tiles * m_tiles;
+    for (int split = 1; split <= umma::kSplitMax; split++) {
+      if (split > 1 && (mt > 128 || split > kblocks / 2)) break;
+      const int64_t clusters = std::min<int64_t>(tiles, clusters_that_fit(sm_count, split, umma_per_sm((int)mt, src)));
+      for (int half = 0; half < 2; half++) {
+        if (half && !umma_half_possible((int)mt, split, tiles > clusters, src)) continue;
+        if (!half && src == umma::kBytes && umma_per_sm((int)mt, src) == 2 && umma_half_possible((int)mt, split, tiles > clusters, src)) continue;
+        const double smem_ns = 2.0 * ((src == umma::kTile ? 16384 : weight_unit) + mt * 128) / 128 / 1.85;
+        const double unit_ns = std::max({smem_ns, 2.0 * mt / 1.85, src == umma::kTile && !half ? 250.0 : 305.0});
+        const double cta_ns = (double)((tiles + clusters - 1) / clusters) * (double)((kblocks + split - 1) / split) * unit_ns;
+        const double hbm_ns = (double)n_tiles * kblocks * weight_unit / 6500.0;
+        const double ns = std::pow(std::pow(cta_ns, 4) + std::pow(hbm_ns, 4), 0.25) + (half ? 0 : 1500) + (split > 1 ? 600 + 8.0 * mt : 0);
+        if (best.ns == 0 || ns < best.ns * 0.99) best = UmmaChoice{ns, (int)mt, split, half != 0};
+      }
+    }
+  }
+  return best;
+}
+
+DotScratch umma_plan(const DotShape* shapes, int count, int sm_count, int kind) {
   DotScratch p;
   const DotShape& s = shapes[0];
-  p.path = k_major ? 4 : 1;
+  const int src = umma_source(s);
+  p.path = kind == 1 ? 1 : 4;
   p.umma = 1;
-  p.m_tile = (int)std::min<int64_t>(256, (s.m + 15) / 16 * 16);
+  const UmmaChoice choice = umma_choose(shapes, count, sm_count, src);
+  p.m_tile = choice.m_tile;
+  p.ksplit = choice.ksplit;
   const int64_t m_tiles = (s.m + p.m_tile - 1) / p.m_tile;
-  // 256-column tiles (two accumulators per tile) are available behind PJRTX_B200_UMMA_WIDE=1; measured on B200 they
-  // stream no faster than 128-column tiles and leave more partial sums to fold, so they are off by default.
-  int64_t tiles128 = 0;
-  for (int g = 0; g < count; g++) tiles128 += (shapes[g].n + 127) / 128 * m_tiles;
-  static const int wide = env_int("PJRTX_B200_UMMA_WIDE", 0);
-  p.nh = (wide && !s.rhs_s8 && p.m_tile <= 128 && tiles128 * ((s.k + 63) / 64) >= 16 * (int64_t)sm_count) ? 2 : 1;
-  const int tw = umma::kTileN * p.nh;
   int64_t tiles = 0;
-  for (int g = 0; g < count; g++) tiles += (shapes[g].n + tw - 1) / tw * m_tiles;
-  // Short activation tiles leave room for two CTAs per SM (half the shared memory each; PJRTX_B200_UMMA_CTAS=2), so
-  // that one CTA streams while the other folds a tile. Measured on B200 at m = 32 it is slower than one CTA per SM with
-  // the whole ring (8B-width layers 1.665 against 1.640 ms per 8 layers; one eighth of the 70B-shape widths 3.00
-  // against 2.79 ms per 20 layers): twice the partial sums to fold outweigh the overlap. Off by default.
-  static const int ctas_wanted = env_int("PJRTX_B200_UMMA_CTAS", 1);
-  const bool w8 = s.rhs_s8 != 0;
-  const int per_sm = (ctas_wanted >= 2 && p.m_tile <= 64 && !w8 && p.nh == 1) ? 2 : 1;
-  const int64_t slots = (int64_t)sm_count * per_sm;
-  // PJRTX_B200_UMMA_SMEM_KB bounds the ring (experiments: a CTA that leaves half of the shared memory free lets the
-  // first CTAs of the next kernel move in and start their weight copies while this one folds its last tile).
-  static const int smem_kb = env_int("PJRTX_B200_UMMA_SMEM_KB", 0);
-  const bool small_ring = smem_kb >= 48 && smem_kb <= 225 && !w8 && p.m_tile <= 64;
-  const size_t smem_budget = small_ring ? (size_t)smem_kb * 1024 - 2048 : per_sm == 2 ? 112 * 1024 - 2048 : 227 * 1024 - 2048;
-  const int64_t grid = std::max<int64_t>(1, std::min<int64_t>(tiles * ((s.k + 63) / 64), slots));
-  // 128-deep stages once every CTA still gets a long run of them; 64-deep otherwise (finer split, better balance), and
-  // whenever the ring would hold fewer than four of the deep ones.
-  p.sub = (p.nh == 1 && tiles * ((s.k + 127) / 128) >= 32 * grid) ? 2 : 1;
-  if (p.sub == 2 && smem_budget / umma::stage_bytes(p.m_tile, 2, p.nh, w8) < 4) p.sub = 1;
-  // Int8 weights: 128-deep stages (PJRTX_B200_W8_SUB=1 gives 64-deep ones: a deeper ring of raw bytes, but twice the
-  // hand-overs between copies, converters and the MMA lane; measured 1.54 against 1.25 ms for the contractions of eight
-  // 8B-width layers and the LM head at 32 rows).
-  static const int w8_sub = env_int("PJRTX_B200_W8_SUB", 2);
-  if (w8) p.sub = w8_sub == 1 ? 1 : 2;
-  const int64_t kblocks = (s.k + 64 * p.sub - 1) / (64 * p.sub);
-  const int64_t units = tiles * kblocks;
-  p.grid = (int)std::max<int64_t>(1, std::min<int64_t>(units, slots));
-  // A split tile costs its f32 partial twice (written, read back): m_tile x 128 x 8 bytes per contributor, against
-  // 128 x k x 2 bytes of weights per tile. Split only while the partials of a tile stay below about half its weights,
-  // or when whole tiles would leave most of the machine idle.
-  const int64_t split_ok = s.k / (8 * (int64_t)p.m_tile);
-  p.whole_tiles = (split_ok < 2 || (p.m_tile >= 128 && 2 * tiles >= sm_count)) ? 1 : 0;
-  if (p.whole_tiles) p.grid = (int)std::max<int64_t>(1, std::min<int64_t>(tiles, slots));
-  p.per_cta = units / p.grid;
-  p.max_contrib = p.whole_tiles ? 1 : (int)((kblocks + p.per_cta - 1) / p.per_cta) + 1;
-  const size_t stage = umma::stage_bytes(p.m_tile, p.sub, p.nh, w8);
-  const size_t ring_budget = smem_budget - (w8 ? umma::kOperandSlots * umma::operand_bytes(p.sub, p.nh) : 0);
-  p.stages = (int)std::max<size_t>(w8 ? umma::kOperandSlots : 2, std::min<size_t>(w8 ? 16 : 12, ring_budget / stage));
-  p.smem = umma::smem_bytes(p.stages, p.m_tile, p.sub, p.nh, w8);
-  p.ksplit = p.max_contrib;
-  p.partial_bytes = (uint64_t)tiles * p.max_contrib * p.m_tile * tw * sizeof(float);
-  p.counter_bytes = (uint64_t)tiles * sizeof(unsigned);
+  for (int g = 0; g < count; g++) tiles += (shapes[g].n + umma::kTileN - 1) / umma::kTileN * m_tiles;
+  const int64_t clusters = std::min<int64_t>(tiles, clusters_that_fit(sm_count, p.ksplit, umma_per_sm(p.m_tile, src)));
+  p.grid = (int)(clusters * p.ksplit);
+  const int rows_per_rank = (p.m_tile + 4 * p.ksplit - 1) / (4 * p.ksplit) * 4;
+  const size_t sum = umma::sum_bytes(p.ksplit, rows_per_rank, tiles > clusters ? 2 : 1);
+  const size_t ring_budget = (choice.half ? umma::kSharedSmem : 227 * 1024) - 1024 - umma::kBarrierBytes - sum;
+  // 128-deep stages once every CTA gets a long run of them (fewer hand-overs); 64-deep otherwise, and whenever the ring
+  // would hold fewer than four of the deep ones. Converted weights always come 128 deep: 64-deep stages double the
+  // hand-overs between copies, converters and the MMA lane (int8, 8B-width layers at 32 rows: 1.54 against 1.25 ms).
+  const int64_t deep_units = (tiles + clusters - 1) / clusters * ((s.k + 127) / 128) / p.ksplit;
+  p.sub = src != umma::kTile || (deep_units >= 16 && ring_budget / umma::stage_bytes(p.m_tile, 2, src) >= 4) ? 2 : 1;
+  p.stages = (int)std::max<size_t>(2, std::min<size_t>(12, ring_budget / umma::stage_bytes(p.m_tile, p.sub, src)));
+  p.smem = umma::smem_bytes(p.stages, p.m_tile, p.sub, src, sum);
   return p;
 }
 
-template <int SUB, int NH, bool W8 = false>
+template <int SUB, int SRC>
 int launch_umma_sub(const umma::Params& prm, const umma::Maps& maps, const DotScratch& plan, bool pdl, cudaStream_t stream) {
-  if (!raise_smem_limit((const void*)umma::umma_stream_kernel<SUB, NH, W8>, 227 * 1024)) return 0;
+  if (!raise_smem_limit((const void*)umma::umma_stream_kernel<SUB, SRC>, 227 * 1024)) return 0;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)plan.grid);
-  cfg.blockDim = dim3(W8 ? umma::kThreadsW8 : umma::kThreads);
+  cfg.blockDim = dim3(umma::threads_of(SRC));
   cfg.dynamicSmemBytes = plan.smem;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[2];
+  cudaLaunchAttribute attr[3];
   cfg.attrs = attr;
   cfg.numAttrs = fill_launch_attributes(attr, pdl);
-  return cudaLaunchKernelEx(&cfg, umma::umma_stream_kernel<SUB, NH, W8>, prm, maps) == cudaSuccess ? 1 : 0;
+  if (plan.ksplit > 1) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    attr[cfg.numAttrs].val.clusterDim.x = (unsigned)plan.ksplit;
+    attr[cfg.numAttrs].val.clusterDim.y = 1;
+    attr[cfg.numAttrs].val.clusterDim.z = 1;
+    cfg.numAttrs++;
+  }
+  return cudaLaunchKernelEx(&cfg, umma::umma_stream_kernel<SUB, SRC>, prm, maps) == cudaSuccess ? 1 : 0;
 }
 
 int launch_umma(const DotShape* shapes, int count, const DotScratch& plan, const void* lhs, const void* const* rhs, void* const* out,
-                void* partials, void* counters, int* error_flag, bool early_rhs, bool pdl, cudaStream_t stream,
-                const void* const* scales) {
+                int* error_flag, bool early_rhs, bool pdl, cudaStream_t stream, const void* const* scales) {
   const DotShape& s = shapes[0];
   const bool w8 = s.rhs_s8 != 0;
-  if (w8 && (!scales || plan.path == 4 || plan.nh != 1)) return 0;
+  if (w8 && (!scales || plan.path == 4)) return 0;
   EncodeTiledFn enc = encode_tiled();
   if (!enc) return 0;
   const bool k_major = plan.path == 4;
-  const int tw = umma::kTileN * plan.nh;
+  const int tw = umma::kTileN;
   umma::Params p{};
   umma::Maps maps{};
   p.m = (int)s.m;
@@ -867,8 +906,7 @@ int launch_umma(const DotShape* shapes, int count, const DotScratch& plan, const
   const cuuint32_t estr[2] = {1, 1};
   // One 3-d copy per stage when every rhs is made of whole 64-column blocks (a ragged last block would make the
   // view read past the end of the last row).
-  static const int allow_3d = env_int("PJRTX_B200_UMMA_3D", 1);
-  bool use_3d = allow_3d && !k_major && !w8;
+  bool use_3d = !k_major && !w8;
   for (int g = 0; g < count; g++) use_3d &= shapes[g].n % 64 == 0;
   int tiles = 0;
   for (int g = 0; g < count; g++) {
@@ -887,7 +925,8 @@ int launch_umma(const DotShape* shapes, int count, const DotScratch& plan, const
       const cuuint32_t estr3[3] = {1, 1, 1};
       int rank = 2;
       if (w8) {
-        // raw bytes: one box of 128 columns x 64 * SUB rows per stage, no swizzle (the converters place the values)
+        // raw bytes: one box of 128 columns x 64 * SUB rows per stage, swizzled so that the converters' reads of four
+        // columns x one row per thread spread over all banks
         gdim[0] = (cuuint64_t)shapes[g].n; gdim[1] = (cuuint64_t)s.k;
         gstride[0] = (cuuint64_t)shapes[g].rhs_k;
         box[0] = 128; box[1] = (cuuint32_t)(64 * plan.sub);
@@ -895,7 +934,7 @@ int launch_umma(const DotShape* shapes, int count, const DotScratch& plan, const
         // every row and usually lose them again before that tile's turn (measured on the 4096 x 128256 LM head:
         // 742 MB read for 525 MB of weights).
         if (enc(&maps.rhs[g], CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(rhs[g]), gdim, gstride, box, estr3,
-                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
           return false;
         continue;
@@ -904,7 +943,7 @@ int launch_umma(const DotShape* shapes, int count, const DotScratch& plan, const
         rank = 3;
         gdim[0] = 64; gdim[1] = (cuuint64_t)s.k; gdim[2] = (cuuint64_t)shapes[g].n / 64;
         gstride[0] = (cuuint64_t)shapes[g].rhs_k * 2; gstride[1] = 128;
-        box[0] = 64; box[1] = (cuuint32_t)(64 * plan.sub); box[2] = (cuuint32_t)(2 * plan.nh);
+        box[0] = 64; box[1] = (cuuint32_t)(64 * plan.sub); box[2] = 2;
       } else if (k_major) {
         gdim[0] = (cuuint64_t)s.k; gdim[1] = (cuuint64_t)shapes[g].n;
         gstride[0] = (cuuint64_t)shapes[g].rhs_n * 2;
@@ -936,21 +975,20 @@ int launch_umma(const DotShape* shapes, int count, const DotScratch& plan, const
       return 0;
   }
   p.kblocks = (int)((s.k + 64 * plan.sub - 1) / (64 * plan.sub));
-  p.units = (long long)tiles * p.kblocks;
-  p.max_contrib = plan.max_contrib;
-  p.partials = static_cast<float*>(partials);
-  p.counters = static_cast<unsigned*>(counters);
+  p.tiles = tiles;
+  p.ksplit = plan.ksplit;
+  p.rows_per_rank = (plan.m_tile + 4 * plan.ksplit - 1) / (4 * plan.ksplit) * 4;
+  p.sum_buffers = tiles > plan.grid / plan.ksplit ? 2 : 1;
   p.error_flag = error_flag;
   p.stages = plan.stages;
   p.is_bf16 = s.dtype == kBF16;
   p.rhs_k_major = k_major ? 1 : 0;
   p.early_rhs = early_rhs ? 1 : 0;
-  p.whole_tiles = plan.whole_tiles;
-  if (w8)
-    return plan.sub == 2 ? launch_umma_sub<2, 1, true>(p, maps, plan, pdl, stream) : launch_umma_sub<1, 1, true>(p, maps, plan, pdl, stream);
-  if (plan.nh == 2)
-    return plan.sub == 2 ? launch_umma_sub<2, 2>(p, maps, plan, pdl, stream) : launch_umma_sub<1, 2>(p, maps, plan, pdl, stream);
-  return plan.sub == 2 ? launch_umma_sub<2, 1>(p, maps, plan, pdl, stream) : launch_umma_sub<1, 1>(p, maps, plan, pdl, stream);
+  switch (umma_source(s)) {
+    case umma::kBytes: return launch_umma_sub<2, umma::kBytes>(p, maps, plan, pdl, stream);
+    default:
+      return plan.sub == 2 ? launch_umma_sub<2, umma::kTile>(p, maps, plan, pdl, stream) : launch_umma_sub<1, umma::kTile>(p, maps, plan, pdl, stream);
+  }
 }
 
 }  // namespace
@@ -1047,7 +1085,7 @@ int dot_group_launch(const DotShape* shapes, int count, const DotScratch& plan, 
                      void* const* out, void* partials, void* counters, int* error_flag, bool early_rhs, bool pdl,
                      cudaStream_t stream, const void* const* scales) {
   if (count < 1 || count > kDotGroupMax) return 0;
-  if (plan.umma) return launch_umma(shapes, count, plan, lhs, rhs, out, partials, counters, error_flag, early_rhs, pdl, stream, scales);
+  if (plan.umma) return launch_umma(shapes, count, plan, lhs, rhs, out, error_flag, early_rhs, pdl, stream, scales);
   if (shapes[0].rhs_s8) return 0;  // int8 weights run on the tensor-core stream only
   if (plan.tma) {
     switch (shapes[0].dtype) {
@@ -1074,8 +1112,7 @@ DotScratch dot_plan(const DotShape& s, int sm_count) {
   auto aligned = [&](int64_t stride) { return stride % V == 0; };
   const bool batches_fit = batch <= 65535;
   const int tensor = umma_eligible(s);
-  if (tensor == 1) return umma_plan(&s, 1, sm_count, false);
-  if (tensor == 2) return umma_plan(&s, 1, sm_count, true);
+  if (tensor) return umma_plan(&s, 1, sm_count, tensor);
   if (s.m <= 8 && s.rhs_n == 1 && s.n % V == 0 && aligned(s.rhs_k) && aligned(s.rhs_b0) && aligned(s.rhs_b1) &&
       batches_fit && s.k >= 1) {
     p.path = 1;

@@ -492,3 +492,36 @@ def test_int8_dequantising_contraction(gpu_backend, m, k, n, dtype):
     ulp = 2.0 ** (-8 if dtype == P.BF16_CODE else -11)
     bound = (1.01 if n % 16 == 0 else 3.0) * ulp * np.max(np.abs(want))
     assert np.max(np.abs(got - want)) <= bound, (np.max(np.abs(got - want)), np.max(np.abs(want)))
+
+
+@pytest.mark.parametrize("dtype", [P.BF16_CODE, P.F16])
+@pytest.mark.parametrize("m,k,n,count", [
+    (3, 128, 128, 1),      # one tile, two 64-deep blocks
+    (16, 2048, 2048, 1),   # several CTAs of a cluster per tile: their sum goes through distributed shared memory
+    (5, 4096, 200, 1),     # few tiles, the largest split, rows that are no multiple of four
+    (32, 1000, 2056, 3),   # ragged k and n, three contractions sharing one launch
+    (33, 512, 8192, 1),    # several tiles per cluster
+    (100, 2048, 512, 1),   # a split tile of more than 64 rows
+])
+def test_cluster_split_contractions_against_f64(gpu_backend, dtype, m, k, n, count):
+    """16-bit contractions whose k is shared by a thread-block cluster. Error: the f32 sums (2^-24 of the summed magnitudes
+    per addition, at most k of them) and one rounding of the output (half a unit in the last place); run-to-run identical."""
+    rng = np.random.default_rng(m * 7919 + n)
+    dt = P.np_dtype(dtype)
+    x = rng.standard_normal((m, k), dtype=np.float32).astype(dt)
+    ws = [rng.standard_normal((k, n + 64 * g), dtype=np.float32).astype(dt) for g in range(count)]
+    b = PlanBuilder()
+    px = b.parameter(dtype, x.shape)
+    b.set_outputs([b.dot_general(px, b.parameter(dtype, w.shape), [1], [0]) for w in ws])
+    exe = gpu_backend.compile_executable(b, [0])
+    steps = [s for s in exe.describe()["kernel_plan"]["steps"] if s["type"] == "dot"]
+    assert len(steps) == 1 and steps[0]["umma"] == 1 and steps[0]["group"] == count, steps
+    got = run_backend(gpu_backend, b, [x] + ws, exe=exe)
+    again = run_backend(gpu_backend, b, [x] + ws, exe=exe)
+    exe.destroy()
+    ulp = 2.0 ** (-9 if dtype == P.BF16_CODE else -12)
+    for g, a, w in zip(got, again, ws):
+        assert np.array_equal(g.view(np.uint16), a.view(np.uint16))
+        want = x.astype(np.float64) @ w.astype(np.float64)
+        mag = np.abs(x.astype(np.float64)) @ np.abs(w.astype(np.float64))
+        assert np.all(np.abs(g.astype(np.float64) - want) <= 2 * ulp * np.abs(want) + k * 2.0 ** -24 * mag + 2.0 ** -24)
