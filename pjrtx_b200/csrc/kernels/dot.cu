@@ -758,22 +758,31 @@ int env_int(const char* name, int fallback) {
   return v && *v ? atoi(v) : fallback;
 }
 
-// 0: not eligible, 1: rhs[K,N] with N contiguous, 2: rhs[N,K] with K contiguous. The tensor maps need 16-byte
-// multiples for every row stride; lhs must be k-contiguous.
+// 0: not eligible, 1: rhs[K,N] with N contiguous, 2: rhs[N,K] with K contiguous, 3: rhs[K,N] with N contiguous whose rows
+// the tensor maps cannot describe. Tensor maps need 16-byte multiples for every row stride; lhs must be k-contiguous.
+// Case 3 (odd vocabularies) has no lower bound on m: the alternative is one thread per output (path 0) or 64 x 64 tiles on
+// the CUDA cores (path 3). Measured, 5 x 2048 x 32001 f16: 739 us on path 0. Below 64 columns or a k of 64 a tile would be
+// mostly padding and the other paths stay.
 int umma_eligible(const DotShape& s) {
   static const int enabled = env_int("PJRTX_B200_UMMA", 1);
   static const int min_m = env_int("PJRTX_B200_UMMA_MIN_M", 3);
   if (!enabled || (s.dtype != kF16 && s.dtype != kBF16)) return 0;
-  if (s.b0 * s.b1 != 1 || s.m < min_m || s.k < 1 || s.n < 1) return 0;
+  if (s.b0 * s.b1 != 1 || s.m < 1 || s.k < 1 || s.n < 1) return 0;
   if (s.lhs_k != 1 || (s.m > 1 && s.lhs_m % 8 != 0)) return 0;
   if (s.m > (1 << 20) || s.n > (1ll << 30) || s.k > (1ll << 30)) return 0;
-  if (s.rhs_s8) return s.rhs_n == 1 && s.rhs_k % 16 == 0 && s.rhs_k >= s.n ? 1 : 0;  // byte rows: 16-byte pitch
-  if (s.rhs_n == 1 && s.rhs_k % 8 == 0 && s.rhs_k >= s.n) return 1;
+  const bool pitch_ok = s.rhs_s8 ? s.rhs_k % 16 == 0 : s.rhs_k % 8 == 0;
+  if (s.rhs_n == 1 && s.rhs_k >= s.n) {
+    if (pitch_ok) return s.m >= min_m ? 1 : 0;
+    return s.n >= 64 && s.k >= 64 && !s.rhs_s8 ? 3 : 0;
+  }
+  if (s.rhs_s8 || s.m < min_m) return 0;
   if (s.rhs_k == 1 && s.rhs_n % 8 == 0 && s.rhs_n >= s.k) return 2;
   return 0;
 }
 
-int umma_source(const DotShape& s) { return s.rhs_s8 ? umma::kBytes : umma::kTile; }
+int umma_source(const DotShape& s, bool loose) {
+  return s.rhs_s8 ? umma::kBytes : loose ? umma::kLoose : umma::kTile;
+}
 
 // Clusters of `size` CTAs, `per_sm` CTAs on an SM, that fit the chip at once. A cluster stays inside a GPC, so SMs are left
 // over; the table is what cudaOccupancyMaxActiveClusters answers for one CTA per SM on a B200 (148 SMs).
@@ -790,7 +799,7 @@ int umma_per_sm(int m_tile, int src) { return src == umma::kBytes && umma::tmem_
 // Shared memory of a CTA: half where the tensor memory of two CTAs fits and the ring still holds four stages or more.
 bool umma_half_possible(int m_tile, int ksplit, bool several_tiles, int src) {
   const int sub = src == umma::kTile ? 1 : 2, rows = (m_tile + 4 * ksplit - 1) / (4 * ksplit) * 4;
-  return umma::tmem_columns(m_tile, sub, src) <= 256 &&
+  return src != umma::kLoose && umma::tmem_columns(m_tile, sub, src) <= 256 &&
          umma::sum_bytes(ksplit, rows, several_tiles ? 2 : 1) + 4 * umma::stage_bytes(m_tile, sub, src) + umma::kBarrierBytes + 1024 <=
              umma::kSharedSmem;
 }
@@ -809,7 +818,7 @@ struct UmmaChoice {
 };
 UmmaChoice umma_choose(const DotShape* shapes, int count, int sm_count, int src) {
   const DotShape& s = shapes[0];
-  const double weight_unit = umma::weight_stage_bytes(src, 1);
+  const double weight_unit = umma::weight_stage_bytes(src == umma::kLoose ? umma::kTile : src, 1);
   const int64_t kblocks = (s.k + 127) / 128 * 2;
   UmmaChoice best;
   int64_t n_tiles = 0;
@@ -841,8 +850,8 @@ UmmaChoice umma_choose(const DotShape* shapes, int count, int sm_count, int src)
 DotScratch umma_plan(const DotShape* shapes, int count, int sm_count, int kind) {
   DotScratch p;
   const DotShape& s = shapes[0];
-  const int src = umma_source(s);
-  p.path = kind == 1 ? 1 : 4;
+  const int src = umma_source(s, kind == 3);
+  p.path = kind == 1 ? 1 : kind == 2 ? 4 : 5;
   p.umma = 1;
   const UmmaChoice choice = umma_choose(shapes, count, sm_count, src);
   p.m_tile = choice.m_tile;
@@ -889,7 +898,7 @@ int launch_umma_sub(const umma::Params& prm, const umma::Maps& maps, const DotSc
 int launch_umma(const DotShape* shapes, int count, const DotScratch& plan, const void* lhs, const void* const* rhs, void* const* out,
                 int* error_flag, bool early_rhs, bool pdl, cudaStream_t stream, const void* const* scales) {
   const DotShape& s = shapes[0];
-  const bool w8 = s.rhs_s8 != 0;
+  const bool w8 = s.rhs_s8 != 0, loose = plan.path == 5;
   if (w8 && (!scales || plan.path == 4)) return 0;
   EncodeTiledFn enc = encode_tiled();
   if (!enc) return 0;
@@ -906,11 +915,13 @@ int launch_umma(const DotShape* shapes, int count, const DotScratch& plan, const
   const cuuint32_t estr[2] = {1, 1};
   // One 3-d copy per stage when every rhs is made of whole 64-column blocks (a ragged last block would make the
   // view read past the end of the last row).
-  bool use_3d = !k_major && !w8;
+  bool use_3d = !k_major && !w8 && !loose;
   for (int g = 0; g < count; g++) use_3d &= shapes[g].n % 64 == 0;
   int tiles = 0;
   for (int g = 0; g < count; g++) {
-    if ((reinterpret_cast<uintptr_t>(rhs[g]) & 15) != 0) return 0;
+    if (!loose && (reinterpret_cast<uintptr_t>(rhs[g]) & 15) != 0) return 0;
+    p.rhs[g] = rhs[g];
+    p.rhs_pitch[g] = shapes[g].rhs_k;
     p.tile_begin[g] = tiles;
     tiles += (int)((shapes[g].n + tw - 1) / tw) * p.m_tiles;
     p.out[g] = out[g];
@@ -960,7 +971,7 @@ int launch_umma(const DotShape* shapes, int count, const DotScratch& plan, const
     return true;
   };
   if (use_3d && !encode_rhs(true)) use_3d = false;  // the driver refused the view: fall back to two boxes per half
-  if (!use_3d && !encode_rhs(false)) return 0;
+  if (!use_3d && !loose && !encode_rhs(false)) return 0;
   p.rhs_3d = use_3d ? 1 : 0;
   for (int g = count; g <= umma::kGroupMax; g++) p.tile_begin[g] = tiles;
   for (int g = count; g < umma::kGroupMax; g++) maps.rhs[g] = maps.rhs[0];
@@ -984,8 +995,9 @@ int launch_umma(const DotShape* shapes, int count, const DotScratch& plan, const
   p.is_bf16 = s.dtype == kBF16;
   p.rhs_k_major = k_major ? 1 : 0;
   p.early_rhs = early_rhs ? 1 : 0;
-  switch (umma_source(s)) {
+  switch (umma_source(s, loose)) {
     case umma::kBytes: return launch_umma_sub<2, umma::kBytes>(p, maps, plan, pdl, stream);
+    case umma::kLoose: return launch_umma_sub<2, umma::kLoose>(p, maps, plan, pdl, stream);
     default:
       return plan.sub == 2 ? launch_umma_sub<2, umma::kTile>(p, maps, plan, pdl, stream) : launch_umma_sub<1, umma::kTile>(p, maps, plan, pdl, stream);
   }

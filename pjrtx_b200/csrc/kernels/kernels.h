@@ -89,12 +89,12 @@ struct DotScratch {
   uint64_t counter_bytes = 0;
   int ksplit = 1;
   // 0 generic, 1 streaming rhs[K,N] (N contiguous), 2 streaming rhs[N,K] (K contiguous), 3 f32 tile,
-  // 4 tensor-core stream with rhs[N,K] (K contiguous)
+  // 4 tensor-core stream with rhs[N,K] (K contiguous), 5 tensor-core stream with rhs[K,N] rows TMA cannot describe
   int path = 0;
   // Path 1 without batch axes runs the TMA-fed persistent kernel (stream-K decomposition).
   int tma = 0;
-  // Paths 1 and 4 for 16-bit floats without batch axes can run on the tensor cores (tcgen05, accumulator in TMEM).
-  // `ksplit` CTAs of a cluster then share a tile of 128 columns x m_tile rows, contracting 1/ksplit of k each;
+  // Paths 1 and 4 for 16-bit floats without batch axes can run on the tensor cores (tcgen05, accumulator in TMEM); path 5
+  // always does. `ksplit` CTAs of a cluster then share a tile of 128 columns x m_tile rows, contracting 1/ksplit of k each;
   // nothing goes through scratch memory.
   int umma = 0, m_tile = 0, sub = 1;
   int grid = 0, stages = 0, max_contrib = 0;

@@ -45,6 +45,8 @@
 //            the written program stays finite here.
 //            Converting into shared memory instead moved 110 KB through it per 128-deep stage (1630 cycles on the
 //            4096 x 128256 LM head, where HBM needs 715); through TMEM it is 36 KB.
+//   kLoose   16-bit weights of any pitch and alignment (an odd vocabulary, say): converter warps read them with plain
+//            loads, one column per thread, and write them to TMEM. TMA cannot describe such rows.
 //
 // Programmatic dependent launch: weights are never written by earlier work of the stream (`early_rhs`), so their
 // copies for the first ring of stages are issued before griddepcontrol.wait; activation copies and all stores wait.
@@ -73,9 +75,10 @@ constexpr int kSplitMax = 8;         // CTAs of a cluster (the portable limit)
 constexpr int kBaseThreads = 192;    // warps 0-3 epilogue, warp 4 TMA producer, warp 5 MMA issuer
 constexpr unsigned long long kTimeoutNs = 2000000000ull;  // budget of one launch for all of its waits
 
-enum Source { kTile = 0, kBytes = 1 };
-// Converter warps (from warp 6 on): two per quarter of the 128 columns.
-__host__ __device__ constexpr int converter_warps(int src) { return src == kTile ? 0 : 8; }
+enum Source { kTile = 0, kBytes = 1, kLoose = 2 };
+// Converter warps (from warp 6 on): four per quarter of the 128 columns where the loads come from global memory (the
+// bytes in flight are theirs), two where TMA brings the bytes.
+__host__ __device__ constexpr int converter_warps(int src) { return src == kTile ? 0 : src == kBytes ? 8 : 16; }
 __host__ __device__ constexpr int threads_of(int src) { return kBaseThreads + 32 * converter_warps(src); }
 // Weight operand tiles in TMEM (sources other than kTile), 32 * SUB columns each.
 constexpr int kOperandSlots = 3;
@@ -101,6 +104,8 @@ struct Params {
   int rhs_3d;            // rhs [k, n] with n % 64 == 0: one copy per stage through a 3-d view {64 n, k, n / 64}
   int early_rhs;         // rhs copies may start before the preceding kernel of the stream has finished
   const void* scale[kGroupMax];  // int8: f16 scale per weight column
+  const void* rhs[kGroupMax];    // kLoose
+  long long rhs_pitch[kGroupMax];
 };
 
 struct Maps {
@@ -268,9 +273,9 @@ __device__ __forceinline__ bool cluster_wait(uint64_t* bar, unsigned parity, con
   }
 }
 
-// A stage of the ring: the weight tile (16-bit and swizzled, or raw bytes) and the activation tile behind it.
+// A stage of the ring: the weight tile (16-bit and swizzled, or raw bytes, or nothing) and the activation tile behind it.
 __host__ __device__ constexpr uint32_t weight_stage_bytes(int src, int sub) {
-  return src == kTile ? (uint32_t)sub * 16384u : (uint32_t)sub * 8192u;
+  return src == kTile ? (uint32_t)sub * 16384u : src == kBytes ? (uint32_t)sub * 8192u : 0u;
 }
 __host__ __device__ inline size_t stage_bytes(int m_tile, int sub, int src) {
   return (size_t)sub * m_tile * 128 + weight_stage_bytes(src, sub);
@@ -338,6 +343,14 @@ __device__ __forceinline__ void widen_bytes(uint32_t word, int is_bf16, uint32_t
   }
 }
 
+// Sixteen registers per thread: 32 lanes (one per thread) x 16 columns.
+__device__ __forceinline__ void tmem_store_rows(uint32_t addr, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(addr),
+      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]),
+      "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+      : "memory");
+}
 // Four 16-lane x 8-column blocks next to each other: of every four registers, 0 and 1 go to lane t/4, columns 2*(t%4) and
 // + 1; 2 and 3 to lane t/4 + 8.
 __device__ __forceinline__ void tmem_store_blocks(uint32_t addr, const uint32_t (&r)[16]) {
@@ -350,7 +363,7 @@ __device__ __forceinline__ void tmem_store_blocks(uint32_t addr, const uint32_t 
 
 // SUB: 64-deep k sub-blocks per stage (1 or 2; the sources other than kTile use 2).
 template <int SUB, int SRC>
-__global__ void __launch_bounds__(threads_of(SRC), 2) umma_stream_kernel(const Params p, const __grid_constant__ Maps maps) {
+__global__ void __launch_bounds__(threads_of(SRC), SRC == kLoose ? 1 : 2) umma_stream_kernel(const Params p, const __grid_constant__ Maps maps) {
   extern __shared__ unsigned char smem_dyn[];
   // 128-byte swizzled tiles need 1024-byte aligned bases.
   const uint32_t base = (smem_u32(smem_dyn) + 1023u) & ~1023u;
@@ -380,7 +393,7 @@ __global__ void __launch_bounds__(threads_of(SRC), 2) umma_stream_kernel(const P
   const uint32_t tmem_cols = tmem_columns(p.m_tile, SUB, SRC);
 
   if (threadIdx.x == 4 * 32) {
-    for (int g = 0; g < p.count; g++) asm volatile("prefetch.tensormap [%0];" ::"l"(&maps.rhs[g]) : "memory");
+    for (int g = 0; g < p.count && (SRC == kTile || SRC == kBytes); g++) asm volatile("prefetch.tensormap [%0];" ::"l"(&maps.rhs[g]) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&maps.lhs) : "memory");
     for (int s = 0; s < p.stages; s++) {
       mbar_init(&full[s], 1);
@@ -610,6 +623,46 @@ __global__ void __launch_bounds__(threads_of(SRC), 2) umma_stream_kernel(const P
           stage = 0;
           phase ^= 1;
         }
+      }
+    } else if constexpr (SRC == kLoose) {
+      // One column per thread, 16 * SUB rows per unit; the next unit's loads are in flight while this one is converted.
+      constexpr int R = 16 * SUB;
+      if (!p.early_rhs) asm volatile("griddepcontrol.wait;" ::: "memory");
+      int tile = cluster, kb = kb_begin;
+      Tile t = locate_tile(p, min(tile, p.tiles - 1));
+      unsigned short next[R];
+      auto request = [&]() {
+        const long long n = (long long)t.n_tile * kTileN + quarter * 32 + lane;
+        const int k0 = kb * kDepth + part * R;
+        const long long pitch = p.rhs_pitch[t.group];
+        const unsigned short* src = static_cast<const unsigned short*>(p.rhs[t.group]) + (long long)k0 * pitch + n;
+        const bool in = n < p.n[t.group];
+        const int rows = p.k - k0;
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+          next[r] = (in && r < rows) ? __ldg(src) : (unsigned short)0;
+          src += pitch;
+        }
+        if (++kb == kb_end) {
+          kb = kb_begin;
+          tile += clusters;
+          if (tile < p.tiles) t = locate_tile(p, tile);
+        }
+      };
+      if (count > 0) request();
+      for (int i = 0; i < count; i++) {
+        uint32_t packed[R / 2];
+#pragma unroll
+        for (int r = 0; r < R / 2; r++) packed[r] = (uint32_t)next[2 * r] | (uint32_t)next[2 * r + 1] << 16;
+        if (i + 1 < count) request();
+        const bool ok = slot_free(i);
+        if (!__all_sync(0xffffffffu, ok)) {
+          if (lane == 0) atomicExch(p.error_flag, 15);
+          break;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        tmem_store_rows(operand_base + quarter_addr + (uint32_t)(slot * 32 * SUB + part * (R / 2)), packed);
+        publish();
       }
     }
   } else if (warp < 4) {

@@ -525,3 +525,32 @@ def test_cluster_split_contractions_against_f64(gpu_backend, dtype, m, k, n, cou
         want = x.astype(np.float64) @ w.astype(np.float64)
         mag = np.abs(x.astype(np.float64)) @ np.abs(w.astype(np.float64))
         assert np.all(np.abs(g.astype(np.float64) - want) <= 2 * ulp * np.abs(want) + k * 2.0 ** -24 * mag + 2.0 ** -24)
+
+
+@pytest.mark.parametrize("dtype", [P.BF16_CODE, P.F16])
+@pytest.mark.parametrize("m,k,n", [
+    (1, 64, 65),        # the smallest the path takes: half a unit, one column past half a tile
+    (2, 136, 333),      # rows that stop inside a unit
+    (5, 2048, 1001),    # several CTAs of a cluster per tile
+    (40, 264, 4099),    # several tiles per cluster
+    (130, 128, 257),    # two tiles of rows
+])
+def test_contractions_with_unaligned_weight_rows_against_f64(gpu_backend, dtype, m, k, n):
+    """Weight rows of an odd pitch (an odd vocabulary), which tensor maps cannot describe. Same error bound as the aligned
+    rows: f32 sums and one rounding of the output."""
+    rng = np.random.default_rng(m * 31 + n)
+    dt = P.np_dtype(dtype)
+    x = rng.standard_normal((m, k), dtype=np.float32).astype(dt)
+    w = rng.standard_normal((k, n), dtype=np.float32).astype(dt)
+    b = PlanBuilder()
+    b.set_outputs([b.dot_general(b.parameter(dtype, x.shape), b.parameter(dtype, w.shape), [1], [0])])
+    exe = gpu_backend.compile_executable(b, [0])
+    steps = [s for s in exe.describe()["kernel_plan"]["steps"] if s["type"] == "dot"]
+    assert len(steps) == 1 and steps[0]["umma"] == 1 and steps[0]["path"] == 5, steps
+    got, again = (run_backend(gpu_backend, b, [x, w], exe=exe)[0] for _ in range(2))
+    exe.destroy()
+    assert np.array_equal(got.view(np.uint16), again.view(np.uint16))
+    want = x.astype(np.float64) @ w.astype(np.float64)
+    mag = np.abs(x.astype(np.float64)) @ np.abs(w.astype(np.float64))
+    ulp = 2.0 ** (-9 if dtype == P.BF16_CODE else -12)
+    assert np.all(np.abs(got.astype(np.float64) - want) <= 2 * ulp * np.abs(want) + k * 2.0 ** -24 * mag + 2.0 ** -24)
