@@ -30,6 +30,7 @@
 #include "kernels.h"
 #include "stream_tma.cuh"
 #include "umma_gemm.cuh"
+#include "umma_pair.cuh"
 
 namespace pjrtx {
 
@@ -847,6 +848,28 @@ UmmaChoice umma_choose(const DotShape* shapes, int count, int sm_count, int src)
   return best;
 }
 
+// The same model for CTA pairs (umma_pair.cuh): MMAs, copies at 110 bytes per ns and SM, weights as above.
+double umma_pair_choose(const DotShape* shapes, int count, int sm_count, int* m_tile) {
+  const DotShape& s = shapes[0];
+  const int64_t kblocks = (s.k + 63) / 64;
+  int64_t n_tiles = 0;
+  for (int g = 0; g < count; g++) n_tiles += (shapes[g].n + umma::kPairN - 1) / umma::kPairN;
+  double best = 0;
+  for (int64_t cap = 256; cap >= 64; cap -= 32) {
+    const int64_t m_tiles = (s.m + cap - 1) / cap;
+    const int64_t mt = ((s.m + m_tiles - 1) / m_tiles + 31) / 32 * 32;
+    const int64_t pairs = std::min<int64_t>(n_tiles * m_tiles, sm_count / 2);
+    const double unit_ns = std::max({2.0 * mt / 1.85, (16384.0 + mt * 64) / 110, 250.0});
+    const double cta_ns = (double)((n_tiles * m_tiles + pairs - 1) / pairs) * kblocks * unit_ns;
+    const double t = std::max(cta_ns, (double)n_tiles * umma::kPairN * s.k * 2 / 6500.0);
+    if (best == 0 || t < best * 0.98) {
+      best = t;
+      *m_tile = (int)mt;
+    }
+  }
+  return best;
+}
+
 DotScratch umma_plan(const DotShape* shapes, int count, int sm_count, int kind) {
   DotScratch p;
   const DotShape& s = shapes[0];
@@ -856,6 +879,18 @@ DotScratch umma_plan(const DotShape* shapes, int count, int sm_count, int kind) 
   const UmmaChoice choice = umma_choose(shapes, count, sm_count, src);
   p.m_tile = choice.m_tile;
   p.ksplit = choice.ksplit;
+  int pair_tile = 0;
+  if (src == umma::kTile && s.m > 64 && umma_pair_choose(shapes, count, sm_count, &pair_tile) < choice.ns) {
+    int64_t tiles = 0;
+    for (int g = 0; g < count; g++) tiles += (shapes[g].n + umma::kPairN - 1) / umma::kPairN * ((s.m + pair_tile - 1) / pair_tile);
+    p.pair = 1;
+    p.m_tile = pair_tile;
+    p.ksplit = 1;
+    p.grid = 2 * (int)std::min<int64_t>(tiles, sm_count / 2);
+    p.stages = (int)std::min<size_t>(12, (227 * 1024 - 1024 - umma::kBarrierBytes) / umma::pair_stage_bytes(pair_tile));
+    p.smem = umma::pair_smem_bytes(p.stages, pair_tile);
+    return p;
+  }
   const int64_t m_tiles = (s.m + p.m_tile - 1) / p.m_tile;
   int64_t tiles = 0;
   for (int g = 0; g < count; g++) tiles += (shapes[g].n + umma::kTileN - 1) / umma::kTileN * m_tiles;
@@ -893,6 +928,24 @@ int launch_umma_sub(const umma::Params& prm, const umma::Maps& maps, const DotSc
     cfg.numAttrs++;
   }
   return cudaLaunchKernelEx(&cfg, umma::umma_stream_kernel<SUB, SRC>, prm, maps) == cudaSuccess ? 1 : 0;
+}
+
+int launch_umma_pair(const umma::PairParams& prm, const umma::Maps& maps, const DotScratch& plan, bool pdl, cudaStream_t stream) {
+  if (!raise_smem_limit((const void*)umma::umma_pair_kernel, 227 * 1024)) return 0;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)plan.grid);
+  cfg.blockDim = dim3(umma::kBaseThreads);
+  cfg.dynamicSmemBytes = plan.smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[3];
+  cfg.attrs = attr;
+  cfg.numAttrs = fill_launch_attributes(attr, pdl);
+  attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+  attr[cfg.numAttrs].val.clusterDim.x = 2;
+  attr[cfg.numAttrs].val.clusterDim.y = 1;
+  attr[cfg.numAttrs].val.clusterDim.z = 1;
+  cfg.numAttrs++;
+  return cudaLaunchKernelEx(&cfg, umma::umma_pair_kernel, prm, maps) == cudaSuccess ? 1 : 0;
 }
 
 int launch_umma(const DotShape* shapes, int count, const DotScratch& plan, const void* lhs, const void* const* rhs, void* const* out,
@@ -980,12 +1033,36 @@ int launch_umma(const DotShape* shapes, int count, const DotScratch& plan, const
     cuuint64_t gdim[2] = {(cuuint64_t)s.k, (cuuint64_t)s.m};
     // A single row has no stride to honour; any 16-byte multiple that covers the row will do.
     cuuint64_t gstride[1] = {(cuuint64_t)(s.m > 1 ? s.lhs_m : (s.k + 7) / 8 * 8) * 2};
-    cuuint32_t box[2] = {64, (cuuint32_t)plan.m_tile};
+    cuuint32_t box[2] = {64, (cuuint32_t)(plan.pair ? plan.m_tile / 2 : plan.m_tile)};
     if (enc(&maps.lhs, dt, 2, const_cast<void*>(lhs), gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
       return 0;
   }
   p.kblocks = (int)((s.k + 64 * plan.sub - 1) / (64 * plan.sub));
+  if (plan.pair) {
+    umma::PairParams q{};
+    q.m = p.m;
+    q.k = p.k;
+    q.m_tile = p.m_tile;
+    q.m_tiles = p.m_tiles;
+    q.count = count;
+    for (int g = 0; g < count; g++) {
+      q.n_tile_begin[g] = q.n_tiles;
+      q.n_tiles += (int)((shapes[g].n + umma::kPairN - 1) / umma::kPairN);
+      q.out[g] = p.out[g];
+      q.n[g] = p.n[g];
+      q.ldo[g] = p.ldo[g];
+    }
+    for (int g = count; g <= umma::kGroupMax; g++) q.n_tile_begin[g] = q.n_tiles;
+    q.kblocks = p.kblocks;
+    q.stages = plan.stages;
+    q.is_bf16 = s.dtype == kBF16;
+    q.rhs_k_major = k_major ? 1 : 0;
+    q.rhs_3d = p.rhs_3d;
+    q.early_rhs = early_rhs ? 1 : 0;
+    q.error_flag = error_flag;
+    return launch_umma_pair(q, maps, plan, pdl, stream);
+  }
   p.tiles = tiles;
   p.ksplit = plan.ksplit;
   p.rows_per_rank = (plan.m_tile + 4 * plan.ksplit - 1) / (4 * plan.ksplit) * 4;

@@ -96,7 +96,8 @@ struct DotScratch {
   // Paths 1 and 4 for 16-bit floats without batch axes can run on the tensor cores (tcgen05, accumulator in TMEM); path 5
   // always does. `ksplit` CTAs of a cluster then share a tile of 128 columns x m_tile rows, contracting 1/ksplit of k each;
   // nothing goes through scratch memory.
-  int umma = 0, m_tile = 0, sub = 1;
+  // `pair`: CTA pairs work on tiles of 256 columns (umma_pair.cuh).
+  int umma = 0, m_tile = 0, sub = 1, pair = 0;
   int grid = 0, stages = 0, max_contrib = 0;
   long long per_cta = 0;
   uint64_t smem = 0;

@@ -554,3 +554,33 @@ def test_contractions_with_unaligned_weight_rows_against_f64(gpu_backend, dtype,
     mag = np.abs(x.astype(np.float64)) @ np.abs(w.astype(np.float64))
     ulp = 2.0 ** (-9 if dtype == P.BF16_CODE else -12)
     assert np.all(np.abs(got.astype(np.float64) - want) <= 2 * ulp * np.abs(want) + k * 2.0 ** -24 * mag + 2.0 ** -24)
+
+
+@pytest.mark.parametrize("k_major", [False, True])
+@pytest.mark.parametrize("m,k,n,count", [
+    (300, 64, 256, 1),      # one block of k, one tile of columns
+    (257, 200, 520, 1),     # ragged k; the last tile's second CTA has eight columns, the last row tile one row
+    (512, 1024, 1000, 2),   # two contractions in one launch, columns that are no multiple of 64
+    (1000, 576, 4096, 1),   # several bands of weight tiles
+    (2048, 448, 2816, 1),   # several tiles per pair: both accumulators in turn, a last band that is not full
+])
+def test_paired_sm_contractions_against_f64(gpu_backend, k_major, m, k, n, count):
+    """Large 16-bit contractions on CTA pairs, both rhs layouts. Error: f32 sums and one rounding of the output."""
+    rng = np.random.default_rng(m + n)
+    dt = P.np_dtype(P.BF16_CODE)
+    x = rng.standard_normal((m, k), dtype=np.float32).astype(dt)
+    ws = [rng.standard_normal((k, n + 24 * g), dtype=np.float32).astype(dt) for g in range(count)]
+    b = PlanBuilder()
+    px = b.parameter(P.BF16_CODE, x.shape)
+    b.set_outputs([b.dot_general(px, b.parameter(P.BF16_CODE, w.T.shape if k_major else w.shape), [1], [1 if k_major else 0]) for w in ws])
+    exe = gpu_backend.compile_executable(b, [0])
+    steps = [s for s in exe.describe()["kernel_plan"]["steps"] if s["type"] == "dot"]
+    assert all(s["umma"] == 1 and s["pair"] == 1 for s in steps) and len(steps) == (count if k_major else 1), steps
+    args = [x] + [np.ascontiguousarray(w.T) if k_major else w for w in ws]
+    got, again = (run_backend(gpu_backend, b, args, exe=exe) for _ in range(2))
+    exe.destroy()
+    for g, a, w in zip(got, again, ws):
+        assert np.array_equal(g.view(np.uint16), a.view(np.uint16))
+        want = x.astype(np.float64) @ w.astype(np.float64)
+        mag = np.abs(x.astype(np.float64)) @ np.abs(w.astype(np.float64))
+        assert np.all(np.abs(g.astype(np.float64) - want) <= 2.0 ** -8 * np.abs(want) + k * 2.0 ** -24 * mag + 2.0 ** -24)
