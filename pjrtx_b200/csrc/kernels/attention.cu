@@ -25,6 +25,7 @@
 
 #include "../common.h"
 #include "kernels.h"
+#include "umma_attention.cuh"
 
 namespace pjrtx {
 
@@ -1028,13 +1029,18 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
 
 // A cache as the 4-d tensor [head_dim][keys][KV heads][sequences] (strides in elements come with the launch); the box
 // is 64 elements x kMmaStageKeys keys of one head of one sequence.
-bool encode_kv_map(CUtensorMap* map, const void* base, bool f16, const DecodeArgs& a, int head_dim) {
-  static const EncodeTiledFn enc = [] {
+EncodeTiledFn encode_tiled() {
+  static const EncodeTiledFn fn = [] {
     void* p = nullptr;
     cudaDriverEntryPointQueryResult q;
     if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess) p = nullptr;
     return (EncodeTiledFn)p;
   }();
+  return fn;
+}
+
+bool encode_kv_map(CUtensorMap* map, const void* base, bool f16, const DecodeArgs& a, int head_dim) {
+  const EncodeTiledFn enc = encode_tiled();
   if (!enc) return false;
   // A dimension of extent 1 may come with any stride (0 included); the encoder wants multiples of 16 bytes that
   // are not smaller than the dimension below, so give those dimensions the stride of the whole cache.
@@ -1141,295 +1147,58 @@ int dispatch_decode(int rep, int hd, const DecodeArgs& a, dim3 grid, const void*
 }
 
 
-// ---- Causal self-attention over whole sequences (prefill) ---------------------------------------------------------
-//
-// out[b, g, s, r, :] = softmax_j( q[b, g, s, r, :] . k[b, j, g, :] * scale  for j <= s ) . v[b, j, g, :]
-//
-// q and out are [batch, kv_heads, seq, rep, head_dim] (the operand and result layout of the recognised
-// dot_general -> masked softmax -> dot_general form), so the `seq * rep` query rows that share one KV head are one
-// contiguous row-major matrix; row `x` belongs to position x / rep. One CTA (4 warps) owns 64 consecutive rows and
-// walks the keys 0..(its last position) in stages of 64 through the same ring of tiled tensor-map copies and swizzled
-// layout as the decode kernel above; every warp owns 16 rows and multiplies them with all 64 keys of a stage:
-//   S[16 x 64] = Q[16 x HD] . K^T (mma.m16n8k16, Q fragments in registers), mask key <= position, online softmax on
-//   the fragments, O[16 x HD] += P[16 x 64] . V with the rounded probabilities as A fragments.
-// Scores and probabilities never leave the SM (the explicit form writes and re-reads batch*heads*seq*seq elements
-// twice per layer). Row tiles are scheduled longest first (the last rows see the most keys), and a warp skips the
-// stages that lie wholly above its rows' diagonal.
-struct PrefillArgs {
-  long long seq = 0, rows = 0;  // rows = seq * rep per (sequence, KV head)
-  int rep = 1, kv_heads = 1;
-  long long kv_batch_stride = 0, kv_row_stride = 0, kv_head_stride = 0;
-  float scale = 1.f;
-  int* error_flag = nullptr;
-};
-constexpr int kPrefillRows = 16 * kMmaWarps;
-constexpr int kPrefillStages = 2;  // 64 KiB per CTA at head_dim 128: three CTAs (twelve warps) per SM
+// ---- Causal self-attention over whole sequences (prefill, umma_attention.cuh) ---------------------------------------
 
-__device__ __forceinline__ float ex2_approx(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
+// q as [rows of all (sequence, KV head) matrices][head_dim], boxes of 128 rows x 64 elements.
+bool encode_query_map(CUtensorMap* map, const void* base, bool f16, long long rows, int head_dim) {
+  const EncodeTiledFn enc = encode_tiled();
+  if (!enc) return false;
+  const cuuint64_t gdim[2] = {(cuuint64_t)head_dim, (cuuint64_t)rows};
+  const cuuint64_t gstride[1] = {(cuuint64_t)head_dim * 2};
+  const cuuint32_t box[2] = {64, (cuuint32_t)umma::kAttnRows};
+  const cuuint32_t estr[2] = {1, 1};
+  return enc(map, f16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), gdim, gstride,
+             box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <typename T, int HD>
-__global__ void __launch_bounds__(kMmaWarps * 32, 3)
-attn_prefill_mma_kernel(PrefillArgs a, const T* __restrict__ q, const __grid_constant__ CUtensorMap kmap,
-                        const __grid_constant__ CUtensorMap vmap, T* __restrict__ out) {
-  static_assert(sizeof(T) == 2 && (HD == 64 || HD == 128), "16-bit elements, head_dim 64 or 128");
-  constexpr int HALVES = HD / 64;
-  constexpr int TILE_BYTES = kMmaStageKeys * HD * 2;
-  constexpr int STAGE_BYTES = 2 * TILE_BYTES;
-  // The swizzle of a tiled copy follows the absolute shared-memory address: tiles start on 1024-byte boundaries.
-  extern __shared__ unsigned char smem_prefill_raw[];
-  unsigned char* smem_attn = smem_prefill_raw + ((1024u - (attn_smem_u32(smem_prefill_raw) & 1023u)) & 1023u);
-  __shared__ int gave_up;
-  __shared__ __align__(8) uint64_t full[kPrefillStages];
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  if (threadIdx.x == 0) {
-    for (int st = 0; st < kPrefillStages; st++)
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(attn_smem_u32(&full[st])), "r"(1));
-    gave_up = 0;
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  __syncthreads();
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int g = blockIdx.y, b = blockIdx.z;
-  const long long tile_row0 = (long long)(gridDim.x - 1 - blockIdx.x) * kPrefillRows;  // longest tiles first
-  const long long last_row = min(tile_row0 + kPrefillRows, a.rows) - 1;
-  const int j_end = (int)(last_row / a.rep) + 1;  // keys 0 .. last position of the tile
-  const int stages_total = (j_end + kMmaStageKeys - 1) / kMmaStageKeys;
-
-  const long long bg = ((long long)b * a.kv_heads + g) * a.rows;
-  const unsigned smem_base = (unsigned)__cvta_generic_to_shared(smem_attn);
-  auto tile_offset = [](int row, int c) { return (unsigned)((c >> 3) * (kMmaStageKeys * 128) + row * 128 + (((c & 7) ^ (row & 7)) << 4)); };
-  // A stage is 64 K rows and 64 V rows, brought by one tiled copy per 128-byte column block of each (the decode
-  // kernel's maps and layout); one thread issues them. Keys past the tile's last position are other positions' rows
-  // (masked: their probabilities are zero and their values finite), keys past the sequence arrive as zeros.
-  auto issue_stage = [&](int st) {
-    if (threadIdx.x != 0) return;
-    const int slot = st % kPrefillStages;
-    const unsigned bar = attn_smem_u32(&full[slot]);
-    const unsigned dst = smem_base + (unsigned)slot * STAGE_BYTES;
-    const int j0 = st * kMmaStageKeys;
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(STAGE_BYTES) : "memory");
-#pragma unroll
-    for (int c = 0; c < HALVES; c++) {
-      asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(
-                       dst + c * (kMmaStageKeys * 128)),
-                   "l"(&kmap), "r"(c * 64), "r"(j0), "r"(g), "r"(b), "r"(bar)
-                   : "memory");
-      asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(
-                       dst + TILE_BYTES + c * (kMmaStageKeys * 128)),
-                   "l"(&vmap), "r"(c * 64), "r"(j0), "r"(g), "r"(b), "r"(bar)
-                   : "memory");
-    }
-  };
-  for (int st = 0; st < kPrefillStages - 1; st++)
-    if (st < stages_total) issue_stage(st);
-  unsigned long long deadline;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(deadline));
-  deadline += 2000000000ull;
-
-  // This thread's two rows (accumulator rows lane / 4 and lane / 4 + 8 of the warp's 16) and their positions;
-  // rows past the matrix end get position -1: every key is masked and nothing is stored.
-  const long long row_lo = tile_row0 + warp * 16 + (lane >> 2);
-  const long long rows2[2] = {row_lo, row_lo + 8};
-  int pos[2];
-#pragma unroll
-  for (int h = 0; h < 2; h++) pos[h] = rows2[h] < a.rows ? (int)(rows2[h] / a.rep) : -1;
-  const int warp_first_pos = (int)((tile_row0 + warp * 16) / a.rep);
-  const int warp_last_pos = (int)(min(tile_row0 + warp * 16 + 15, a.rows - 1) / a.rep);
-
-  unsigned qa[HD / 16][4];
-  {
-    const int c0 = (lane & 3) * 2;
-    const T* qrow0 = q + (bg + rows2[0]) * HD;
-    const T* qrow1 = q + (bg + rows2[1]) * HD;
-    const bool in0 = rows2[0] < a.rows, in1 = rows2[1] < a.rows;
-#pragma unroll
-    for (int ks = 0; ks < HD / 16; ks++) {
-      qa[ks][0] = in0 ? __ldg(reinterpret_cast<const unsigned*>(qrow0 + ks * 16 + c0)) : 0u;
-      qa[ks][1] = in1 ? __ldg(reinterpret_cast<const unsigned*>(qrow1 + ks * 16 + c0)) : 0u;
-      qa[ks][2] = in0 ? __ldg(reinterpret_cast<const unsigned*>(qrow0 + ks * 16 + c0 + 8)) : 0u;
-      qa[ks][3] = in1 ? __ldg(reinterpret_cast<const unsigned*>(qrow1 + ks * 16 + c0 + 8)) : 0u;
-    }
-  }
-  // Scores are kept in log2 units (score * scale * log2 e), so a probability is one ex2 of a difference. The row
-  // sums are one more accumulator tile: P times a matrix of ones, in the tensor pipe instead of 32 adds per thread.
-  const float c_log2 = a.scale * 1.4426950408889634f;
-  const unsigned ones = MmaOps<T>::pack(1.f, 1.f);
-  float m_run[2] = {-INFINITY, -INFINITY};
-  float lacc[4] = {0.f, 0.f, 0.f, 0.f};
-  float o[HD / 8][4];
-#pragma unroll
-  for (int nt = 0; nt < HD / 8; nt++)
-#pragma unroll
-    for (int e = 0; e < 4; e++) o[nt][e] = 0.f;
-
-  bool arrived = true;
-  for (int st = 0; st < stages_total; st++) {
-    {  // stage st has landed (bounded by time)
-      const unsigned bar = attn_smem_u32(&full[st % kPrefillStages]), parity = (unsigned)(st / kPrefillStages) & 1u;
-      for (unsigned spin = 0;; spin++) {
-        unsigned ok;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(ok)
-            : "r"(bar), "r"(parity)
-            : "memory");
-        if (ok) break;
-        if ((spin & 255) == 255) {
-          unsigned long long now;
-          asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
-          if (now > deadline || *reinterpret_cast<volatile int*>(&gave_up)) {
-            gave_up = 1;
-            arrived = false;
-            break;
-          }
-        }
-      }
-    }
-    // Everyone is done with stage st - 1 (its slot is refilled below); a thread that gave up tells the others here.
-    arrived = __syncthreads_and(arrived ? 1 : 0) != 0;
-    if (!arrived) break;
-    if (st + kPrefillStages - 1 < stages_total) issue_stage(st + kPrefillStages - 1);
-    const int key0 = st * kMmaStageKeys;
-    if (key0 > warp_last_pos) continue;  // wholly above this warp's diagonal
-
-    const unsigned ktile = smem_base + (unsigned)(st % kPrefillStages) * STAGE_BYTES;
-    const unsigned vtile = ktile + TILE_BYTES;
-    // S = Q . K^T for 64 keys: eight accumulator tiles of 8 keys.
-    float sc[kMmaStageKeys / 8][4];
-#pragma unroll
-    for (int nt = 0; nt < kMmaStageKeys / 8; nt++)
-#pragma unroll
-      for (int e = 0; e < 4; e++) sc[nt][e] = 0.f;
-#pragma unroll
-    for (int kb16 = 0; kb16 < kMmaStageKeys / 16; kb16++) {
-#pragma unroll
-      for (int ks = 0; ks < HD / 16; ks++) {
-        unsigned bk[4];
-        const int key = kb16 * 16 + ((lane >> 4) << 3) + (lane & 7);
-        const int chunk = ks * 2 + ((lane >> 3) & 1);
-        ldmatrix_x4(bk, ktile + tile_offset(key, chunk));
-        MmaOps<T>::mma(sc[2 * kb16], qa[ks], bk[0], bk[1]);
-        MmaOps<T>::mma(sc[2 * kb16 + 1], qa[ks], bk[2], bk[3]);
-      }
-    }
-    // Accumulator element e of tile nt: row h = e / 2, key key0 + nt * 8 + (lane % 4) * 2 + (e % 2). The explicit
-    // form rounds q.k to the element type before it scales; only stages that touch the diagonal need the mask.
-    const bool diagonal = key0 + kMmaStageKeys - 1 > warp_first_pos;
-    const int key_base = key0 + (lane & 3) * 2;
-    float mx[2] = {-INFINITY, -INFINITY};
-#pragma unroll
-    for (int nt = 0; nt < kMmaStageKeys / 8; nt++)
-#pragma unroll
-      for (int e = 0; e < 4; e++) {
-        float d = Elem<T>::round(sc[nt][e]) * c_log2;
-        if (diagonal && key_base + nt * 8 + (e & 1) > pos[e >> 1]) d = -INFINITY;
-        sc[nt][e] = d;
-        mx[e >> 1] = fmaxf(mx[e >> 1], d);
-      }
-    unsigned pa[kMmaStageKeys / 16][4];
-#pragma unroll
-    for (int h = 0; h < 2; h++) {
-      mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], 1));
-      mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], 2));
-      const float m_new = fmaxf(m_run[h], mx[h]);
-      // Rows with no visible key yet (only rows past the matrix end) keep everything at zero.
-      const float m_use = m_new == -INFINITY ? 0.f : m_new;
-      const float corr = ex2_approx(m_run[h] - m_use);
-      if (m_new != m_run[h]) {
-        lacc[2 * h] *= corr;
-        lacc[2 * h + 1] *= corr;
-#pragma unroll
-        for (int nt = 0; nt < HD / 8; nt++) {
-          o[nt][2 * h] *= corr;
-          o[nt][2 * h + 1] *= corr;
-        }
-      }
-      m_run[h] = m_new;
-#pragma unroll
-      for (int kb16 = 0; kb16 < kMmaStageKeys / 16; kb16++) {
-        // The probabilities enter both products (values and row sum) rounded to the element type.
-        pa[kb16][h] = MmaOps<T>::pack(ex2_approx(sc[2 * kb16][2 * h] - m_use), ex2_approx(sc[2 * kb16][2 * h + 1] - m_use));
-        pa[kb16][2 + h] = MmaOps<T>::pack(ex2_approx(sc[2 * kb16 + 1][2 * h] - m_use), ex2_approx(sc[2 * kb16 + 1][2 * h + 1] - m_use));
-      }
-    }
-    // O += P . V and l += P . 1
-#pragma unroll
-    for (int kb16 = 0; kb16 < kMmaStageKeys / 16; kb16++) {
-      MmaOps<T>::mma(lacc, pa[kb16], ones, ones);
-#pragma unroll
-      for (int np = 0; np < HD / 16; np++) {
-        unsigned bv[4];
-        const int key = kb16 * 16 + (((lane >> 3) & 1) << 3) + (lane & 7);
-        const int chunk = np * 2 + (lane >> 4);
-        ldmatrix_x4_trans(bv, vtile + tile_offset(key, chunk));
-        MmaOps<T>::mma(o[2 * np], pa[kb16], bv[0], bv[1]);
-        MmaOps<T>::mma(o[2 * np + 1], pa[kb16], bv[2], bv[3]);
-      }
-    }
-  }
-  if (!arrived) {
-    // Copies of the next stage may still be in flight towards this CTA's shared memory: give them a bounded time
-    // before leaving, then report (nothing is stored).
-    for (int st = 0; st < stages_total; st++) {
-      const unsigned bar = attn_smem_u32(&full[st % kPrefillStages]), parity = (unsigned)(st / kPrefillStages) & 1u;
-      for (unsigned spin = 0; spin < (1u << 16); spin++) {
-        unsigned ok;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(ok)
-            : "r"(bar), "r"(parity)
-            : "memory");
-        if (ok) break;
-      }
-    }
-    if (threadIdx.x == 0 && a.error_flag) atomicExch(a.error_flag, 8);
-    return;
-  }
-
-  const int c0 = (lane & 3) * 2;
-#pragma unroll
-  for (int h = 0; h < 2; h++) {
-    if (rows2[h] >= a.rows) continue;
-    const float l = lacc[2 * h];
-    const float inv = l > 0.f ? 1.f / l : 0.f;
-    T* orow = out + (bg + rows2[h]) * HD + c0;
-#pragma unroll
-    for (int nt = 0; nt < HD / 8; nt++)
-      *reinterpret_cast<unsigned*>(orow + nt * 8) = MmaOps<T>::pack(o[nt][2 * h] * inv, o[nt][2 * h + 1] * inv);
-  }
-}
-
-template <typename T, int HD>
-int launch_prefill_mma(const PrefillArgs& a, dim3 grid, const void* q, const void* k, const void* v, void* out, bool pdl,
-                       cudaStream_t stream) {
-  constexpr size_t smem = 1024 + (size_t)kPrefillStages * 2 * kMmaStageKeys * HD * 2;
-  if (!raise_smem_limit((const void*)attn_prefill_mma_kernel<T, HD>, (int)smem)) return 0;
-  if (((reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v)) & 15) != 0) return 0;
-  // K and V as [head_dim][keys][KV heads][sequences], the decode kernel's maps.
-  DecodeArgs view{};
-  view.kv_len = a.seq;
-  view.kv_heads = a.kv_heads;
-  view.batch = grid.z;
-  view.kv_batch_stride = a.kv_batch_stride;
-  view.kv_row_stride = a.kv_row_stride;
-  view.kv_head_stride = a.kv_head_stride;
-  CUtensorMap kmap, vmap;
-  const bool f16 = std::is_same<T, __half>::value;
-  if (!encode_kv_map(&kmap, k, f16, view, HD) || !encode_kv_map(&vmap, v, f16, view, HD)) return 0;
-  return launch_kernel(attn_prefill_mma_kernel<T, HD>, grid, dim3(kMmaWarps * 32), smem, stream, pdl, a, (const T*)q, kmap, vmap,
-                       (T*)out) == cudaSuccess
+template <bool BF16, int HD, int TILES>
+int launch_prefill_tiles(const AttnPrefillShape& s, const umma::AttnParams& p, const CUtensorMap& qmap, const CUtensorMap& kmap,
+                         const CUtensorMap& vmap, void* out, bool pdl, cudaStream_t stream) {
+  constexpr size_t smem = umma::attn_smem_bytes(HD, TILES);
+  if (!raise_smem_limit((const void*)umma::umma_attention_kernel<BF16, HD, TILES>, (int)smem)) return 0;
+  const dim3 grid((unsigned)((p.rows + umma::kAttnRows * TILES - 1) / (umma::kAttnRows * TILES)), (unsigned)s.kv_heads, (unsigned)s.batch);
+  return launch_kernel(umma::umma_attention_kernel<BF16, HD, TILES>, grid, dim3(128 * TILES + 64), smem, stream, pdl, p, qmap, kmap, vmap,
+                       out) == cudaSuccess
              ? 1
              : 0;
+}
+
+template <bool BF16, int HD>
+int launch_prefill(const AttnPrefillShape& s, const umma::AttnParams& p, const void* q, const void* k, const void* v, void* out, bool pdl,
+                   cudaStream_t stream) {
+  if (((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) |
+        reinterpret_cast<uintptr_t>(out)) & 15) != 0)
+    return 0;
+  // K and V as [head_dim][keys][KV heads][sequences], the decode kernel's maps (boxes of 64 keys).
+  DecodeArgs view{};
+  view.kv_len = s.seq;
+  view.kv_heads = p.kv_heads;
+  view.batch = s.batch;
+  view.kv_batch_stride = s.kv_batch_stride;
+  view.kv_row_stride = s.kv_row_stride;
+  view.kv_head_stride = s.kv_head_stride;
+  CUtensorMap qmap, kmap, vmap;
+  if (!encode_query_map(&qmap, q, !BF16, p.rows * s.kv_heads * s.batch, HD) || !encode_kv_map(&kmap, k, !BF16, view, HD) ||
+      !encode_kv_map(&vmap, v, !BF16, view, HD))
+    return 0;
+  // Two row tiles per CTA share every key block and let one tile's softmax overlap the other's products; one tile per CTA
+  // where that would leave SMs without work.
+  int device = 0, sms = 148;
+  if (cudaGetDevice(&device) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+  const long long pairs = (p.rows + 2 * umma::kAttnRows - 1) / (2 * umma::kAttnRows) * s.kv_heads * s.batch;
+  return pairs >= sms ? launch_prefill_tiles<BF16, HD, 2>(s, p, qmap, kmap, vmap, out, pdl, stream)
+                      : launch_prefill_tiles<BF16, HD, 1>(s, p, qmap, kmap, vmap, out, pdl, stream);
 }
 
 }  // namespace
@@ -1576,7 +1345,7 @@ bool attn_prefill_supported(const AttnPrefillShape& s) {
   if (s.head_dim != 64 && s.head_dim != 128) return false;
   if (s.batch < 1 || s.kv_heads < 1 || s.rep < 1 || s.seq < 1 || s.seq > (1LL << 30)) return false;
   if (s.batch > 65535 || s.kv_heads > 65535) return false;
-  if ((s.seq * s.rep + kPrefillRows - 1) / kPrefillRows > 0x7fffffffLL) return false;
+  if ((s.seq * s.rep + umma::kAttnRows - 1) / umma::kAttnRows > 0x7fffffffLL) return false;
   // 16-byte key/value rows.
   if (s.kv_row_stride % 8 || s.kv_head_stride % 8 || s.kv_batch_stride % 8) return false;
   return true;
@@ -1585,22 +1354,17 @@ bool attn_prefill_supported(const AttnPrefillShape& s) {
 int attn_prefill_launch(const AttnPrefillShape& s, const void* q, const void* k, const void* v, void* out, bool pdl,
                         cudaStream_t stream, int* error_flag) {
   if (!attn_prefill_supported(s)) return 0;
-  PrefillArgs a;
-  a.error_flag = error_flag;
-  a.seq = s.seq;
-  a.rep = (int)s.rep;
-  a.rows = s.seq * s.rep;
-  a.kv_heads = (int)s.kv_heads;
-  a.kv_batch_stride = s.kv_batch_stride;
-  a.kv_row_stride = s.kv_row_stride;
-  a.kv_head_stride = s.kv_head_stride;
-  a.scale = s.scale;
-  dim3 grid((unsigned)((a.rows + kPrefillRows - 1) / kPrefillRows), (unsigned)s.kv_heads, (unsigned)s.batch);
+  umma::AttnParams p;
+  p.rows = s.seq * s.rep;
+  p.rep = (int)s.rep;
+  p.kv_heads = (int)s.kv_heads;
+  p.sign = s.scale > 0.f ? 1.f : s.scale < 0.f ? -1.f : 0.f;
+  p.scale_log2 = s.scale == 0.f ? 1.f : fabsf(s.scale) * 1.4426950408889634f;
+  p.is_bf16 = s.dtype == kBF16;
+  p.error_flag = error_flag;
   if (s.dtype == kBF16)
-    return s.head_dim == 128 ? launch_prefill_mma<__nv_bfloat16, 128>(a, grid, q, k, v, out, pdl, stream)
-                             : launch_prefill_mma<__nv_bfloat16, 64>(a, grid, q, k, v, out, pdl, stream);
-  return s.head_dim == 128 ? launch_prefill_mma<__half, 128>(a, grid, q, k, v, out, pdl, stream)
-                           : launch_prefill_mma<__half, 64>(a, grid, q, k, v, out, pdl, stream);
+    return s.head_dim == 128 ? launch_prefill<true, 128>(s, p, q, k, v, out, pdl, stream) : launch_prefill<true, 64>(s, p, q, k, v, out, pdl, stream);
+  return s.head_dim == 128 ? launch_prefill<false, 128>(s, p, q, k, v, out, pdl, stream) : launch_prefill<false, 64>(s, p, q, k, v, out, pdl, stream);
 }
 
 }  // namespace pjrtx

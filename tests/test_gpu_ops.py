@@ -438,6 +438,29 @@ def test_prefill_attention_matches_oracle(gpu_backend, dtype, kv_heads, rep, seq
     assert_outputs(b, got, run_oracle(b, args), f"prefill attention {kv_heads}x{rep} seq {seq} hd {hd}")
 
 
+@pytest.mark.parametrize("dtype,batch,kv_heads,rep,seq,hd,spread", [
+    (P.BF16_CODE, 2, 8, 4, 700, 128, 1.0),  # two row tiles per CTA, six key blocks: the copy ring wraps
+    (P.F16, 5, 8, 4, 257, 64, 1.0),         # two row tiles, a third block that holds one key
+    (P.F16, 1, 2, 1, 385, 64, 8.0),         # scores in the hundreds: maxima grow by more than 2^8 between blocks
+    (P.BF16_CODE, 2, 37, 1, 300, 128, 8.0),  # the same with two row tiles; a row tile spans a whole key block
+])
+def test_prefill_attention_against_f64(gpu_backend, dtype, batch, kv_heads, rep, seq, hd, spread):
+    """Two row tiles per CTA and rescaled outputs, against the exact attention. The probabilities enter the second product
+    in the element type (half a unit in the last place of the largest value) and the result is rounded once more; a score's
+    f32 error moves its probability by less than that."""
+    b, args = cases.prefill_attention(dtype=dtype, batch=batch, kv_heads=kv_heads, rep=rep, seq=seq, head_dim=hd)
+    q, k, v = args
+    q = (q.astype(np.float32) * spread).astype(q.dtype)
+    got = run_backend(gpu_backend, b, [q, k, v])[0].astype(np.float64)
+    q64, k64, v64 = (a.astype(np.float64) for a in (q, k, v))
+    s = np.einsum("bgsrd,bjgd->bgsrj", q64, k64) / np.float64(np.float32(np.sqrt(np.float32(hd))))
+    s = np.where(np.arange(seq)[:, None, None] >= np.arange(seq)[None, None, :], s, -np.inf)
+    p = np.exp(s - s.max(-1, keepdims=True))
+    want = np.einsum("bgsrj,bjgd->bgsrd", p / p.sum(-1, keepdims=True), v64)
+    ulp = 2.0 ** (-9 if dtype == P.BF16_CODE else -12)
+    assert np.max(np.abs(got - want)) <= 3 * ulp * np.max(np.abs(v64))
+
+
 def test_prefill_attention_same_as_written_chain(gpu_backend, monkeypatch):
     """The kernel and the unfused chain (dot -> softmax row kernel -> dot) agree within the 16-bit tolerance."""
     b, args = cases.prefill_attention(seq=150, rep=4, head_dim=128)
