@@ -6,6 +6,7 @@
 #include <cstring>
 #include <functional>
 #include <map>
+#include <numeric>
 
 namespace pjrtx {
 
@@ -210,6 +211,13 @@ struct VecAccess {
   std::string array;
 };
 
+// How an index expression moves over the `vec` consecutive elements of one vector: value(v) = value(0) + coef * v, and
+// value(0) is a multiple of `align` (0: the value is zero).
+struct Run {
+  bool known = false;
+  int64_t coef = 0, align = 1;
+};
+
 class Gen {
  public:
   Gen(const Plan& plan, const std::vector<size_t>& nodes, const std::vector<uint32_t>& outputs,
@@ -276,6 +284,9 @@ class Gen {
   std::map<uint32_t, std::string> reduce_var_;  // reduce result value -> row-scope variable
   std::vector<Scope*> scopes_;
   std::vector<VecAccess> vec_loads_;  // of the loop body being emitted
+  std::vector<std::string> run_decls_;  // declarations of what the first element of a vector loads for all of them
+  std::map<std::string, Run> runs_;     // index variables of the loop body being emitted
+  int per_element_ = 0;                 // > 0: inside a branch or loop that is not the same for a whole vector
   bool in_vec_loop_ = false;
 
   [[noreturn]] void fail(const std::string& why) { throw Fail{why}; }
@@ -403,6 +414,89 @@ class Gen {
       while (vec_ > 1 && extent % vec_ != 0) vec_ /= 2;
   }
 
+  // ---- runs over a vector -------------------------------------------------
+  // An operand reached through views (transpose, slice, concatenate, broadcast ...) has an index computed per element, and
+  // reading it element by element makes the kernel bound by load instructions: the rotation of q and k over 4 x 2048
+  // positions took 249 us for 268 MB that way. Where every quotient and remainder on the way works on whole vectors, the
+  // elements of a vector are neighbours in the operand too (coef 1, one vector load) or all the same one (coef 0, one
+  // scalar load). The loop over a vector is unrolled, so the load is written `if (v == 0)`: the index arithmetic of the
+  // other elements is dead code.
+  Run run_of(const std::string& expr) const {
+    const char* p = expr.c_str();
+    Run r = run_sum(&p);
+    return *p == 0 ? r : Run{};
+  }
+  static void skip_space(const char** p) {
+    while (**p == ' ') (*p)++;
+  }
+  Run run_sum(const char** p) const {
+    Run a = run_product(p);
+    for (skip_space(p); **p == '+' || **p == '-'; skip_space(p)) {
+      const bool minus = *(*p)++ == '-';
+      const Run b = run_product(p);
+      a = Run{a.known && b.known, a.coef + (minus ? -b.coef : b.coef), std::gcd(a.align, b.align)};
+    }
+    return a;
+  }
+  Run run_product(const char** p) const {
+    Run a = run_atom(p);
+    for (skip_space(p); **p == '*' || **p == '/' || **p == '%'; skip_space(p)) {
+      const char op = *(*p)++;
+      skip_space(p);
+      char* end;
+      const int64_t n = strtoll(*p, &end, 10);
+      if (end == *p || n <= 0) return Run{};
+      *p = end;
+      // Over a whole vector a value that starts at a multiple of vec_ stays inside one block of n (a multiple of vec_).
+      const bool whole = a.coef == 0 || (a.coef == 1 && a.align % vec_ == 0 && n % vec_ == 0);
+      if (op == '*') a = Run{a.known, a.coef * n, a.align * n};
+      else if (op == '/') a = Run{a.known && whole, 0, a.align % n == 0 ? a.align / n : 1};
+      else a = Run{a.known && whole, a.coef, std::gcd(a.align, n)};
+    }
+    return a;
+  }
+  Run run_atom(const char** p) const {
+    skip_space(p);
+    if (!strncmp(*p, "(idx_t)", 7)) {
+      *p += 7;
+      return run_atom(p);
+    }
+    if (**p == '(') {
+      (*p)++;
+      Run r = run_sum(p);
+      skip_space(p);
+      if (**p != ')') return Run{};
+      (*p)++;
+      return r;
+    }
+    if (isdigit((unsigned char)**p)) {
+      char* end;
+      const int64_t n = strtoll(*p, &end, 10);
+      *p = end;
+      return Run{true, 0, n};
+    }
+    std::string name;
+    while (isalnum((unsigned char)**p) || **p == '_') name += *(*p)++;
+    if (**p == '(') return Run{};  // a call
+    if (name == "i" || name == "c") return Run{true, 1, vec_};
+    if (name == "r") return Run{true, 0, 1};
+    auto it = runs_.find(name);
+    return it == runs_.end() ? Run{} : it->second;
+  }
+  // `index < bound` has the same answer for every element of a vector.
+  bool uniform_below(const std::string& index, int64_t bound) const {
+    const Run r = run_of(index);
+    return r.known && (r.coef == 0 || (r.coef == 1 && r.align % vec_ == 0 && bound % vec_ == 0));
+  }
+  bool runs_apply() const { return in_vec_loop_ && vec_ > 1 && per_element_ == 0; }
+  // A condition that is the same for every element of a vector is evaluated for the first one.
+  std::string hoisted_condition(const std::string& cond) {
+    const std::string b = tmp("B");
+    run_decls_.push_back("bool " + b + " = false;");
+    line("if (v == 0) " + b + " = " + cond + ";");
+    return b;
+  }
+
   // ---- index helpers ----------------------------------------------------
   std::string index_var(const std::string& expr) {
     auto it = scope().index_memo.find(expr);
@@ -415,6 +509,10 @@ class Gen {
     std::string v = tmp("j");
     line("const idx_t " + v + " = " + expr + ";");
     scope().index_memo[expr] = v;
+    if (in_vec_loop_) {
+      const Run r = run_of(expr);
+      if (r.known) runs_[v] = r;
+    }
     return v;
   }
 
@@ -557,6 +655,20 @@ class Gen {
       VecAccess a{v, idx.cls, strfmt("L%d%s", s, idx.cls == IdxClass::LIN ? "i" : "c")};
       vec_loads_.push_back(a);
       return load_conv(value.dtype, a.array + "[v]");
+    }
+    if (runs_apply()) {
+      const Run r = run_of(idx.var);
+      const std::string g = r.known ? tmp("G") : "";
+      if (r.known && r.coef == 1 && r.align % vec_ == 0) {
+        run_decls_.push_back(strfmt("__align__(16) %s %s[%d];", ctype(value.dtype), g.c_str(), vec_));
+        line(strfmt("if (v == 0) ldvec<%s, %d>(%s, in%d + %s);", ctype(value.dtype), vec_, g.c_str(), s, idx.var.c_str()));
+        return load_conv(value.dtype, g + "[v]");
+      }
+      if (r.known && r.coef == 0) {
+        run_decls_.push_back(strfmt("%s %s;", ctype(value.dtype), g.c_str()));
+        line(strfmt("if (v == 0) %s = __ldg(in%d + %s);", g.c_str(), s, idx.var.c_str()));
+        return load_conv(value.dtype, g);
+      }
     }
     return load_conv(value.dtype, strfmt("__ldg(in%d + %s)", s, idx.var.c_str()));
   }
@@ -782,12 +894,14 @@ class Gen {
         if (lo.size() != sd.size() || (!interior.empty() && interior.size() != sd.size())) fail("pad attributes do not match the operand rank");
         std::vector<std::string> oc = coords(idx.var, out.dims), sc(sd.size());
         std::string cond;
+        bool uniform = true;
         for (size_t d = 0; d < sd.size(); d++) {
           const int64_t step = (interior.empty() ? 0 : interior[d]) + 1;
           if (step < 1) fail("negative interior padding");
           std::string t = index_var("((idx_t)" + oc[d] + " - (idx_t)" + std::to_string(lo[d]) + ")");
           std::string inside = "(" + t + " >= 0 && " + t + " < (idx_t)" + std::to_string((sd[d] - 1) * step + 1);
           if (step > 1) inside += " && " + t + " % " + std::to_string(step) + " == 0";
+          uniform &= uniform_below(t, (sd[d] - 1) * step + 1) && (step == 1 || run_of(t).coef == 0);
           inside += ")";
           cond += (cond.empty() ? "" : " && ") + inside;
           sc[d] = step > 1 ? "(" + t + " / " + std::to_string(step) + ")" : t;
@@ -795,7 +909,9 @@ class Gen {
         if (cond.empty()) cond = "true";
         std::string name = tmp("t");
         line(std::string(comp_type(dt)) + " " + name + ";");
+        if (runs_apply() && uniform) cond = hoisted_condition(cond);
         line("if (" + cond + ") {");
+        if (!uniform) per_element_++;
         {
           Scope inner;
           inner.indent = scope().indent + 2;
@@ -815,6 +931,7 @@ class Gen {
           scopes_.pop_back();
           scope().code += inner.code;
         }
+        if (!uniform) per_element_--;
         line("}");
         scope().memo[{v, idx.var}] = name;
         return name;
@@ -825,11 +942,21 @@ class Gen {
         std::string name = tmp("t");
         line(std::string(comp_type(dt)) + " " + name + ";");
         int64_t offset = 0;
+        bool uniform = true;
+        std::vector<std::string> conds;
+        for (size_t k = 0; k + 1 < ins.inputs.size(); k++) {
+          offset += val(in(k)).dims[dim];
+          conds.push_back(strfmt("%s < %lld", oc[dim].c_str(), (long long)offset));
+          uniform &= uniform_below(oc[dim], offset);
+        }
+        if (runs_apply() && uniform)
+          for (std::string& c : conds) c = hoisted_condition(c);
+        if (!uniform) per_element_++;
+        offset = 0;
         for (size_t k = 0; k < ins.inputs.size(); k++) {
           const auto& sd = val(in(k)).dims;
           bool last = k + 1 == ins.inputs.size();
-          std::string cond = last ? "" : strfmt("if (%s < %lld) ", oc[dim].c_str(), (long long)(offset + sd[dim]));
-          line(std::string(k ? "else " : "") + cond + "{");
+          line(std::string(k ? "else " : "") + (last ? "" : "if (" + conds[k] + ") ") + "{");
           Scope inner;
           inner.indent = scope().indent + 2;
           scopes_.push_back(&inner);
@@ -842,6 +969,7 @@ class Gen {
           line("}");
           offset += sd[dim];
         }
+        if (!uniform) per_element_--;
         scope().memo[{v, idx.var}] = name;
         return name;
       }
@@ -856,6 +984,8 @@ class Gen {
         std::string d = index_var("(" + idx.var + " % " + std::to_string(row_elems) + ")");
         std::string id = emit(in(1), Idx{b, IdxClass::GEN});
         std::string rowv = index_var(strfmt("min(max((idx_t)%s, (idx_t)0), (idx_t)%lld)", id.c_str(), (long long)(od[0] - 1)));
+        // One id for the whole vector: one row.
+        if (in_vec_loop_ && run_of(b).known && run_of(b).coef == 0) runs_[rowv] = Run{true, 0, 1};
         return emit(in(0), Idx{index_var("(idx_t)" + rowv + " * " + std::to_string(row_elems) + " + " + d), IdxClass::GEN});
       }
       case Kind::reduce_sum: case Kind::reduce_max: case Kind::reduce_min: case Kind::reduce_and: case Kind::reduce_or: {
@@ -949,6 +1079,7 @@ class Gen {
     Scope inner;
     inner.indent = scope().indent;
     scopes_.push_back(&inner);
+    per_element_++;  // the loads below repeat inside the loops just opened
     Idx sidx{index_var(linearize(sc, src.dims)), IdxClass::GEN};
     std::string e = emit(ins.inputs[0], sidx);
     if (pair) {
@@ -959,6 +1090,7 @@ class Gen {
     } else {
       line(acc + " = " + reduce_combine(ins.kind, dt, acc, e) + ";");
     }
+    per_element_--;
     scopes_.pop_back();
     scope().code += inner.code;
     for (int k = 0; k < opened; k++) {
@@ -1018,6 +1150,8 @@ class Gen {
       scopes_.push_back(&body);
       in_vec_loop_ = true;
       vec_loads_.clear();
+      run_decls_.clear();
+      runs_.clear();
       Idx lin{"i", IdxClass::LIN};
       std::vector<std::string> decl, after;
       for (const Item& it : all) {
@@ -1067,6 +1201,7 @@ class Gen {
           loops += strfmt("    __align__(16) %s %s[%d]; ldvec<%s, %d>(%s, in%d + i0);\n", t, a.array.c_str(), vec_, t, vec_,
                           a.array.c_str(), input_slot_[a.value]);
         }
+        for (const std::string& d : run_decls_) loops += "    " + d + "\n";
         for (const std::string& d : decl) loops += d;
         loops += strfmt("#pragma unroll\n    for (int v = 0; v < %d; v++) {\n      const idx_t i = i0 + v;\n", vec_);
         loops += body.code;
@@ -1166,6 +1301,8 @@ class Gen {
       scopes_.push_back(&body);
       in_vec_loop_ = true;
       vec_loads_.clear();
+      run_decls_.clear();
+      runs_.clear();
       Idx lin{"i", IdxClass::LIN};
       for (size_t q = 0; q < stage_reduces.size(); q++) {
         const Instruction* ins = stage_reduces[q];
@@ -1198,6 +1335,7 @@ class Gen {
           code += strfmt("      __align__(16) %s %s[%d]; ldvec<%s, %d>(%s, in%d + %s);\n", t, a.array.c_str(), vec_, t, vec_,
                          a.array.c_str(), input_slot_[a.value], a.cls == IdxClass::LIN ? "i0" : "c0");
         }
+        for (const std::string& d : run_decls_) code += "      " + d + "\n";
         for (size_t s : lin_outputs) code += strfmt("      __align__(16) %s S%zu[%d];\n", ctype(val(outputs_[s]).dtype), s, vec_);
         code += strfmt("#pragma unroll\n      for (int v = 0; v < %d; v++) {\n        const idx_t c = c0 + v; const idx_t i = i0 + v;\n", vec_);
         code += body.code;

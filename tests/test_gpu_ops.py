@@ -607,3 +607,27 @@ def test_paired_sm_contractions_against_f64(gpu_backend, k_major, m, k, n, count
         want = x.astype(np.float64) @ w.astype(np.float64)
         mag = np.abs(x.astype(np.float64)) @ np.abs(w.astype(np.float64))
         assert np.all(np.abs(g.astype(np.float64) - want) <= 2.0 ** -8 * np.abs(want) + k * 2.0 ** -24 * mag + 2.0 ** -24)
+
+
+@pytest.mark.parametrize("dtype,half,lead", [
+    (P.BF16_CODE, 64, (3, 5)),   # whole vectors everywhere: vector reads through every view
+    (P.F16, 12, (4, 7)),         # the concatenation's boundary falls inside a vector of eight
+    (P.F32, 3, (6, 4)),          # rows that are no multiple of a vector
+    (P.F32, 2, (2, 3)),          # a boundary inside a vector of four
+])
+def test_reads_through_views_are_exact(gpu_backend, dtype, half, lead):
+    """Slices, a concatenation, a transpose, broadcasts and a pad reach the operand at computed indices; the kernel reads
+    whole vectors where the indices of a vector are neighbours. Only moves, negations and one product: bit-exact."""
+    rng = np.random.default_rng(half)
+    a, c = lead
+    d = 2 * half
+    x = rng.standard_normal((a, c, d), dtype=np.float32).astype(P.np_dtype(dtype))
+    s = rng.standard_normal((c, d), dtype=np.float32).astype(P.np_dtype(dtype))
+    b = PlanBuilder()
+    px, ps = b.parameter(dtype, x.shape), b.parameter(dtype, s.shape)
+    lo, hi = b.slice(px, [0, 0, 0], [a, c, half]), b.slice(px, [0, 0, half], [a, c, d])
+    rot = b.concatenate([-hi, lo], 2) * b.broadcast_in_dim(ps, [a, c, d], [1, 2])
+    b.set_outputs([b.transpose(rot, [1, 0, 2]), b.reshape(b.transpose(px, [1, 0, 2]), [c, a * d])])
+    got = run_backend(gpu_backend, b, [x, s])
+    for g, w in zip(got, run_oracle(b, [x, s])):
+        assert np.array_equal(g.view(np.uint8), w.view(np.uint8))
