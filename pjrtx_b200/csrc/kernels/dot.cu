@@ -454,6 +454,128 @@ inline bool sgemm_ok(const DotShape& s, const void* lhs, const void* rhs, const 
          al16(lhs) && al16(rhs) && al16(out) && (s.m + kSgBM - 1) / kSgBM <= 65535;
 }
 
+// ---------------------------------------------------------------- small streaming contractions
+// out[m, n] = sum_k lhs[m, k] * rhs[k, n] for m <= 8, n contiguous and k so small (kSmallRows) that a CTA can hold its
+// whole share of the rhs in registers: toy decoders, closed-over blocks. What bounds such a contraction is the chain of
+// dependent latencies, not bytes. The persistent kernel's chain is tensor map -> copy -> mbarrier -> partial sums in global
+// memory -> arrival counter -> fold; here a CTA owns 64 columns for all of k, requests every 16-byte piece of its weights
+// at once (before the preceding kernel has finished, where nothing writes them), then the lhs, multiplies, and folds the
+// eight warps through shared memory in a fixed order.
+constexpr int kSmallCols = 64, kSmallThreads = 256, kSmallPasses = 16;
+// Rows a CTA covers in one round of loads: 8 warps x 32 lanes x 16 bytes over 64 columns.
+__host__ __device__ constexpr int small_rows_per_pass(int esize) { return kSmallThreads * 16 / (kSmallCols * esize); }
+__host__ __device__ constexpr int small_max_k(int esize) { return kSmallPasses * small_rows_per_pass(esize); }
+
+struct SmallGroup {
+  int count;
+  int tile_begin[kDotGroupMax + 1];
+  const void* rhs[kDotGroupMax];
+  void* out[kDotGroupMax];
+  long long n[kDotGroupMax], rhs_k[kDotGroupMax], out_m[kDotGroupMax];
+  int m, k;
+  long long lhs_m, lhs_k;
+  int early_rhs;
+};
+
+template <typename T, int M>
+__global__ void __launch_bounds__(kSmallThreads) small_dot_kernel(SmallGroup grp, const T* __restrict__ lhs) {
+  constexpr int V = 16 / sizeof(T), LANES = kSmallCols / V, RP = small_rows_per_pass(sizeof(T));
+  __shared__ float fold[kSmallThreads / 32][M][kSmallCols];
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  int g = 0;
+#pragma unroll
+  for (int q = 1; q < kDotGroupMax; q++)
+    if (q < grp.count && (int)blockIdx.x >= grp.tile_begin[q]) g = q;
+  const long long n0 = (long long)((int)blockIdx.x - grp.tile_begin[g]) * kSmallCols;
+  const int chunk = threadIdx.x % LANES, row0 = threadIdx.x / LANES;  // this thread: V columns of rows row0, row0 + RP, ...
+  const long long n = n0 + chunk * V;
+  const bool in = n < grp.n[g];  // (n is a multiple of V)
+  const T* rhs = static_cast<const T*>(grp.rhs[g]) + n;
+  uint4 w[kSmallPasses];
+  auto load_rhs = [&]() {
+#pragma unroll
+    for (int i = 0; i < kSmallPasses; i++) {
+      const int k = row0 + i * RP;
+      w[i] = in && k < grp.k ? ld_stream(rhs + (long long)k * grp.rhs_k[g]) : make_uint4(0, 0, 0, 0);
+    }
+  };
+  if (grp.early_rhs) load_rhs();
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (!grp.early_rhs) load_rhs();
+  float acc[M][V];
+#pragma unroll
+  for (int m = 0; m < M; m++)
+#pragma unroll
+    for (int j = 0; j < V; j++) acc[m][j] = 0.f;
+  float x[M][kSmallPasses];
+#pragma unroll
+  for (int m = 0; m < M; m++)
+#pragma unroll
+    for (int i = 0; i < kSmallPasses; i++) {
+      const int k = row0 + i * RP;
+      x[m][i] = m < grp.m && k < grp.k ? to_f(__ldcg(lhs + m * grp.lhs_m + k * grp.lhs_k)) : 0.f;
+    }
+#pragma unroll
+  for (int i = 0; i < kSmallPasses; i++) {
+    const T* e = reinterpret_cast<const T*>(&w[i]);
+#pragma unroll
+    for (int j = 0; j < V; j++) {
+      const float v = to_f(e[j]);
+#pragma unroll
+      for (int m = 0; m < M; m++) acc[m][j] = fmaf(x[m][i], v, acc[m][j]);
+    }
+  }
+  // Lanes of a warp that hold the same columns, then the eight warps.
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+#pragma unroll
+  for (int m = 0; m < M; m++)
+#pragma unroll
+    for (int j = 0; j < V; j++) {
+#pragma unroll
+      for (int o = LANES; o < 32; o <<= 1) acc[m][j] += __shfl_xor_sync(0xffffffffu, acc[m][j], o);
+      if (lane < LANES) fold[warp][m][lane * V + j] = acc[m][j];
+    }
+  __syncthreads();
+  for (int o = threadIdx.x; o < M * kSmallCols; o += kSmallThreads) {
+    const int m = o / kSmallCols, c = o % kSmallCols;
+    float v = fold[0][m][c];
+#pragma unroll
+    for (int q = 1; q < kSmallThreads / 32; q++) v += fold[q][m][c];
+    if (m < grp.m && n0 + c < grp.n[g]) static_cast<T*>(grp.out[g])[m * grp.out_m[g] + n0 + c] = from_f<T>(v);
+  }
+}
+
+template <typename T>
+int launch_small(const DotShape* shapes, int count, const void* lhs, const void* const* rhs, void* const* out, bool early_rhs, bool pdl,
+                 cudaStream_t stream) {
+  const DotShape& s = shapes[0];
+  SmallGroup grp{};
+  grp.count = count;
+  int tiles = 0;
+  for (int g = 0; g < count; g++) {
+    if ((reinterpret_cast<uintptr_t>(rhs[g]) & 15) != 0) return 0;
+    grp.tile_begin[g] = tiles;
+    tiles += (int)((shapes[g].n + kSmallCols - 1) / kSmallCols);
+    grp.rhs[g] = rhs[g];
+    grp.out[g] = out[g];
+    grp.n[g] = shapes[g].n;
+    grp.rhs_k[g] = shapes[g].rhs_k;
+    grp.out_m[g] = shapes[g].out_m;
+  }
+  for (int g = count; g <= kDotGroupMax; g++) grp.tile_begin[g] = tiles;
+  grp.m = (int)s.m;
+  grp.k = (int)s.k;
+  grp.lhs_m = s.lhs_m;
+  grp.lhs_k = s.lhs_k;
+  grp.early_rhs = early_rhs ? 1 : 0;
+  const T* a = static_cast<const T*>(lhs);
+  cudaError_t e;
+#define SMALL(MM) e = launch_kernel(small_dot_kernel<T, MM>, dim3((unsigned)tiles), dim3(kSmallThreads), 0, stream, pdl, grp, a)
+  if (s.m <= 1) SMALL(1); else if (s.m <= 2) SMALL(2); else if (s.m <= 4) SMALL(4); else SMALL(8);
+#undef SMALL
+  return e == cudaSuccess ? 1 : 0;
+}
+
 template <typename T>
 int launch_group_typed(const DotShape* shapes, int count, const DotScratch& plan, const void* lhs, const void* const* rhs,
                        void* const* out, void* partials, void* counters, bool pdl, cudaStream_t stream) {
@@ -579,6 +701,12 @@ DotScratch dot_group_plan(const DotShape* shapes, int count, int sm_count, bool 
     if (all_umma) return umma_plan(shapes, count, sm_count, 1);
   }
   if (batch == 1) {
+    // A k that one round of loads covers and at most a wave of CTAs: the kernel without rings and folds. Measured per
+    // launch, before and now: 2 x 256 x 512 bf16 7.5 / 6.2 us, 2 x 256 x 1024 bf16 7.6 / 6.5 us,
+    // 4 x 16 x 48 f32 6.5 / 4.4 us (a launch with nothing in it is about 2).
+    int64_t small_tiles = 0;
+    for (int g = 0; g < count; g++) small_tiles += (shapes[g].n + kSmallCols - 1) / kSmallCols;
+    p.small = s.k <= small_max_k(esize) && small_tiles <= sm_count ? 1 : 0;
     // Persistent TMA kernel: equal shares of (column tile, row chunk) units per CTA, two CTAs per SM with a ring of
     // 32 KiB stages each. Measured on the 8B-shape decode step (ms per step): two CTAs x 3 stages 3.50; one CTA x 5
     // stages 3.67; two CTAs x 6 stages of 16 KiB 3.94; one CTA x 6 stages of 16 KiB 4.95.
@@ -1176,6 +1304,14 @@ int dot_group_launch(const DotShape* shapes, int count, const DotScratch& plan, 
   if (count < 1 || count > kDotGroupMax) return 0;
   if (plan.umma) return launch_umma(shapes, count, plan, lhs, rhs, out, error_flag, early_rhs, pdl, stream, scales);
   if (shapes[0].rhs_s8) return 0;  // int8 weights run on the tensor-core stream only
+  if (plan.small) {
+    switch (shapes[0].dtype) {
+      case kF32: return launch_small<float>(shapes, count, lhs, rhs, out, early_rhs, pdl, stream);
+      case kF16: return launch_small<__half>(shapes, count, lhs, rhs, out, early_rhs, pdl, stream);
+      case kBF16: return launch_small<__nv_bfloat16>(shapes, count, lhs, rhs, out, early_rhs, pdl, stream);
+      default: return 0;
+    }
+  }
   if (plan.tma) {
     switch (shapes[0].dtype) {
       case kF32: return launch_tma<float>(shapes, count, plan, lhs, rhs, out, partials, counters, error_flag, early_rhs, pdl, stream);

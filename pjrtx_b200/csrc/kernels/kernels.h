@@ -93,6 +93,8 @@ struct DotScratch {
   int path = 0;
   // Path 1 without batch axes runs the TMA-fed persistent kernel (stream-K decomposition).
   int tma = 0;
+  // ... or, for a k that a CTA's registers hold, the kernel without rings and folds.
+  int small = 0;
   // Paths 1 and 4 for 16-bit floats without batch axes can run on the tensor cores (tcgen05, accumulator in TMEM); path 5
   // always does. `ksplit` CTAs of a cluster then share a tile of 128 columns x m_tile rows, contracting 1/ksplit of k each;
   // nothing goes through scratch memory.

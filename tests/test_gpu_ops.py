@@ -631,3 +631,33 @@ def test_reads_through_views_are_exact(gpu_backend, dtype, half, lead):
     got = run_backend(gpu_backend, b, [x, s])
     for g, w in zip(got, run_oracle(b, [x, s])):
         assert np.array_equal(g.view(np.uint8), w.view(np.uint8))
+
+
+@pytest.mark.parametrize("dtype,m,k,n,count", [
+    (P.F32, 1, 1, 4, 1),           # the smallest
+    (P.F32, 4, 16, 16, 3),         # one partly filled tile each, three contractions in one launch
+    (P.F32, 8, 256, 260, 1),       # the largest k and m, four columns in the last tile
+    (P.F32, 3, 255, 64, 2),        # rows that stop inside a round of loads
+    (P.BF16_CODE, 2, 512, 1024, 1),
+    (P.F16, 1, 511, 72, 1),
+])
+def test_small_contractions_against_f64(gpu_backend, dtype, m, k, n, count):
+    """Contractions whose whole k a CTA holds in registers. Error: f32 sums, and one rounding of a 16-bit output."""
+    rng = np.random.default_rng(k + n)
+    dt = P.np_dtype(dtype)
+    x = rng.standard_normal((m, k), dtype=np.float32).astype(dt)
+    ws = [rng.standard_normal((k, n + 8 * g), dtype=np.float32).astype(dt) for g in range(count)]
+    b = PlanBuilder()
+    px = b.parameter(dtype, x.shape)
+    b.set_outputs([b.dot_general(px, b.parameter(dtype, w.shape), [1], [0]) for w in ws])
+    exe = gpu_backend.compile_executable(b, [0])
+    steps = [s for s in exe.describe()["kernel_plan"]["steps"] if s["type"] == "dot"]
+    assert len(steps) == 1 and steps[0]["small"] == 1, steps
+    got, again = (run_backend(gpu_backend, b, [x] + ws, exe=exe) for _ in range(2))
+    exe.destroy()
+    ulp = {P.F32: 2.0 ** -24, P.BF16_CODE: 2.0 ** -9, P.F16: 2.0 ** -12}[dtype]
+    for g, a, w in zip(got, again, ws):
+        assert np.array_equal(g.view(np.uint8), a.view(np.uint8))
+        want = x.astype(np.float64) @ w.astype(np.float64)
+        mag = np.abs(x.astype(np.float64)) @ np.abs(w.astype(np.float64))
+        assert np.all(np.abs(g.astype(np.float64) - want) <= 2 * ulp * np.abs(want) + k * 2.0 ** -24 * mag + 2.0 ** -24)
