@@ -920,11 +920,6 @@ int64_t clusters_that_fit(int sm_count, int size, int per_sm) {
   return std::max<int64_t>(1, (int64_t)on_b200[size] * per_sm * sm_count / 148);
 }
 
-// CTAs of one launch that share an SM: two with int8 weights, whose units are a chain of copy, conversion and MMA that one
-// CTA cannot keep full. The 16-bit stream runs one (two: twice the partial sums), but in half the shared memory, so that
-// the next launch's CTA moves in, sets up and requests its first weights while this one streams.
-int umma_per_sm(int m_tile, int src) { return src == umma::kBytes && umma::tmem_columns(m_tile, 2, src) <= 256 ? 2 : 1; }
-
 // Shared memory of a CTA: half where the tensor memory of two CTAs fits and the ring still holds four stages or more.
 bool umma_half_possible(int m_tile, int ksplit, bool several_tiles, int src) {
   const int sub = src == umma::kTile ? 1 : 2, rows = (m_tile + 4 * ksplit - 1) / (4 * ksplit) * 4;
@@ -933,16 +928,20 @@ bool umma_half_possible(int m_tile, int ksplit, bool several_tiles, int src) {
              umma::kSharedSmem;
 }
 
-// Tile height, split of k and ring size with the least modelled time, in nanoseconds. The weights arrive at the HBM rate or
-// at the rate of one CTA, 16 KiB per 250 ns with the whole ring and per 305 ns with half of it (32 x 14336 x 4096 by 32 CTAs:
-// 64 and 79 us, the same for 16 to 128 rows); near the crossing the two add up softly. Tall tiles are bound by shared memory
-// (copies in and the tensor core's reads out, 128 bytes per cycle) or by the MMAs. The half ring saves about 1.5 us of
-// start-up, the cluster's sum costs about 0.6 us. Measured, us per launch in a chain at 32 rows, best against the others:
-// 4096 x 4096 4 CTAs per tile, half ring 15.5 (whole 17.6; 2 CTAs 16.8, 1 CTA 24.0); 14336 x 4096 4, whole 28.6 (half 30.8;
-// 2 CTAs 37.5); 4096 x 28672 1, whole 49.5 (half 53.5; 2 CTAs 52.4); 8192 x 57344 3 155 (2 160, 1 170).
+// Tile height, split of k, CTAs per SM and ring size with the least modelled time, in nanoseconds. The weights arrive at the
+// HBM rate or at the rate of the CTAs, 16 KiB per 250 ns with the whole ring, per 305 ns with half of it and per 400 ns where
+// two CTAs of the launch share an SM (32 x 14336 x 4096 by 32 CTAs: 64 us with the whole ring, 79 with half, the same for 16
+// to 128 rows); near the crossing the two add up softly. Tall tiles are bound by shared memory, the copies in and the tensor
+// core's reads out at about 88 bytes per cycle. One CTA per SM with half of the shared memory lets the next launch's CTA move
+// in, set up and request its first weights meanwhile, which is worth 1 to 1.5 us against two CTAs and the whole ring. The
+// cluster's sum costs about 0.6 us and the exchange of its rows. Int8 weights run two CTAs per SM wherever they fit: a unit
+// is a chain of copy, conversion and MMA that one CTA cannot keep full.
+// Measured, us per launch in a chain at 32 rows, best against the others: 4096 x 4096 4 CTAs per tile, half ring 15.4 (whole
+// 17.6; two per SM 16.5; 1 CTA per tile 24); 14336 x 4096 4, whole 28.6 (half 30.8); 4096 x 28672 1, two per SM 44.4 (whole
+// 49.3, half 53.5); 8192 x 57344 1, two per SM 150 (3 CTAs per tile 153); 28672 x 8192 4, two per SM 75.8 (2, whole 77).
 struct UmmaChoice {
   double ns = 0;
-  int m_tile = 0, ksplit = 1;
+  int m_tile = 0, ksplit = 1, per_sm = 1;
   bool half = false;
 };
 UmmaChoice umma_choose(const DotShape* shapes, int count, int sm_count, int src) {
@@ -960,23 +959,29 @@ UmmaChoice umma_choose(const DotShape* shapes, int count, int sm_count, int src)
     const int64_t tiles = n_tiles * m_tiles;
     for (int split = 1; split <= umma::kSplitMax; split++) {
       if (split > 1 && (mt > 128 || split > kblocks / 2)) break;
-      const int64_t clusters = std::min<int64_t>(tiles, clusters_that_fit(sm_count, split, umma_per_sm((int)mt, src)));
-      for (int half = 0; half < 2; half++) {
-        if (half && !umma_half_possible((int)mt, split, tiles > clusters, src)) continue;
-        if (!half && src == umma::kBytes && umma_per_sm((int)mt, src) == 2 && umma_half_possible((int)mt, split, tiles > clusters, src)) continue;
-        const double smem_ns = 2.0 * ((src == umma::kTile ? 16384 : weight_unit) + mt * 128) / 128 / 1.85;
-        const double unit_ns = std::max({smem_ns, 2.0 * mt / 1.85, src == umma::kTile && !half ? 250.0 : 305.0});
+      bool shared = false;  // two CTAs per SM are possible
+      for (int mode = 2; mode >= 0; mode--) {  // 2: two CTAs per SM, 1: half of the shared memory, 0: all of it
+        const int per_sm = mode == 2 ? 2 : 1;
+        const int64_t clusters = std::min<int64_t>(tiles, clusters_that_fit(sm_count, split, per_sm));
+        if (mode > 0 && !umma_half_possible((int)mt, split, tiles > clusters, src)) continue;
+        if (mode == 2) shared = true;
+        else if (shared && src == umma::kBytes) continue;
+        const double smem_ns = 2.9 * ((src == umma::kTile ? 16384 : weight_unit) + mt * 128) / 128 / 1.85;
+        const double unit_ns = std::max(smem_ns, src != umma::kTile ? 305.0 : mode == 0 ? 250.0 : mode == 1 ? 305.0 : 400.0);
         const double cta_ns = (double)((tiles + clusters - 1) / clusters) * (double)((kblocks + split - 1) / split) * unit_ns;
         const double hbm_ns = (double)n_tiles * kblocks * weight_unit / 6500.0;
-        const double ns = std::pow(std::pow(cta_ns, 4) + std::pow(hbm_ns, 4), 0.25) + (half ? 0 : 1500) + (split > 1 ? 600 + 8.0 * mt : 0);
-        if (best.ns == 0 || ns < best.ns * 0.99) best = UmmaChoice{ns, (int)mt, split, half != 0};
+        const double ns = std::pow(std::pow(cta_ns, 4) + std::pow(hbm_ns, 4), 0.25) + (mode == 0 ? 1500 : mode == 2 ? 1000 : 0) +
+                          (split > 1 ? 600 + 8.0 * mt : 0);
+        if (best.ns == 0 || ns < best.ns * 0.99) best = UmmaChoice{ns, (int)mt, split, per_sm, mode > 0};
       }
     }
   }
   return best;
 }
 
-// The same model for CTA pairs (umma_pair.cuh): MMAs, copies at 110 bytes per ns and SM, weights as above.
+// The same model for CTA pairs (umma_pair.cuh), whose units take 300 ns and half a nanosecond per row. Measured, us, one SM
+// per tile and pairs: 128 x 4096 x 4096 20 / 31, 128 x 4096 x 28672 87 / 59, 256 x 14336 x 4096 52 / 81, 256 x 4096 x 28672
+// 84 / 68, 517 x 4096 x 4096 40 / 34.
 double umma_pair_choose(const DotShape* shapes, int count, int sm_count, int* m_tile) {
   const DotShape& s = shapes[0];
   const int64_t kblocks = (s.k + 63) / 64;
@@ -987,7 +992,7 @@ double umma_pair_choose(const DotShape* shapes, int count, int sm_count, int* m_
     const int64_t m_tiles = (s.m + cap - 1) / cap;
     const int64_t mt = ((s.m + m_tiles - 1) / m_tiles + 31) / 32 * 32;
     const int64_t pairs = std::min<int64_t>(n_tiles * m_tiles, sm_count / 2);
-    const double unit_ns = std::max({2.0 * mt / 1.85, (16384.0 + mt * 64) / 110, 250.0});
+    const double unit_ns = 300 + 0.5 * mt;
     const double cta_ns = (double)((n_tiles * m_tiles + pairs - 1) / pairs) * kblocks * unit_ns;
     const double t = std::max(cta_ns, (double)n_tiles * umma::kPairN * s.k * 2 / 6500.0);
     if (best == 0 || t < best * 0.98) {
@@ -1022,7 +1027,7 @@ DotScratch umma_plan(const DotShape* shapes, int count, int sm_count, int kind) 
   const int64_t m_tiles = (s.m + p.m_tile - 1) / p.m_tile;
   int64_t tiles = 0;
   for (int g = 0; g < count; g++) tiles += (shapes[g].n + umma::kTileN - 1) / umma::kTileN * m_tiles;
-  const int64_t clusters = std::min<int64_t>(tiles, clusters_that_fit(sm_count, p.ksplit, umma_per_sm(p.m_tile, src)));
+  const int64_t clusters = std::min<int64_t>(tiles, clusters_that_fit(sm_count, p.ksplit, choice.per_sm));
   p.grid = (int)(clusters * p.ksplit);
   const int rows_per_rank = (p.m_tile + 4 * p.ksplit - 1) / (4 * p.ksplit) * 4;
   const size_t sum = umma::sum_bytes(p.ksplit, rows_per_rank, tiles > clusters ? 2 : 1);

@@ -582,8 +582,8 @@ def test_contractions_with_unaligned_weight_rows_against_f64(gpu_backend, dtype,
 @pytest.mark.parametrize("k_major", [False, True])
 @pytest.mark.parametrize("m,k,n,count", [
     (300, 64, 256, 1),      # one block of k, one tile of columns
-    (257, 200, 520, 1),     # ragged k; the last tile's second CTA has eight columns, the last row tile one row
-    (512, 1024, 1000, 2),   # two contractions in one launch, columns that are no multiple of 64
+    (513, 200, 4104, 1),    # ragged k; the last tile's first CTA has eight columns, its second none
+    (1024, 1024, 2024, 2),  # two contractions in one launch, columns that are no multiple of 64
     (1000, 576, 4096, 1),   # several bands of weight tiles
     (2048, 448, 2816, 1),   # several tiles per pair: both accumulators in turn, a last band that is not full
 ])
