@@ -661,3 +661,26 @@ def test_small_contractions_against_f64(gpu_backend, dtype, m, k, n, count):
         want = x.astype(np.float64) @ w.astype(np.float64)
         mag = np.abs(x.astype(np.float64)) @ np.abs(w.astype(np.float64))
         assert np.all(np.abs(g.astype(np.float64) - want) <= 2 * ulp * np.abs(want) + k * 2.0 ** -24 * mag + 2.0 ** -24)
+
+
+@pytest.mark.parametrize("cols", [4, 100, 4096, 4099])
+def test_row_argmax_with_row_maximum_edge_values(gpu_backend, cols):
+    """The column-counting maximum with index: ties, a row of the type's lowest value, infinities, and the first NaN wins;
+    the plain row maximum of the same operand in the same kernel is that reduction's value."""
+    rng = np.random.default_rng(cols)
+    x = rng.integers(-3, 4, size=(7, cols)).astype(np.float32)
+    x[1] = -np.inf
+    x[2] = 5.0
+    x[3, cols // 2:] = np.inf
+    x[4, cols - 1] = np.nan
+    x[5, cols // 3] = np.nan
+    x[5, cols - 1] = np.nan
+    x[6] = np.finfo(np.float32).min
+    b = PlanBuilder()
+    p = b.parameter(P.F32, x.shape)
+    y = b.unary("abs", p) * p
+    _, idx = b.argmax(y, 1)
+    b.set_outputs([b.reduce("reduce_sum", y, [1]), b.reduce("reduce_max", y, [1]), idx])
+    got, want = run_backend(gpu_backend, b, [x]), run_oracle(b, [x])
+    assert np.array_equal(got[2], want[2])
+    assert np.array_equal(got[1], want[1], equal_nan=True)
