@@ -454,6 +454,205 @@ inline bool sgemm_ok(const DotShape& s, const void* lhs, const void* rhs, const 
          al16(lhs) && al16(rhs) && al16(out) && (s.m + kSgBM - 1) / kSgBM <= 65535;
 }
 
+// ---------------------------------------------------------------- 64 x 64 tiles, k split over a cluster
+// out[m, n] = sum_k lhs[m, k] * rhs[k, n] in true f32, lhs k-contiguous, rhs n-contiguous, any pitch: f32 contractions that
+// do not fill the chip with the tiles of the kernel above or do not have its 16-byte rows, and 16-bit ones of pitches the
+// tensor cores cannot take, widened on the way in. Those ran one or a few CTAs through all of k with a load, a barrier and
+// a latency per slab of 16.
+// 64 x 64 outputs per CTA of 64 threads, 8 x 8 per thread, k in slabs of 16 through two shared-memory buffers; the next slab
+// travels (cp.async for f32) while the current one is multiplied. `split` CTAs of a cluster contract a slice of k each and
+// sum their tiles through distributed shared memory in rank order.
+// Measured: a call with a small ragged product 112 -> 49 us. Where 128 x 64 tiles fill the chip the kernel above is ahead
+// (1024^3 70 us against 75 here: both are bound by shared-memory reads beside the FMAs, and this one also sums four parts).
+constexpr int kSplitTile = 64, kSplitBK = 16, kSplitThreads = 64, kSplitPad = 4;
+
+__device__ __forceinline__ void cp_async(void* dst, const void* src, int bytes, bool vec) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  if (vec) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(bytes) : "memory");
+  else asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d), "l"(src), "r"(bytes) : "memory");
+}
+
+template <typename T, bool VEC>
+__global__ void __launch_bounds__(kSplitThreads, sizeof(T) == 4 ? 8 : 6)
+split_tile_kernel(DotShape s, const T* __restrict__ lhs, const T* __restrict__ rhs, T* __restrict__ out, int split) {
+  constexpr bool F32 = sizeof(T) == 4;
+  __shared__ __align__(16) float smem[2 * kSplitTile * (kSplitBK + kSplitPad) + 2 * kSplitBK * kSplitTile];
+  float (*As)[kSplitTile][kSplitBK + kSplitPad] = reinterpret_cast<float (*)[kSplitTile][kSplitBK + kSplitPad]>(smem);
+  float (*Bs)[kSplitBK][kSplitTile] = reinterpret_cast<float (*)[kSplitBK][kSplitTile]>(smem + 2 * kSplitTile * (kSplitBK + kSplitPad));
+  PJRTX_PDL_PROLOGUE();
+  const int tid = threadIdx.x, tx = tid & 7, ty = tid >> 3;
+  const int rank = (int)blockIdx.x % split;
+  const int64_t batch = blockIdx.z, b0 = batch / s.b1, b1 = batch % s.b1;
+  const T* a = lhs + b0 * s.lhs_b0 + b1 * s.lhs_b1;
+  const T* b = rhs + b0 * s.rhs_b0 + b1 * s.rhs_b1;
+  T* o = out + b0 * s.out_b0 + b1 * s.out_b1;
+  const int64_t m0 = (int64_t)blockIdx.y * kSplitTile, n0 = (int64_t)(blockIdx.x / split) * kSplitTile;
+  const int64_t slabs = (s.k + kSplitBK - 1) / kSplitBK;
+  const int64_t first = rank * slabs / split, last = (rank + 1) * slabs / split;
+
+  T ra[F32 ? 1 : 16], rb[F32 ? 1 : 16];  // 16-bit operands pass through registers
+  auto request = [&](int64_t slab, int buf) {
+    const int64_t k0 = slab * kSplitBK;
+    if constexpr (F32) {
+      if (VEC) {
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+          const int row = (tid >> 2) + 16 * i, kc = (tid & 3) * 4;  // lhs: 64 rows x 4 chunks
+          const int64_t left = m0 + row < s.m ? s.k - k0 - kc : 0;
+          cp_async(&As[buf][row][kc], left > 0 ? a + (m0 + row) * s.lhs_m + k0 + kc : a, (int)(left <= 0 ? 0 : left < 4 ? left : 4) * 4, true);
+          const int kr = (tid >> 4) + 4 * i, nc = (tid & 15) * 4;  // rhs: 16 rows x 16 chunks
+          const int64_t wide = k0 + kr < s.k ? s.n - n0 - nc : 0;
+          cp_async(&Bs[buf][kr][nc], wide > 0 ? b + (k0 + kr) * s.rhs_k + n0 + nc : b, (int)(wide <= 0 ? 0 : wide < 4 ? wide : 4) * 4, true);
+        }
+      } else {
+#pragma unroll 4
+        for (int i = 0; i < 16; i++) {
+          const int row = (tid >> 4) + 4 * i, kc = tid & 15;
+          const bool in = m0 + row < s.m && k0 + kc < s.k;
+          cp_async(&As[buf][row][kc], in ? a + (m0 + row) * s.lhs_m + k0 + kc : a, in ? 4 : 0, false);
+          const bool inb = k0 + i < s.k && n0 + tid < s.n;
+          cp_async(&Bs[buf][i][tid], inb ? b + (k0 + i) * s.rhs_k + n0 + tid : b, inb ? 4 : 0, false);
+        }
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    } else {
+#pragma unroll
+      for (int i = 0; i < 16; i++) {
+        const int row = (tid >> 4) + 4 * i, kc = tid & 15;
+        ra[i] = m0 + row < s.m && k0 + kc < s.k ? a[(m0 + row) * s.lhs_m + k0 + kc] : from_f<T>(0.f);
+        rb[i] = k0 + i < s.k && n0 + tid < s.n ? b[(k0 + i) * s.rhs_k + n0 + tid] : from_f<T>(0.f);
+      }
+    }
+  };
+  auto deposit = [&](int buf) {
+    if constexpr (!F32) {
+#pragma unroll
+      for (int i = 0; i < 16; i++) {
+        As[buf][(tid >> 4) + 4 * i][tid & 15] = to_f(ra[i]);
+        Bs[buf][i][tid] = to_f(rb[i]);
+      }
+    } else {
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+    }
+  };
+  float acc[8][8] = {};  // rows ty + 8 i, columns 32 h + 4 tx + j
+  if (first < last) {
+    request(first, 0);
+    deposit(0);
+  }
+  __syncthreads();
+  for (int64_t t = first; t < last; t++) {
+    const int buf = (int)((t - first) & 1);
+    if (t + 1 < last) request(t + 1, buf ^ 1);
+#pragma unroll
+    for (int k4 = 0; k4 < kSplitBK; k4 += 4) {
+      float4 av[8];
+#pragma unroll
+      for (int i = 0; i < 8; i++) av[i] = *reinterpret_cast<const float4*>(&As[buf][ty + 8 * i][k4]);
+#pragma unroll
+      for (int kk = 0; kk < 4; kk++) {
+        const float4 blo = *reinterpret_cast<const float4*>(&Bs[buf][k4 + kk][4 * tx]);
+        const float4 bhi = *reinterpret_cast<const float4*>(&Bs[buf][k4 + kk][32 + 4 * tx]);
+        const float bw[8] = {blo.x, blo.y, blo.z, blo.w, bhi.x, bhi.y, bhi.z, bhi.w};
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+          const float ai = kk == 0 ? av[i].x : kk == 1 ? av[i].y : kk == 2 ? av[i].z : av[i].w;
+#pragma unroll
+          for (int j = 0; j < 8; j++) acc[i][j] = fmaf(ai, bw[j], acc[i][j]);
+        }
+      }
+    }
+    if (t + 1 < last) deposit(buf ^ 1);
+    __syncthreads();
+  }
+  auto store = [&](int i, int h, float4 v) {
+    const int64_t gm = m0 + ty + 8 * i, gn = n0 + 32 * h + 4 * tx;
+    if (gm >= s.m) return;
+    T* dst = o + gm * s.out_m + gn;
+    if (VEC && F32 && gn + 3 < s.n) {
+      *reinterpret_cast<float4*>(dst) = v;
+    } else {
+      const float e[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int j = 0; j < 4; j++)
+        if (gn + j < s.n) dst[j] = from_f<T>(e[j]);
+    }
+  };
+  if (split == 1) {
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+#pragma unroll
+      for (int h = 0; h < 2; h++) store(i, h, make_float4(acc[i][4 * h], acc[i][4 * h + 1], acc[i][4 * h + 2], acc[i][4 * h + 3]));
+    return;
+  }
+  // The slabs' memory receives the cluster's tiles: [source CTA][rows i of this CTA][h][thread], once every CTA is done.
+  const int rows = 8 / split;
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+  const unsigned base = (unsigned)__cvta_generic_to_shared(smem) + (unsigned)tid * 16u;
+#pragma unroll
+  for (int i = 0; i < 8; i++) {
+    unsigned remote;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(base), "r"(i / rows));
+#pragma unroll
+    for (int h = 0; h < 2; h++)
+      asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(remote + (unsigned)(((rank * rows + i % rows) * 2 + h) * kSplitThreads * 16)),
+                   "f"(acc[i][4 * h]), "f"(acc[i][4 * h + 1]), "f"(acc[i][4 * h + 2]), "f"(acc[i][4 * h + 3])
+                   : "memory");
+  }
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+  const float4* got = reinterpret_cast<const float4*>(smem) + tid;
+  for (int r = 0; r < rows; r++)
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      float4 v = got[(r * 2 + h) * kSplitThreads];
+      for (int q = 1; q < split; q++) {
+        const float4 w = got[((q * rows + r) * 2 + h) * kSplitThreads];
+        v.x += w.x;
+        v.y += w.y;
+        v.z += w.z;
+        v.w += w.w;
+      }
+      store(rank * rows + r, h, v);
+    }
+}
+
+// True when the split-tile kernel can take the contraction as it lies in memory.
+inline bool split_tile_ok(const DotShape& s) {
+  return s.lhs_k == 1 && s.rhs_n == 1 && (s.m + kSplitTile - 1) / kSplitTile <= 65535 && (s.n + kSplitTile - 1) / kSplitTile <= (1ll << 27);
+}
+// CTAs per tile: pieces of at least 64 k, until every SM holds about seven.
+inline int split_tile_parts(const DotShape& s, int64_t batch) {
+  const int64_t tiles = (s.m + kSplitTile - 1) / kSplitTile * ((s.n + kSplitTile - 1) / kSplitTile) * batch;
+  int split = 1;
+  while (split < 8 && tiles * split < 148 * 4 && s.k / (2 * split) >= 64) split *= 2;
+  return split;
+}
+
+template <typename T>
+int launch_split_tile(const DotShape& s, const T* a, const T* b, T* o, int64_t batch, bool pdl, cudaStream_t stream) {
+  auto al16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
+  const bool vec = sizeof(T) == 4 && (s.lhs_m & 3) == 0 && (s.rhs_k & 3) == 0 && (s.out_m & 3) == 0 && (s.lhs_b0 & 3) == 0 &&
+                   (s.lhs_b1 & 3) == 0 && (s.rhs_b0 & 3) == 0 && (s.rhs_b1 & 3) == 0 && (s.out_b0 & 3) == 0 && (s.out_b1 & 3) == 0 &&
+                   al16(a) && al16(b) && al16(o);
+  const int split = split_tile_parts(s, batch);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)((s.n + kSplitTile - 1) / kSplitTile * split), (unsigned)((s.m + kSplitTile - 1) / kSplitTile), (unsigned)batch);
+  cfg.blockDim = dim3(kSplitThreads);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[3];
+  cfg.attrs = attr;
+  cfg.numAttrs = fill_launch_attributes(attr, pdl);
+  if (split > 1) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    attr[cfg.numAttrs].val.clusterDim.x = (unsigned)split;
+    attr[cfg.numAttrs].val.clusterDim.y = 1;
+    attr[cfg.numAttrs].val.clusterDim.z = 1;
+    cfg.numAttrs++;
+  }
+  if (vec) return cudaLaunchKernelEx(&cfg, split_tile_kernel<T, sizeof(T) == 4>, s, a, b, o, split) == cudaSuccess ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, split_tile_kernel<T, false>, s, a, b, o, split) == cudaSuccess ? 1 : 0;
+}
+
 // ---------------------------------------------------------------- small streaming contractions
 // out[m, n] = sum_k lhs[m, k] * rhs[k, n] for m <= 8, n contiguous and k so small (kSmallRows) that a CTA can hold its
 // whole share of the rhs in registers: toy decoders, closed-over blocks. What bounds such a contraction is the chain of
@@ -636,10 +835,13 @@ int launch_typed(const DotShape& s, const DotScratch& plan, const void* lhs, con
     return e == cudaSuccess ? 1 : 0;
   }
   if (plan.path == 3) {
-    if (sgemm_ok(s, lhs, rhs, out)) {
+    const int64_t wide_tiles = (s.n + kSgBN - 1) / kSgBN * ((s.m + kSgBM - 1) / kSgBM) * batch;
+    // 128 x 64 tiles where they fill the chip, one per SM; 64 x 64 tiles with k split over a cluster otherwise.
+    if (wide_tiles >= 112 && sgemm_ok(s, lhs, rhs, out)) {
       dim3 grid((unsigned)((s.n + kSgBN - 1) / kSgBN), (unsigned)((s.m + kSgBM - 1) / kSgBM), (unsigned)batch);
       return launch_kernel(sgemm_kernel, grid, dim3(256), 0, stream, pdl, s, (const float*)lhs, (const float*)rhs, (float*)out) == cudaSuccess ? 1 : 0;
     }
+    if (split_tile_ok(s)) return launch_split_tile<T>(s, a, b, o, batch, pdl, stream);
     dim3 grid((unsigned)((s.n + kTile - 1) / kTile), (unsigned)((s.m + kTile - 1) / kTile), (unsigned)batch);
     return launch_kernel(tile_kernel<T>, grid, dim3(256), 0, stream, pdl, s, a, b, o) == cudaSuccess ? 1 : 0;
   }
@@ -1354,7 +1556,9 @@ DotScratch dot_plan(const DotShape& s, int sm_count) {
     p.path = 2;
     return p;
   }
-  if (s.m > 8 && batches_fit && (s.m + kTile - 1) / kTile <= 65535) {
+  // Few rows of pitches the streaming kernels cannot take: tiles, unless there is too little work for one to matter.
+  const bool few = s.lhs_k == 1 && s.rhs_n == 1 && s.k >= 64 && s.n >= 64;
+  if ((s.m > 8 || few) && batches_fit && (s.m + kTile - 1) / kTile <= 65535) {
     p.path = 3;
     return p;
   }

@@ -684,3 +684,33 @@ def test_row_argmax_with_row_maximum_edge_values(gpu_backend, cols):
     got, want = run_backend(gpu_backend, b, [x]), run_oracle(b, [x])
     assert np.array_equal(got[2], want[2])
     assert np.array_equal(got[1], want[1], equal_nan=True)
+
+
+@pytest.mark.parametrize("dtype,m,k,n", [
+    (P.F32, 9, 64, 64),        # one tile
+    (P.F32, 65, 130, 68),      # ragged in every direction, 16-byte pitches for rhs only
+    (P.F32, 100, 2048, 256),   # k shared by eight CTAs
+    (P.F32, 64, 1000, 101),    # odd pitch: 4-byte copies
+    (P.F32, 3, 200, 77),       # few rows of an odd pitch
+    (P.F16, 40, 333, 129),     # 16-bit operands whose rows the tensor cores cannot take
+    (P.BF16_CODE, 5, 1001, 65),
+])
+def test_register_blocked_contractions_against_f64(gpu_backend, dtype, m, k, n):
+    """f32 (and loosely pitched 16-bit) contractions in 64 x 64 tiles with k split over a cluster: f32 sums, one rounding of
+    the output, run-to-run identical."""
+    rng = np.random.default_rng(m * k + n)
+    dt = P.np_dtype(dtype)
+    x = rng.standard_normal((m, k), dtype=np.float32).astype(dt)
+    w = rng.standard_normal((k, n), dtype=np.float32).astype(dt)
+    b = PlanBuilder()
+    b.set_outputs([b.dot_general(b.parameter(dtype, x.shape), b.parameter(dtype, w.shape), [1], [0])])
+    exe = gpu_backend.compile_executable(b, [0])
+    steps = [s for s in exe.describe()["kernel_plan"]["steps"] if s["type"] == "dot"]
+    assert len(steps) == 1 and steps[0]["path"] == 3, steps
+    got, again = (run_backend(gpu_backend, b, [x, w], exe=exe)[0] for _ in range(2))
+    exe.destroy()
+    assert np.array_equal(got.view(np.uint8), again.view(np.uint8))
+    want = x.astype(np.float64) @ w.astype(np.float64)
+    mag = np.abs(x.astype(np.float64)) @ np.abs(w.astype(np.float64))
+    ulp = {P.F32: 2.0 ** -24, P.BF16_CODE: 2.0 ** -9, P.F16: 2.0 ** -12}[dtype]
+    assert np.all(np.abs(got.astype(np.float64) - want) <= 2 * ulp * np.abs(want) + k * 2.0 ** -24 * mag + 2.0 ** -24)
