@@ -1168,7 +1168,8 @@ int launch_prefill_tiles(const AttnPrefillShape& s, const umma::AttnParams& p, c
   constexpr size_t smem = umma::attn_smem_bytes(HD, TILES);
   if (!raise_smem_limit((const void*)umma::umma_attention_kernel<BF16, HD, TILES>, (int)smem)) return 0;
   const dim3 grid((unsigned)((p.rows + umma::kAttnRows * TILES - 1) / (umma::kAttnRows * TILES)), (unsigned)s.kv_heads, (unsigned)s.batch);
-  return launch_kernel(umma::umma_attention_kernel<BF16, HD, TILES>, grid, dim3(128 * TILES + 64), smem, stream, pdl, p, qmap, kmap, vmap,
+  (void)pdl;  // fully ordered after its predecessor: it takes all of an SM's tensor memory
+  return launch_kernel(umma::umma_attention_kernel<BF16, HD, TILES>, grid, dim3(128 * TILES + 64), smem, stream, /*pdl=*/false, p, qmap, kmap, vmap,
                        out) == cudaSuccess
              ? 1
              : 0;

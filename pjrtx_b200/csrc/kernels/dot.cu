@@ -1254,7 +1254,7 @@ int launch_umma_sub(const umma::Params& prm, const umma::Maps& maps, const DotSc
   cfg.stream = stream;
   cudaLaunchAttribute attr[3];
   cfg.attrs = attr;
-  cfg.numAttrs = fill_launch_attributes(attr, pdl);
+  cfg.numAttrs = fill_launch_attributes(attr, pdl && SRC != umma::kLoose);  // (kLoose: ordered like the pairs below)
   if (plan.ksplit > 1) {
     attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
     attr[cfg.numAttrs].val.clusterDim.x = (unsigned)plan.ksplit;
@@ -1265,7 +1265,7 @@ int launch_umma_sub(const umma::Params& prm, const umma::Maps& maps, const DotSc
   return cudaLaunchKernelEx(&cfg, umma::umma_stream_kernel<SUB, SRC>, prm, maps) == cudaSuccess ? 1 : 0;
 }
 
-int launch_umma_pair(const umma::PairParams& prm, const umma::Maps& maps, const DotScratch& plan, bool pdl, cudaStream_t stream) {
+int launch_umma_pair(const umma::PairParams& prm, const umma::Maps& maps, const DotScratch& plan, cudaStream_t stream) {
   if (!raise_smem_limit((const void*)umma::umma_pair_kernel, 227 * 1024)) return 0;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)plan.grid);
@@ -1274,7 +1274,9 @@ int launch_umma_pair(const umma::PairParams& prm, const umma::Maps& maps, const 
   cfg.stream = stream;
   cudaLaunchAttribute attr[3];
   cfg.attrs = attr;
-  cfg.numAttrs = fill_launch_attributes(attr, pdl);
+  // Fully ordered after its predecessor: kernels that take most of an SM's tensor memory never start beside one that is
+  // leaving (a prefill step with such overlaps did not finish).
+  cfg.numAttrs = fill_launch_attributes(attr, false);
   attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
   attr[cfg.numAttrs].val.clusterDim.x = 2;
   attr[cfg.numAttrs].val.clusterDim.y = 1;
@@ -1396,7 +1398,7 @@ int launch_umma(const DotShape* shapes, int count, const DotScratch& plan, const
     q.rhs_3d = p.rhs_3d;
     q.early_rhs = early_rhs ? 1 : 0;
     q.error_flag = error_flag;
-    return launch_umma_pair(q, maps, plan, pdl, stream);
+    return launch_umma_pair(q, maps, plan, stream);
   }
   p.tiles = tiles;
   p.ksplit = plan.ksplit;

@@ -290,7 +290,11 @@ __global__ void __launch_bounds__(kBaseThreads, 1) umma_pair_kernel(const PairPa
     __syncwarp();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(tmem_cols) : "memory");
+    __syncwarp();
   }
+  // The pair frees its tensor memory as one: neither CTA leaves its SM to a successor's CTA, whose allocation would be
+  // waiting for these columns, before both have freed them.
+  cluster_sync();
 }
 
 }  // namespace umma
