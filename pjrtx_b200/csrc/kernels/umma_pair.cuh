@@ -136,15 +136,21 @@ __global__ void __launch_bounds__(kBaseThreads, 1) umma_pair_kernel(const PairPa
     flags[0] = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  // The paired allocation is collective: its warp may issue it only once the peer CTA is known to have launched, and the
+  // peer has to stay until the paired free has completed (the last barrier of the kernel). CTAs of a cluster are scheduled
+  // together, but nothing else says that the peer already runs. The same barrier publishes the mbarriers.
+  cluster_sync();
   if (warp == 5) {
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(tmem_cols) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  cluster_sync();  // both CTAs have their barriers and tensor memory
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  // This CTA has its tensor memory: the MMA warp waits for the peer's word before the first MMA, which writes both CTAs'
+  // columns, everybody else at the exit.
+  asm volatile("barrier.cluster.arrive.release;" ::: "memory");
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 4) {
@@ -203,6 +209,8 @@ __global__ void __launch_bounds__(kBaseThreads, 1) umma_pair_kernel(const PairPa
     }
   } else if (warp == 5) {
     // ---- MMA issuer (leader) -----------------------------------------------------------------------------------------
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+    __syncwarp();
     if (rank == 0 && lane == 0) {
       // M = 256: twice the single-CTA instruction's.
       const uint32_t idesc = instr_desc(p.is_bf16, p.m_tile, !p.rhs_k_major) + ((uint32_t)(kTileN >> 4) << 24);
@@ -285,6 +293,7 @@ __global__ void __launch_bounds__(kBaseThreads, 1) umma_pair_kernel(const PairPa
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   }
   __syncwarp();
+  if (warp != 5) asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
   cluster_sync();  // nobody frees or leaves while the peer may still write here
   if (warp == 5) {
     __syncwarp();
@@ -292,8 +301,7 @@ __global__ void __launch_bounds__(kBaseThreads, 1) umma_pair_kernel(const PairPa
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(tmem_cols) : "memory");
     __syncwarp();
   }
-  // The pair frees its tensor memory as one: neither CTA leaves its SM to a successor's CTA, whose allocation would be
-  // waiting for these columns, before both have freed them.
+  // The paired free is collective too: neither CTA leaves before both have issued it.
   cluster_sync();
 }
 

@@ -120,6 +120,33 @@ def test_tiny_prefill(gpu_backend):
     assert outs[0].to_numpy().shape == (batch,)
 
 
+def test_prefill_on_cta_pairs_many_times(gpu_backend):
+    """CTA pairs between the prefill attention, the cluster-split stream and the unaligned head, pass after pass: paired
+    tensor memory is allocated and freed beside CTAs that come and go. Parity of the first pass, equal bits in every other."""
+    import dataclasses
+
+    be = gpu_backend
+    cfg = dataclasses.replace(llama.TINY, layers=3, d_model=512, heads=4, head_dim=128, ffn=1792, vocab=1001, dtype=P.F16)
+    batch, seq = 4, 177
+    builder, names = llama.build_prefill(cfg, batch, seq, return_logits=True)
+    weights = llama.make_weights(cfg, seed=0)
+    tokens = np.random.default_rng(3).integers(0, cfg.vocab, size=(batch, seq), dtype=np.int32)
+    args = [tokens] + [weights[n] for n in names[1:]]
+    exe = be.compile_executable(builder, [0])
+    steps = exe.describe()["kernel_plan"]["steps"]
+    dots = [s for s in steps if s["type"] == "dot"]
+    assert any(s["pair"] for s in dots) and any(s["ksplit"] > 1 for s in dots) and any(s["path"] == 5 for s in dots)
+    assert [s["type"] for s in steps].count("attention_prefill") == cfg.layers
+    bufs = [be.buffer_from_host(a) for a in args]
+    first = be.execute_executable(exe, bufs)[1].to_numpy()
+    assert_close(first, run_oracle(builder, args)[1], 2e-2, what="prefill logits")
+    for _ in range(10):
+        for _ in range(9):
+            be.execute_executable(exe, bufs)
+        again = be.execute_executable(exe, bufs)[1].to_numpy()
+        assert np.array_equal(first.view(np.uint16), again.view(np.uint16))
+
+
 @pytest.mark.parametrize("batch,dtype", [(2, P.BF16_CODE), (16, P.BF16_CODE), (5, P.BF16_CODE), (16, P.F16)])
 def test_int8_weight_only_decode(gpu_backend, monkeypatch, batch, dtype):
     """Dequantisation written as convert + multiply feeding dot_general. From three rows up the contractions read the
