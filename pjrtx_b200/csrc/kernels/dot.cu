@@ -1224,6 +1224,8 @@ DotScratch umma_plan(const DotShape* shapes, int count, int sm_count, int kind) 
     p.grid = 2 * (int)std::min<int64_t>(tiles, sm_count / 2);
     p.stages = (int)std::min<size_t>(12, (227 * 1024 - 1024 - umma::kBarrierBytes) / umma::pair_stage_bytes(pair_tile));
     p.smem = umma::pair_smem_bytes(p.stages, pair_tile);
+    p.tmem = (int)umma::tmem_columns(pair_tile, 1, umma::kTile);
+    p.ordered = 1;
     return p;
   }
   const int64_t m_tiles = (s.m + p.m_tile - 1) / p.m_tile;
@@ -1241,6 +1243,11 @@ DotScratch umma_plan(const DotShape* shapes, int count, int sm_count, int kind) 
   p.sub = src != umma::kTile || (deep_units >= 16 && ring_budget / umma::stage_bytes(p.m_tile, 2, src) >= 4) ? 2 : 1;
   p.stages = (int)std::max<size_t>(2, std::min<size_t>(12, ring_budget / umma::stage_bytes(p.m_tile, p.sub, src)));
   p.smem = umma::smem_bytes(p.stages, p.m_tile, p.sub, src, sum);
+  p.tmem = (int)umma::tmem_columns(p.m_tile, p.sub, src);
+  // Launches that take more than half of an SM's tensor memory start after their predecessor has completed, like pairs and
+  // the prefill attention: one prefill that had such kernels start beside leaving ones did not finish, and what stopped it
+  // was not observed. Unaligned rows took part in it and are ordered at any size.
+  p.ordered = p.tmem > 256 || src == umma::kLoose ? 1 : 0;
   return p;
 }
 
@@ -1254,7 +1261,7 @@ int launch_umma_sub(const umma::Params& prm, const umma::Maps& maps, const DotSc
   cfg.stream = stream;
   cudaLaunchAttribute attr[3];
   cfg.attrs = attr;
-  cfg.numAttrs = fill_launch_attributes(attr, pdl && SRC != umma::kLoose);  // (kLoose: ordered like the pairs below)
+  cfg.numAttrs = fill_launch_attributes(attr, pdl && !plan.ordered);
   if (plan.ksplit > 1) {
     attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
     attr[cfg.numAttrs].val.clusterDim.x = (unsigned)plan.ksplit;
@@ -1274,9 +1281,7 @@ int launch_umma_pair(const umma::PairParams& prm, const umma::Maps& maps, const 
   cfg.stream = stream;
   cudaLaunchAttribute attr[3];
   cfg.attrs = attr;
-  // Fully ordered after its predecessor: kernels that take most of an SM's tensor memory never start beside one that is
-  // leaving (a prefill step with such overlaps did not finish).
-  cfg.numAttrs = fill_launch_attributes(attr, false);
+  cfg.numAttrs = fill_launch_attributes(attr, false);  // (plan.ordered)
   attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
   attr[cfg.numAttrs].val.clusterDim.x = 2;
   attr[cfg.numAttrs].val.clusterDim.y = 1;

@@ -100,6 +100,9 @@ struct DotScratch {
   // nothing goes through scratch memory.
   // `pair`: CTA pairs work on tiles of 256 columns (umma_pair.cuh).
   int umma = 0, m_tile = 0, sub = 1, pair = 0;
+  // Tensor-memory columns of a CTA, and whether the launch waits for its predecessor to complete whatever the stream's
+  // setting for programmatic dependent launch.
+  int tmem = 0, ordered = 0;
   int grid = 0, stages = 0, max_contrib = 0;
   long long per_cta = 0;
   uint64_t smem = 0;

@@ -26,8 +26,8 @@
 // warp-level kernel before this one (mma.sync, 64 rows per CTA) 627 us, this one 241 us; 1 x 517 positions 24 and 14 us.
 //
 // Row tiles are scheduled longest first. Waits are bounded by time (code 8 is reported); dependents are released after the
-// tensor-memory allocation, and a CTA asks for more than half of the shared memory so that nothing else that allocates
-// tensor memory shares its SM.
+// tensor-memory allocation, and a CTA asks for so much of the shared memory that nothing else that allocates tensor memory
+// fits beside it (least_smem).
 #pragma once
 
 #include "umma_gemm.cuh"
@@ -50,7 +50,8 @@ struct AttnParams {
 __host__ __device__ constexpr int attn_slot_bytes(int hd) { return kAttnKeys * hd * 2; }
 __host__ __device__ constexpr size_t attn_smem_bytes(int hd, int tiles) {
   const size_t bytes = (size_t)tiles * kAttnRows * hd * 2 + (size_t)kAttnSlots * attn_slot_bytes(hd) + 512 + 1024;
-  return bytes < 120 * 1024 ? 120 * 1024 : bytes;
+  const size_t least = least_smem(512);
+  return bytes < least ? least : bytes;
 }
 
 __device__ __forceinline__ void tma_load_4d(uint32_t smem_dst, const CUtensorMap* map, int x, int y, int z, int w, uint64_t* bar) {

@@ -292,15 +292,17 @@ __host__ __device__ inline uint32_t tmem_columns(int m_tile, int sub, int src) {
   while (cols < 2u * m_tile + (src == kTile ? 0u : kOperandSlots * 32u * sub)) cols <<= 1;
   return cols;
 }
-// An SM's tensor memory (512 columns) must hold the allocations of all CTAs that fit its shared memory: a CTA whose
-// allocation blocks could keep its cluster waiting. At most 256 columns: two CTAs (at least 80 KiB each, at most
-// kSharedSmem). More: one CTA (at least 120 KiB).
+// An SM's tensor memory (512 columns) must hold the allocations of all CTAs that fit its shared memory (228 KiB, 1 KiB of
+// it per CTA reserved), whichever kernels they belong to: a CTA whose allocation blocks could keep its cluster waiting. A
+// CTA of at most 256 columns asks for at least 80 KiB (two fit, three do not; kSharedSmem is the most two can have), one of
+// more columns for at least 150 KiB (nothing else that allocates tensor memory fits beside it).
 constexpr size_t kSharedSmem = 113 * 1024;
+__host__ __device__ constexpr size_t least_smem(uint32_t tmem_cols) { return (tmem_cols <= 256 ? 80 : 150) * 1024; }
 inline size_t smem_bytes(int stages, int m_tile, int sub, int src, size_t sum) {
   // stages (every block 1024-byte aligned: m_tile is a multiple of 16, so m_tile * 128 is a multiple of 2048) +
   // receive buffers + barriers and flags + slack for aligning the dynamic segment to 1024 bytes.
   const size_t bytes = (size_t)stages * stage_bytes(m_tile, sub, src) + sum + kBarrierBytes + 1024;
-  const size_t least = (tmem_columns(m_tile, sub, src) <= 256 ? 80 : 120) * 1024;
+  const size_t least = least_smem(tmem_columns(m_tile, sub, src));
   return bytes < least ? least : bytes;
 }
 

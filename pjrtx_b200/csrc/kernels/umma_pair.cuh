@@ -50,9 +50,8 @@ struct PairParams {
 
 __host__ __device__ inline size_t pair_stage_bytes(int m_tile) { return 16384 + (size_t)m_tile * 64; }
 inline size_t pair_smem_bytes(int stages, int m_tile) {
-  // Never less than 120 KiB: the allocation takes up to all 512 columns of the SM's tensor memory.
   const size_t bytes = stages * pair_stage_bytes(m_tile) + kBarrierBytes + 1024;
-  return bytes < 120 * 1024 ? 120 * 1024 : bytes;
+  return bytes < least_smem(512) ? least_smem(512) : bytes;
 }
 
 // Copies of a CTA pair: the data lands in the executing CTA, `bar` may be the peer's mbarrier (a shared::cluster address).
@@ -121,8 +120,7 @@ __global__ void __launch_bounds__(kBaseThreads, 1) umma_pair_kernel(const PairPa
   const int tiles = p.m_tiles * p.n_tiles;
   const int my_tiles = pair < tiles ? (tiles - 1 - pair) / pairs + 1 : 0;
   const int count = my_tiles * p.kblocks;
-  uint32_t tmem_cols = 32;
-  while (tmem_cols < 2u * p.m_tile) tmem_cols <<= 1;
+  const uint32_t tmem_cols = tmem_columns(p.m_tile, 1, kTile);  // two accumulators, as there
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < p.stages; s++) {

@@ -373,3 +373,38 @@ def test_decode_attention_kernel_choice_and_grid(backend, monkeypatch):
     monkeypatch.setenv("PJRTX_B200_ATTENTION_MMA", "0")
     st = plan_of(P.BF16_CODE, 1, 32, 8, 128, 3744)
     assert st["mma"] == 0 and st["splits"] == 18
+
+
+def _contraction(backend, source, m, k, n, group=1):
+    """The planned step of a 16-bit contraction: weights that tensor maps can describe, int8 weights, or rows of odd pitch."""
+    b = PlanBuilder()
+    x = b.parameter(P.BF16_CODE, [m, k])
+    outs = []
+    for _ in range(group):
+        if source == "int8":
+            w = b.convert(b.convert(b.parameter(P.S8, [k, n]), P.F16) * b.broadcast_in_dim(b.parameter(P.F16, [n]), [k, n], [1]), P.BF16_CODE)
+        else:
+            w = b.parameter(P.BF16_CODE, [k, n + (source == "loose")])
+        outs.append(b.dot_general(x, w, [1], [0]))
+    b.set_outputs(outs)
+    steps = [s for s in backend.describe_kernels(b)["steps"] if s["type"] == "dot"]
+    assert all(s["umma"] == 1 and s["rhs_s8"] == (source == "int8") for s in steps), (source, m, k, n)
+    return steps
+
+
+TENSOR_SIZES = [(m, k, n) for m in (3, 16, 40, 48, 64, 96, 112, 113, 128, 129, 200, 256, 384, 640, 800, 2048)
+                for k, n in ((128, 128), (512, 2048), (4096, 4096), (4096, 6144), (4096, 28672), (14336, 4096), (4096, 128256))]
+
+
+@pytest.mark.parametrize("source", ["tile", "int8", "loose"])
+def test_tensor_memory_of_an_sm_is_never_oversubscribed(backend, source):
+    """CTAs that fit an SM's 228 KiB of shared memory together (1 KiB each reserved) fit its 512 tensor-memory columns
+    too, and launches of more than half of them wait for their predecessor."""
+    for m, k, n in TENSOR_SIZES:
+        for st in _contraction(backend, source, m, k, n):
+            assert st["tmem"] in (32, 64, 128, 256, 512), st
+            if st["tmem"] > 256:
+                assert st["ordered"] == 1 and st["smem"] + 1024 > (228 - 81) * 1024, st
+            else:
+                assert 3 * (st["smem"] + 1024) > 228 * 1024, st
+            assert st["ordered"] == 1 or (source != "loose" and not st["pair"]), st
