@@ -1122,12 +1122,14 @@ int64_t clusters_that_fit(int sm_count, int size, int per_sm) {
   return std::max<int64_t>(1, (int64_t)on_b200[size] * per_sm * sm_count / 148);
 }
 
-// Shared memory of a CTA: half where the tensor memory of two CTAs fits and the ring still holds four stages or more.
-bool umma_half_possible(int m_tile, int ksplit, bool several_tiles, int src) {
+// Whether the receive buffers of the cluster's sum and a ring worth running fit a CTA's shared memory: all of it, where two
+// stages have to fit (tall int8 tiles split over three CTAs and more leave less than that: 128 rows over three 135 KiB of
+// receive buffers beside stages of 48 KiB), or half of it where the tensor memory of two CTAs fits, with four stages.
+bool umma_fits(int m_tile, int ksplit, bool several_tiles, int src, bool half) {
   const int sub = src == umma::kTile ? 1 : 2, rows = (m_tile + 4 * ksplit - 1) / (4 * ksplit) * 4;
-  return src != umma::kLoose && umma::tmem_columns(m_tile, sub, src) <= 256 &&
-         umma::sum_bytes(ksplit, rows, several_tiles ? 2 : 1) + 4 * umma::stage_bytes(m_tile, sub, src) + umma::kBarrierBytes + 1024 <=
-             umma::kSharedSmem;
+  if (half && (src == umma::kLoose || umma::tmem_columns(m_tile, sub, src) > 256)) return false;
+  return umma::sum_bytes(ksplit, rows, several_tiles ? 2 : 1) + (half ? 4 : 2) * umma::stage_bytes(m_tile, sub, src) + umma::kBarrierBytes + 1024 <=
+         (half ? umma::kSharedSmem : 227 * 1024);
 }
 
 // Tile height, split of k, CTAs per SM and ring size with the least modelled time, in nanoseconds. The weights arrive at the
@@ -1165,7 +1167,7 @@ UmmaChoice umma_choose(const DotShape* shapes, int count, int sm_count, int src)
       for (int mode = 2; mode >= 0; mode--) {  // 2: two CTAs per SM, 1: half of the shared memory, 0: all of it
         const int per_sm = mode == 2 ? 2 : 1;
         const int64_t clusters = std::min<int64_t>(tiles, clusters_that_fit(sm_count, split, per_sm));
-        if (mode > 0 && !umma_half_possible((int)mt, split, tiles > clusters, src)) continue;
+        if (!umma_fits((int)mt, split, tiles > clusters, src, mode > 0)) continue;
         if (mode == 2) shared = true;
         else if (shared && src == umma::kBytes) continue;
         const double smem_ns = 2.9 * ((src == umma::kTile ? 16384 : weight_unit) + mt * 128) / 128 / 1.85;
@@ -1241,7 +1243,7 @@ DotScratch umma_plan(const DotShape* shapes, int count, int sm_count, int kind) 
   // hand-overs between copies, converters and the MMA lane (int8, 8B-width layers at 32 rows: 1.54 against 1.25 ms).
   const int64_t deep_units = (tiles + clusters - 1) / clusters * ((s.k + 127) / 128) / p.ksplit;
   p.sub = src != umma::kTile || (deep_units >= 16 && ring_budget / umma::stage_bytes(p.m_tile, 2, src) >= 4) ? 2 : 1;
-  p.stages = (int)std::max<size_t>(2, std::min<size_t>(12, ring_budget / umma::stage_bytes(p.m_tile, p.sub, src)));
+  p.stages = (int)std::min<size_t>(12, ring_budget / umma::stage_bytes(p.m_tile, p.sub, src));  // two or more (umma_fits)
   p.smem = umma::smem_bytes(p.stages, p.m_tile, p.sub, src, sum);
   p.tmem = (int)umma::tmem_columns(p.m_tile, p.sub, src);
   // Launches that take more than half of an SM's tensor memory start after their predecessor has completed, like pairs and

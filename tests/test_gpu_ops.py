@@ -517,6 +517,40 @@ def test_int8_dequantising_contraction(gpu_backend, m, k, n, dtype):
     assert np.max(np.abs(got - want)) <= bound, (np.max(np.abs(got - want)), np.max(np.abs(want)))
 
 
+@pytest.mark.parametrize("m,k,n,count,dtype", [
+    (113, 4096, 6144, 1, P.BF16_CODE),  # the shortest tile of 128 rows
+    (128, 4096, 7168, 2, P.F16),        # two stages of the ring beside the receive buffers
+    (384, 2048, 2048, 1, P.BF16_CODE),  # several tiles of rows
+    (800, 4096, 4096, 1, P.BF16_CODE),  # several tiles per cluster: two receive buffers
+])
+def test_int8_contractions_of_tall_tiles_against_f64(gpu_backend, m, k, n, count, dtype):
+    """Int8 weights under tiles of up to 128 rows whose k a cluster shares. Error: the f32 sums (2^-24 of the summed
+    magnitudes per addition, at most k of them) and one rounding of the output."""
+    rng = np.random.default_rng(m + n)
+    x = rng.standard_normal((m, k), dtype=np.float32).astype(P.np_dtype(dtype))
+    b, args, outs, ws = PlanBuilder(), [x], [], []
+    px = b.parameter(dtype, x.shape)
+    for _ in range(count):
+        w = rng.integers(-127, 128, size=(k, n), dtype=np.int8)
+        sc = (rng.uniform(0.5, 1.5, size=(n,)) / 127 / np.sqrt(k)).astype(np.float16)
+        wf = b.convert(b.parameter(P.S8, w.shape), P.F16) * b.broadcast_in_dim(b.parameter(P.F16, sc.shape), w.shape, [1])
+        outs.append(b.dot_general(px, wf if dtype == P.F16 else b.convert(wf, dtype), [1], [0]))
+        args += [w, sc]
+        ws.append(w.astype(np.float64) * sc.astype(np.float64))
+    b.set_outputs(outs)
+    exe = gpu_backend.compile_executable(b, [0])
+    dots = [s for s in exe.describe()["kernel_plan"]["steps"] if s["type"] == "dot"]
+    assert len(dots) == 1 and dots[0]["rhs_s8"] == 1 and dots[0]["group"] == count, dots
+    got, again = (run_backend(gpu_backend, b, args, exe=exe) for _ in range(2))
+    exe.destroy()
+    ulp = 2.0 ** (-9 if dtype == P.BF16_CODE else -12)
+    x64 = x.astype(np.float64)
+    for g, a, w in zip(got, again, ws):
+        assert np.array_equal(g.view(np.uint16), a.view(np.uint16))
+        want, mag = x64 @ w, np.abs(x64) @ np.abs(w)
+        assert np.all(np.abs(g.astype(np.float64) - want) <= 2 * ulp * np.abs(want) + k * 2.0 ** -24 * mag + 2.0 ** -24)
+
+
 @pytest.mark.parametrize("dtype", [P.BF16_CODE, P.F16])
 @pytest.mark.parametrize("m,k,n,count", [
     (3, 128, 128, 1),      # one tile, two 64-deep blocks

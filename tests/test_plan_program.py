@@ -408,3 +408,15 @@ def test_tensor_memory_of_an_sm_is_never_oversubscribed(backend, source):
             else:
                 assert 3 * (st["smem"] + 1024) > 228 * 1024, st
             assert st["ordered"] == 1 or (source != "loose" and not st["pair"]), st
+
+
+@pytest.mark.parametrize("source", ["tile", "int8", "loose"])
+def test_every_planned_contraction_fits_an_sm(backend, source):
+    """Ring, receive buffers of the cluster's sum and barriers within the 227 KiB a CTA can have, at least two stages in the
+    ring, a block of k for every CTA of a cluster."""
+    rows = sorted({m for m, _, _ in TENSOR_SIZES} | set(range(97, 131, 5)) | {560, 561, 785, 896, 1000, 4096})
+    widths = [(128, 128), (128, 4096), (512, 2048), (2048, 2048), (4096, 1024), (4096, 4096), (4096, 6144), (8192, 28672), (14336, 4096)]
+    for m in rows:
+        for k, n in widths + [(4096, 14336)]:
+            for st in _contraction(backend, source, m, k, n, group=2 if n == 14336 else 1):
+                assert st["smem"] <= 227 * 1024 and st["stages"] >= 2 and st["ksplit"] <= (k + 127) // 128, st
