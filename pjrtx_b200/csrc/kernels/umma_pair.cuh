@@ -184,7 +184,7 @@ __global__ void __launch_bounds__(kBaseThreads, 1) umma_pair_kernel(const PairPa
       for (int i = 0; i < count; i++) {
         if (i >= first) {
           if (i >= p.stages && !mbar_wait(&empty[stage], phase ^ 1, budget)) {
-            atomicExch(p.error_flag, 21);
+            atomicExch(p.error_flag, 17);
             // The copies in flight get time to land before the pair leaves.
             const unsigned long long until = global_timer_ns() + 50000;
             while (global_timer_ns() < until) {
@@ -218,14 +218,14 @@ __global__ void __launch_bounds__(kBaseThreads, 1) umma_pair_kernel(const PairPa
       for (int seg = 0; seg < my_tiles && ok; seg++) {
         const int buf = seg & 1;
         if (seg >= 2 && !cluster_wait(&acc_empty[buf], ((seg >> 1) & 1) ^ 1, budget)) {
-          atomicExch(p.error_flag, 24);
+          atomicExch(p.error_flag, 20);
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t acc = tmem_base + (uint32_t)(buf * p.m_tile);
         for (int kb = 0; kb < p.kblocks; kb++) {
           if (!cluster_wait(&full[stage], phase, budget)) {
-            atomicExch(p.error_flag, 22);
+            atomicExch(p.error_flag, 18);
             ok = false;
             break;
           }
@@ -253,7 +253,7 @@ __global__ void __launch_bounds__(kBaseThreads, 1) umma_pair_kernel(const PairPa
       const PairTile t = locate_pair_tile(p, pair + seg * pairs);
       const int buf = seg & 1;
       if (!epilogue_all(mbar_wait(&acc_full[buf], (seg >> 1) & 1, budget))) {
-        if (threadIdx.x == 0) atomicExch(p.error_flag, 23);
+        if (threadIdx.x == 0) atomicExch(p.error_flag, 19);
         break;
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");

@@ -420,3 +420,15 @@ def test_every_planned_contraction_fits_an_sm(backend, source):
         for k, n in widths + [(4096, 14336)]:
             for st in _contraction(backend, source, m, k, n, group=2 if n == 14336 else 1):
                 assert st["smem"] <= 227 * 1024 and st["stages"] >= 2 and st["ksplit"] <= (k + 127) // 128, st
+
+
+def test_error_word_codes_belong_to_one_kernel_each():
+    """A caller drops its peers on code 21, so no local wait may raise it; the same for every other code."""
+    kernels = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "pjrtx_b200", "csrc", "kernels")
+    where = {}
+    for name in sorted(os.listdir(kernels)):
+        with open(os.path.join(kernels, name)) as f:
+            for code in re.findall(r"atomicExch\([\w.]*error_flag, (\d+)\)", f.read()):
+                where.setdefault(int(code), set()).add(name)
+    assert where[21] == {"peer_reduce.cu"} and where[31] == {"dot.cu"}
+    assert all(len(files) == 1 for files in where.values()), where
