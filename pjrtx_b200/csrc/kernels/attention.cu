@@ -1322,7 +1322,7 @@ int attn_decode_launch(const AttnDecodeShape& s, const AttnDecodePlan& plan, con
     if (coop_merge_allowed() && plan.mma != 1 && plan.splits > 1 && cudaGetDevice(&device) == cudaSuccess &&
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) == cudaSuccess)
       a.coop_merge = (long long)plan.splits * s.kv_heads * s.batch <= sms ? 1 : 0;
-    a.timeout_ns = 2000000000ull;
+    a.timeout_ns = wait_timeout_ns();
   }
   if (plan.mma == 1 && ((reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v)) & 15) != 0) return 0;  // bulk copies of rows
   if (plan.mma == 2) {
@@ -1363,6 +1363,7 @@ int attn_prefill_launch(const AttnPrefillShape& s, const void* q, const void* k,
   p.scale_log2 = s.scale == 0.f ? 1.f : fabsf(s.scale) * 1.4426950408889634f;
   p.is_bf16 = s.dtype == kBF16;
   p.error_flag = error_flag;
+  p.timeout_ns = wait_timeout_ns();
   if (s.dtype == kBF16)
     return s.head_dim == 128 ? launch_prefill<true, 128>(s, p, q, k, v, out, pdl, stream) : launch_prefill<true, 64>(s, p, q, k, v, out, pdl, stream);
   return s.head_dim == 128 ? launch_prefill<false, 128>(s, p, q, k, v, out, pdl, stream) : launch_prefill<false, 64>(s, p, q, k, v, out, pdl, stream);

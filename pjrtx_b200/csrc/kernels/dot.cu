@@ -862,9 +862,9 @@ int tma_env_int(const char* name, int fallback) {
   const char* v = getenv(name);
   return v && *v ? atoi(v) : fallback;
 }
+}  // namespace
 
-// Budget of one launch for all of its device-side waits (PJRTX_B200_WAIT_TIMEOUT_MS, two seconds by default).
-unsigned long long tma_timeout_ns() {
+unsigned long long wait_timeout_ns() {
   static const unsigned long long ns = [] {
     const int ms = tma_env_int("PJRTX_B200_WAIT_TIMEOUT_MS", 2000);
     return (unsigned long long)(ms < 1 ? 1 : ms) * 1000000ull;
@@ -872,6 +872,7 @@ unsigned long long tma_timeout_ns() {
   return ns;
 }
 
+namespace {
 // Ring depth and CTAs per SM of the TMA streaming kernel: two CTAs per SM with three 32 KiB stages each while the
 // cross-warp fold buffer is small (m <= 2 for 16-bit types), one CTA with a deeper ring otherwise.
 void tma_ring(int M, int V, int* stages, int* per_sm) {
@@ -1023,7 +1024,7 @@ template <typename T>
 int launch_tma_params(tma::Params& p, const tma::Maps& maps, int m, int grid, int stages, size_t smem, int* error_flag,
                       bool early_rhs, bool pdl, cudaStream_t stream) {
   p.error_flag = error_flag;
-  p.timeout_ns = tma_timeout_ns();
+  p.timeout_ns = wait_timeout_ns();
   p.stages = stages;
   p.early_rhs = early_rhs ? 1 : 0;
   static const int env_evict = tma_env_int("PJRTX_B200_TMA_EVICT_FIRST", 1);
@@ -1405,6 +1406,7 @@ int launch_umma(const DotShape* shapes, int count, const DotScratch& plan, const
     q.rhs_3d = p.rhs_3d;
     q.early_rhs = early_rhs ? 1 : 0;
     q.error_flag = error_flag;
+    q.timeout_ns = wait_timeout_ns();
     return launch_umma_pair(q, maps, plan, stream);
   }
   p.tiles = tiles;
@@ -1412,6 +1414,7 @@ int launch_umma(const DotShape* shapes, int count, const DotScratch& plan, const
   p.rows_per_rank = (plan.m_tile + 4 * plan.ksplit - 1) / (4 * plan.ksplit) * 4;
   p.sum_buffers = tiles > plan.grid / plan.ksplit ? 2 : 1;
   p.error_flag = error_flag;
+  p.timeout_ns = wait_timeout_ns();
   p.stages = plan.stages;
   p.is_bf16 = s.dtype == kBF16;
   p.rhs_k_major = k_major ? 1 : 0;

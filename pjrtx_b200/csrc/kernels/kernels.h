@@ -183,6 +183,10 @@ int stream_dot_static_scratch(int device, int dtype, const void* lhs, const void
 // (1) or gave up a bounded device-side wait (0 with last_error set). Allocates nothing.
 int stream_dot_static_scratch_status(int device, cudaStream_t stream);
 
+// Budget of one launch for all of its device-side waits, counted from its start (PJRTX_B200_WAIT_TIMEOUT_MS, read once;
+// two seconds by default).
+unsigned long long wait_timeout_ns();
+
 // Self-test of the bounded device-side waits: one CTA waits (with the wait the streaming kernels use) for an mbarrier
 // that nothing completes, gives up after `timeout_ms` (1..1000) and raises `error_flag` with code 31. The kernel
 // returns normally; nothing faults or hangs.

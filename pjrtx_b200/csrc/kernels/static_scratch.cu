@@ -125,7 +125,7 @@ int launch(const DotShape& s, const DotScratch& plan, const void* lhs, const voi
   sg.partials = reinterpret_cast<float*>(scratch);
   sg.counters = reinterpret_cast<unsigned*>(scratch + kStaticPartialBytes);
   p.error_flag = reinterpret_cast<int*>(scratch + kStaticPartialBytes + kStaticCounterBytes);
-  p.timeout_ns = tma::kDefaultTimeoutNs;
+  p.timeout_ns = wait_timeout_ns();
   p.stages = plan.stages;
   p.early_rhs = 0;
   p.evict_first = 1;

@@ -59,7 +59,6 @@ constexpr int kStageBytes = kUnitRows * kTileBytes;  // 32 KiB
 constexpr int kConsumerWarps = 8;
 constexpr int kConsumers = kConsumerWarps * 32;
 constexpr int kThreads = (kConsumerWarps + 1) * 32;
-constexpr unsigned long long kDefaultTimeoutNs = 2000000000ull;  // budget of one launch for all of its waits
 
 enum LhsKind { kLhsPlain = 0, kLhsRmsNorm = 1, kLhsSiluMul = 2 };
 

@@ -45,6 +45,7 @@ struct AttnParams {
   float sign;        // 1, -1 or 0: what the scores are multiplied by first, so that the largest score has the largest exponent
   int is_bf16;
   int* error_flag;
+  unsigned long long timeout_ns;
 };
 
 __host__ __device__ constexpr int attn_slot_bytes(int hd) { return kAttnKeys * hd * 2; }
@@ -117,7 +118,7 @@ umma_attention_kernel(const AttnParams p, const __grid_constant__ CUtensorMap qm
   uint64_t* o_full = p_ready + TILES;             // [TILES] the last product has completed
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_full + TILES);
   int* flags = reinterpret_cast<int*>(tmem_slot + 1);  // [0] abort
-  const WaitBudget budget{global_timer_ns() + kTimeoutNs, flags};
+  const WaitBudget budget{global_timer_ns() + p.timeout_ns, flags};
   constexpr uint32_t kTmemCols = TILES == 2 ? 512 : 256;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;

@@ -53,10 +53,11 @@
 // Dependents are released only after the tensor-memory allocation: a successor's CTA that moved in first could
 // otherwise take the tensor memory this one is about to ask for and then wait for this grid.
 //
-// Every mbarrier wait is bounded by time (two seconds per launch; the thread that sees the deadline pass sets a CTA-wide
+// Every mbarrier wait is bounded by time (`timeout_ns` per launch, two seconds by default; the thread that sees the deadline pass sets a CTA-wide
 // abort word and every other wait gives up at its next check); the kernel then sets *error_flag, every role falls
 // through to the common exit, the allocating warp frees its tensor memory, and the kernel returns. CTAs of a cluster
-// leave together, so nobody writes into the shared memory of a CTA that is gone.
+// leave together, so nobody writes into the shared memory of a CTA that is gone. Cluster barriers have no limit of their own:
+// like __syncthreads they end because every way to them is bounded.
 #pragma once
 
 #include <cuda.h>
@@ -73,7 +74,6 @@ constexpr int kTileN = 128;          // weight columns per tile (MMA M)
 constexpr int kSubK = 64;            // k elements per swizzle row (128 bytes of 16-bit data)
 constexpr int kSplitMax = 8;         // CTAs of a cluster (the portable limit)
 constexpr int kBaseThreads = 192;    // warps 0-3 epilogue, warp 4 TMA producer, warp 5 MMA issuer
-constexpr unsigned long long kTimeoutNs = 2000000000ull;  // budget of one launch for all of its waits
 
 enum Source { kTile = 0, kBytes = 1, kLoose = 2 };
 // Converter warps (from warp 6 on): four per quarter of the 128 columns where the loads come from global memory (the
@@ -98,6 +98,7 @@ struct Params {
   int rows_per_rank;     // m_tile / ksplit, rounded up to a multiple of 4: rows of a tile that one CTA of the cluster finishes
   int sum_buffers;       // 1 or 2 (a cluster with several tiles): receive buffers for the cluster's sum
   int* error_flag;
+  unsigned long long timeout_ns;  // budget of the launch for all of its waits
   int stages;
   int is_bf16;
   int rhs_k_major;       // 1: rhs is [n, k] with k contiguous
@@ -384,7 +385,7 @@ __global__ void __launch_bounds__(threads_of(SRC), SRC == kLoose ? 1 : 2) umma_s
   uint64_t* slot_empty = ready + kOperandSlots;  // [kOperandSlots] the MMAs that read the slot have completed
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(slot_empty + kOperandSlots);
   int* flags = reinterpret_cast<int*>(tmem_slot + 1);  // [0] abort
-  const WaitBudget budget{global_timer_ns() + kTimeoutNs, flags};
+  const WaitBudget budget{global_timer_ns() + p.timeout_ns, flags};
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int ksplit = p.ksplit;

@@ -46,6 +46,7 @@ struct PairParams {
   int is_bf16;
   int rhs_k_major, rhs_3d, early_rhs;
   int* error_flag;
+  unsigned long long timeout_ns;
 };
 
 __host__ __device__ inline size_t pair_stage_bytes(int m_tile) { return 16384 + (size_t)m_tile * 64; }
@@ -113,7 +114,7 @@ __global__ void __launch_bounds__(kBaseThreads, 1) umma_pair_kernel(const PairPa
   uint64_t* acc_empty = acc_full + 2;     // [2]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
   int* flags = reinterpret_cast<int*>(tmem_slot + 1);  // [0] abort
-  const WaitBudget budget{global_timer_ns() + kTimeoutNs, flags};
+  const WaitBudget budget{global_timer_ns() + p.timeout_ns, flags};
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = (int)blockIdx.x & 1, pair = (int)blockIdx.x >> 1, pairs = (int)gridDim.x >> 1;

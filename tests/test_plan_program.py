@@ -432,3 +432,15 @@ def test_error_word_codes_belong_to_one_kernel_each():
                 where.setdefault(int(code), set()).add(name)
     assert where[21] == {"peer_reduce.cu"} and where[31] == {"dot.cu"}
     assert all(len(files) == 1 for files in where.values()), where
+
+
+def test_every_device_side_wait_takes_its_budget_from_the_launch():
+    """PJRTX_B200_WAIT_TIMEOUT_MS holds for every kernel: no budget is a constant of the device code."""
+    kernels = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "pjrtx_b200", "csrc", "kernels")
+    budgets = []
+    for name in sorted(os.listdir(kernels)):
+        with open(os.path.join(kernels, name)) as f:
+            text = f.read()
+        budgets += [(name, b) for b in re.findall(r"WaitBudget budget\{[\w:]*global_timer_ns\(\) \+ ([\w.]+),", text)]
+        assert not re.search(r"imeout_?ns\w* = \d", text, re.I), name
+    assert len(budgets) == 5 and all(b.endswith("timeout_ns") for _, b in budgets), budgets
