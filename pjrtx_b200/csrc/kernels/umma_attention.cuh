@@ -16,8 +16,10 @@
 // Tensor memory: S_t (128 columns, its first 64 reused for P_t) and O_t (head_dim columns) per tile.
 //
 // O is rescaled only when a row's maximum has grown by more than 2^8 since the scale in use was chosen: until then the
-// probabilities are relative to the older maximum (at most 256, exact in every type involved, as the common factor cancels
-// in the division by the row sum), and the round trip of O through registers is saved. The row sum is kept in f32.
+// probabilities are relative to the older maximum (at most 256, in range for every type involved; the common factor cancels
+// in the division by the row sum), and the round trip of O through registers is saved. The row sum is kept in f32 and is taken
+// of the probabilities as the second product reads them, rounded to the element type, so that their rounding cancels where
+// few keys carry a row: with equal values under all keys the result is that value.
 // A block's S is complete only after the product O += P . V issued before it (one commit covers both), so a softmax thread
 // that has seen S may touch O.
 //
@@ -96,6 +98,22 @@ __device__ __forceinline__ uint32_t pack_pair(float lo, float hi) {
   }
   const __half2 v = __floats2half2_rn(lo, hi);
   return *reinterpret_cast<const uint32_t*>(&v);
+}
+
+// Adds the two elements of a packed pair to two f32 sums (mixed-precision additions, exact in the 16-bit operand).
+// 4 x 2048 positions, 32 heads of 128 over 8: 201 us in bf16 and f16; widening first 201 and 208; sums of the unrounded
+// probabilities 199 and 199.
+template <bool BF16>
+__device__ __forceinline__ void add_pair(uint32_t pair, float& lo, float& hi) {
+  unsigned short l, h;
+  asm("mov.b32 {%0, %1}, %2;" : "=h"(l), "=h"(h) : "r"(pair));
+  if (BF16) {
+    asm("add.rn.f32.bf16 %0, %1, %0;" : "+f"(lo) : "h"(l));
+    asm("add.rn.f32.bf16 %0, %1, %0;" : "+f"(hi) : "h"(h));
+  } else {
+    asm("add.rn.f32.f16 %0, %1, %0;" : "+f"(lo) : "h"(l));
+    asm("add.rn.f32.f16 %0, %1, %0;" : "+f"(hi) : "h"(h));
+  }
 }
 
 template <bool BF16, int HD, int TILES>
@@ -305,9 +323,9 @@ umma_attention_kernel(const AttnParams p, const __grid_constant__ CUtensorMap qm
         for (int e = 0; e < 32; e++) {
           const float x = exp2_approx(fmaf(s[c * 64 + 2 * e], p.scale_log2, shift));
           const float y = exp2_approx(fmaf(s[c * 64 + 2 * e + 1], p.scale_log2, shift));
-          part[(2 * e) & 3] += x;
-          part[(2 * e + 1) & 3] += y;
-          packed[e] = __uint_as_float(pack_pair<BF16>(x, y));
+          const uint32_t pair = pack_pair<BF16>(x, y);
+          add_pair<BF16>(pair, part[(2 * e) & 3], part[(2 * e + 1) & 3]);
+          packed[e] = __uint_as_float(pair);
         }
         tmem_store_32(s_addr + c * 32, packed);
       }

@@ -461,6 +461,19 @@ def test_prefill_attention_against_f64(gpu_backend, dtype, batch, kv_heads, rep,
     assert np.max(np.abs(got - want)) <= 3 * ulp * np.max(np.abs(v64))
 
 
+@pytest.mark.parametrize("dtype,hd,seq,spread", [(P.BF16_CODE, 128, 300, 3.0), (P.F16, 64, 700, 3.0), (P.BF16_CODE, 64, 130, 1.0)])
+def test_prefill_attention_weights_sum_to_one(gpu_backend, dtype, hd, seq, spread):
+    """Where all keys have one value, every row's result is that value: the row sum is taken of the probabilities as the
+    second product reads them (rounded to the element type), so their rounding cancels. What is left, f32 sums of at most
+    `seq` terms (2^-24 each), is far below half a unit in the last place of the element type."""
+    b, (q, k, v) = cases.prefill_attention(dtype=dtype, batch=2, kv_heads=4, rep=4, seq=seq, head_dim=hd)
+    q = (q.astype(np.float32) * spread).astype(q.dtype)
+    v[:] = np.linspace(1.0, 2.0, hd, endpoint=False, dtype=np.float32).astype(v.dtype)
+    got = run_backend(gpu_backend, b, [q, k, v])[0]
+    want = np.broadcast_to(v[0, 0, 0], got.shape)
+    assert np.array_equal(got.view(np.uint16), np.ascontiguousarray(want).view(np.uint16))
+
+
 def test_prefill_attention_same_as_written_chain(gpu_backend, monkeypatch):
     """The kernel and the unfused chain (dot -> softmax row kernel -> dot) agree within the 16-bit tolerance."""
     b, args = cases.prefill_attention(seq=150, rep=4, head_dim=128)
