@@ -1302,7 +1302,9 @@ class Gen {
         if (counting) {
           const auto& dims = val(ins->inputs[1]).dims;
           counting = !dims.empty() && dims.back() == C_ && prod(ins->inputs[1]).scalar("iota_dimension", 0) == (int64_t)dims.size() - 1 &&
-                     dtype_is_int(val(ins->inputs[1]).dtype);
+                     dtype_is_int(val(ins->inputs[1]).dtype) &&
+                     // (an index that wraps round does not ascend)
+                     C_ <= (int64_t)1 << std::min<int64_t>(62, (int64_t)dtype_size(val(ins->inputs[1]).dtype) * 8 - 1);
         }
         counts_columns.push_back(counting);
         if (counting) {

@@ -680,6 +680,19 @@ def test_reads_through_views_are_exact(gpu_backend, dtype, half, lead):
         assert np.array_equal(g.view(np.uint8), w.view(np.uint8))
 
 
+@pytest.mark.parametrize("index,cols", [(P.S16, 32768), (P.S16, 40000), (P.U16, 70000)])
+def test_argmax_ties_where_the_index_type_wraps_round(gpu_backend, index, cols):
+    """Rows wider than the index type counts: among equal maxima the smallest index operand wins, also where a later column
+    has it."""
+    x = np.zeros((2, cols), np.float32)
+    x[0, [4103, cols - 1 - (cols - 1 - 4103) % 4096]] = 1.0  # two columns of one thread
+    x[1, ::1024] = 2.0
+    b = PlanBuilder()
+    b.set_outputs(list(b.argmax(b.parameter(P.F32, x.shape), 1, index)))
+    got, want = run_backend(gpu_backend, b, [x]), run_oracle(b, [x])
+    assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1]), (got[1], want[1])
+
+
 @pytest.mark.parametrize("dtype,m,k,n,count", [
     (P.F32, 1, 1, 4, 1),           # the smallest
     (P.F32, 4, 16, 16, 3),         # one partly filled tile each, three contractions in one launch
