@@ -1164,11 +1164,10 @@ bool encode_query_map(CUtensorMap* map, const void* base, bool f16, long long ro
 
 template <bool BF16, int HD, int TILES>
 int launch_prefill_tiles(const AttnPrefillShape& s, const umma::AttnParams& p, const CUtensorMap& qmap, const CUtensorMap& kmap,
-                         const CUtensorMap& vmap, void* out, bool pdl, cudaStream_t stream) {
+                         const CUtensorMap& vmap, void* out, cudaStream_t stream) {
   constexpr size_t smem = umma::attn_smem_bytes(HD, TILES);
   if (!raise_smem_limit((const void*)umma::umma_attention_kernel<BF16, HD, TILES>, (int)smem)) return 0;
   const dim3 grid((unsigned)((p.rows + umma::kAttnRows * TILES - 1) / (umma::kAttnRows * TILES)), (unsigned)s.kv_heads, (unsigned)s.batch);
-  (void)pdl;  // fully ordered after its predecessor: it takes all of an SM's tensor memory
   return launch_kernel(umma::umma_attention_kernel<BF16, HD, TILES>, grid, dim3(128 * TILES + 64), smem, stream, /*pdl=*/false, p, qmap, kmap, vmap,
                        out) == cudaSuccess
              ? 1
@@ -1176,7 +1175,7 @@ int launch_prefill_tiles(const AttnPrefillShape& s, const umma::AttnParams& p, c
 }
 
 template <bool BF16, int HD>
-int launch_prefill(const AttnPrefillShape& s, const umma::AttnParams& p, const void* q, const void* k, const void* v, void* out, bool pdl,
+int launch_prefill(const AttnPrefillShape& s, const umma::AttnParams& p, const void* q, const void* k, const void* v, void* out,
                    cudaStream_t stream) {
   if (((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) |
         reinterpret_cast<uintptr_t>(out)) & 15) != 0)
@@ -1198,8 +1197,8 @@ int launch_prefill(const AttnPrefillShape& s, const umma::AttnParams& p, const v
   int device = 0, sms = 148;
   if (cudaGetDevice(&device) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
   const long long pairs = (p.rows + 2 * umma::kAttnRows - 1) / (2 * umma::kAttnRows) * s.kv_heads * s.batch;
-  return pairs >= sms ? launch_prefill_tiles<BF16, HD, 2>(s, p, qmap, kmap, vmap, out, pdl, stream)
-                      : launch_prefill_tiles<BF16, HD, 1>(s, p, qmap, kmap, vmap, out, pdl, stream);
+  return pairs >= sms ? launch_prefill_tiles<BF16, HD, 2>(s, p, qmap, kmap, vmap, out, stream)
+                      : launch_prefill_tiles<BF16, HD, 1>(s, p, qmap, kmap, vmap, out, stream);
 }
 
 }  // namespace
@@ -1352,7 +1351,7 @@ bool attn_prefill_supported(const AttnPrefillShape& s) {
   return true;
 }
 
-int attn_prefill_launch(const AttnPrefillShape& s, const void* q, const void* k, const void* v, void* out, bool pdl,
+int attn_prefill_launch(const AttnPrefillShape& s, const void* q, const void* k, const void* v, void* out,
                         cudaStream_t stream, int* error_flag) {
   if (!attn_prefill_supported(s)) return 0;
   umma::AttnParams p;
@@ -1361,12 +1360,11 @@ int attn_prefill_launch(const AttnPrefillShape& s, const void* q, const void* k,
   p.kv_heads = (int)s.kv_heads;
   p.sign = s.scale > 0.f ? 1.f : s.scale < 0.f ? -1.f : 0.f;
   p.scale_log2 = s.scale == 0.f ? 1.f : fabsf(s.scale) * 1.4426950408889634f;
-  p.is_bf16 = s.dtype == kBF16;
   p.error_flag = error_flag;
   p.timeout_ns = wait_timeout_ns();
   if (s.dtype == kBF16)
-    return s.head_dim == 128 ? launch_prefill<true, 128>(s, p, q, k, v, out, pdl, stream) : launch_prefill<true, 64>(s, p, q, k, v, out, pdl, stream);
-  return s.head_dim == 128 ? launch_prefill<false, 128>(s, p, q, k, v, out, pdl, stream) : launch_prefill<false, 64>(s, p, q, k, v, out, pdl, stream);
+    return s.head_dim == 128 ? launch_prefill<true, 128>(s, p, q, k, v, out, stream) : launch_prefill<true, 64>(s, p, q, k, v, out, stream);
+  return s.head_dim == 128 ? launch_prefill<false, 128>(s, p, q, k, v, out, stream) : launch_prefill<false, 64>(s, p, q, k, v, out, stream);
 }
 
 }  // namespace pjrtx

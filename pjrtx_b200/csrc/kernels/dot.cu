@@ -1,6 +1,6 @@
 // dot_general kernels for sm_100a.
 //
-// Four paths behind one canonical contraction out[b0,b1,m,n] = sum_k lhs*rhs
+// The kernels behind one canonical contraction out[b0,b1,m,n] = sum_k lhs*rhs
 // (the reference reaches MLX matmul/tensordot for the same op,
 // src/backend/mlx_metal/api.cc:3349-3498; its generated kernels are the
 // one-thread-per-output and 256-thread tiled dots of
@@ -8,16 +8,21 @@
 //   1  stream_kn : m <= 8, rhs[K,N] with N contiguous. Bandwidth-bound GEMV /
 //                  skinny GEMM: 16-byte loads of rhs rows, f32 accumulators in
 //                  registers, K split over warps and CTAs, deterministic
-//                  last-CTA fold of the f32 partials.
+//                  last-CTA fold of the f32 partials. Without batch axes: the
+//                  TMA-fed persistent kernel (stream_tma.cuh), or small_dot_kernel
+//                  for a k that one round of loads covers.
 //   2  stream_nk : m <= 8, rhs[N,K] with K contiguous (attention scores, tied
 //                  heads): lane groups own output columns and shuffle-reduce.
-//   3  tile      : shared-memory tiled FFMA contraction with f32 accumulate,
-//                  any strides (f32 matmul at 1e-5 needs real FFMA, not TF32).
+//   3  tile      : shared-memory tiled FFMA contraction with f32 accumulate
+//                  (f32 matmul at 1e-5 needs real FFMA, not TF32): 128 x 64
+//                  tiles, 64 x 64 tiles with k split over a cluster, or 64 x 64
+//                  tiles for any strides.
 //   0  generic   : one thread per output element, any strides, any m.
 // 16-bit floats without batch axes whose operands a TMA tensor map can describe run on the tensor cores instead
-// (umma_gemm.cuh): rhs[K,N] as a variant of path 1 (so that q/k/v and gate/up still share one launch), rhs[N,K] as
-// path 4. PJRTX_B200_UMMA=0 turns that off; PJRTX_B200_UMMA_MIN_M (default 3: measured on the
-// 8B decode shapes the CUDA-core kernel is ahead for one and two rows only) keeps the CUDA-core streaming kernels below that m.
+// (umma_gemm.cuh, CTA pairs: umma_pair.cuh): rhs[K,N] as a variant of path 1 (so that q/k/v and gate/up still share one
+// launch), rhs[N,K] as path 4, rhs[K,N] rows that a tensor map cannot describe as path 5. PJRTX_B200_UMMA=0 turns that off; PJRTX_B200_UMMA_MIN_M (default 3: the CUDA-core
+// kernel was ahead for one and two rows on the 8B decode shapes, measured before the cluster-split stream and not again since)
+// keeps the CUDA-core streaming kernels below that m.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -620,21 +625,25 @@ split_tile_kernel(DotShape s, const T* __restrict__ lhs, const T* __restrict__ r
 inline bool split_tile_ok(const DotShape& s) {
   return s.lhs_k == 1 && s.rhs_n == 1 && (s.m + kSplitTile - 1) / kSplitTile <= 65535 && (s.n + kSplitTile - 1) / kSplitTile <= (1ll << 27);
 }
-// CTAs per tile: pieces of at least 64 k, until every SM holds about seven.
-inline int split_tile_parts(const DotShape& s, int64_t batch) {
+// CTAs per tile: pieces of at least 64 k, doubled until there are four CTAs for every SM (four to seven then).
+inline int split_tile_parts(const DotShape& s, int64_t batch, int sm_count) {
   const int64_t tiles = (s.m + kSplitTile - 1) / kSplitTile * ((s.n + kSplitTile - 1) / kSplitTile) * batch;
   int split = 1;
-  while (split < 8 && tiles * split < 148 * 4 && s.k / (2 * split) >= 64) split *= 2;
+  while (split < 8 && tiles * split < (int64_t)sm_count * 4 && s.k / (2 * split) >= 64) split *= 2;
   return split;
+}
+// 128 x 64 tiles (sgemm_kernel, where its 16-byte rows apply) for more than three quarters of the SMs: they run one CTA per
+// SM. One point was measured, 1024^3 with 128 tiles: 70 us against 75 on split tiles; where the two cross was not.
+inline bool wide_tiles_fill(const DotShape& s, int64_t batch, int sm_count) {
+  return (s.n + kSgBN - 1) / kSgBN * ((s.m + kSgBM - 1) / kSgBM) * batch > sm_count * 3 / 4;
 }
 
 template <typename T>
-int launch_split_tile(const DotShape& s, const T* a, const T* b, T* o, int64_t batch, bool pdl, cudaStream_t stream) {
+int launch_split_tile(const DotShape& s, const T* a, const T* b, T* o, int64_t batch, int split, bool pdl, cudaStream_t stream) {
   auto al16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
   const bool vec = sizeof(T) == 4 && (s.lhs_m & 3) == 0 && (s.rhs_k & 3) == 0 && (s.out_m & 3) == 0 && (s.lhs_b0 & 3) == 0 &&
                    (s.lhs_b1 & 3) == 0 && (s.rhs_b0 & 3) == 0 && (s.rhs_b1 & 3) == 0 && (s.out_b0 & 3) == 0 && (s.out_b1 & 3) == 0 &&
                    al16(a) && al16(b) && al16(o);
-  const int split = split_tile_parts(s, batch);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)((s.n + kSplitTile - 1) / kSplitTile * split), (unsigned)((s.m + kSplitTile - 1) / kSplitTile), (unsigned)batch);
   cfg.blockDim = dim3(kSplitThreads);
@@ -654,7 +663,7 @@ int launch_split_tile(const DotShape& s, const T* a, const T* b, T* o, int64_t b
 }
 
 // ---------------------------------------------------------------- small streaming contractions
-// out[m, n] = sum_k lhs[m, k] * rhs[k, n] for m <= 8, n contiguous and k so small (kSmallRows) that a CTA can hold its
+// out[m, n] = sum_k lhs[m, k] * rhs[k, n] for m <= 8, n contiguous and k so small (small_max_k) that a CTA can hold its
 // whole share of the rhs in registers: toy decoders, closed-over blocks. What bounds such a contraction is the chain of
 // dependent latencies, not bytes. The persistent kernel's chain is tensor map -> copy -> mbarrier -> partial sums in global
 // memory -> arrival counter -> fold; here a CTA owns 64 columns for all of k, requests every 16-byte piece of its weights
@@ -835,13 +844,11 @@ int launch_typed(const DotShape& s, const DotScratch& plan, const void* lhs, con
     return e == cudaSuccess ? 1 : 0;
   }
   if (plan.path == 3) {
-    const int64_t wide_tiles = (s.n + kSgBN - 1) / kSgBN * ((s.m + kSgBM - 1) / kSgBM) * batch;
-    // 128 x 64 tiles where they fill the chip, one per SM; 64 x 64 tiles with k split over a cluster otherwise.
-    if (wide_tiles >= 112 && sgemm_ok(s, lhs, rhs, out)) {
+    if (plan.wide && sgemm_ok(s, lhs, rhs, out)) {
       dim3 grid((unsigned)((s.n + kSgBN - 1) / kSgBN), (unsigned)((s.m + kSgBM - 1) / kSgBM), (unsigned)batch);
       return launch_kernel(sgemm_kernel, grid, dim3(256), 0, stream, pdl, s, (const float*)lhs, (const float*)rhs, (float*)out) == cudaSuccess ? 1 : 0;
     }
-    if (split_tile_ok(s)) return launch_split_tile<T>(s, a, b, o, batch, pdl, stream);
+    if (split_tile_ok(s)) return launch_split_tile<T>(s, a, b, o, batch, plan.ksplit, pdl, stream);
     dim3 grid((unsigned)((s.n + kTile - 1) / kTile), (unsigned)((s.m + kTile - 1) / kTile), (unsigned)batch);
     return launch_kernel(tile_kernel<T>, grid, dim3(256), 0, stream, pdl, s, a, b, o) == cudaSuccess ? 1 : 0;
   }
@@ -858,7 +865,7 @@ DotScratch umma_plan(const DotShape* shapes, int count, int sm_count, int kind);
 }  // namespace
 
 namespace {
-int tma_env_int(const char* name, int fallback) {
+int env_int(const char* name, int fallback) {
   const char* v = getenv(name);
   return v && *v ? atoi(v) : fallback;
 }
@@ -866,7 +873,7 @@ int tma_env_int(const char* name, int fallback) {
 
 unsigned long long wait_timeout_ns() {
   static const unsigned long long ns = [] {
-    const int ms = tma_env_int("PJRTX_B200_WAIT_TIMEOUT_MS", 2000);
+    const int ms = env_int("PJRTX_B200_WAIT_TIMEOUT_MS", 2000);
     return (unsigned long long)(ms < 1 ? 1 : ms) * 1000000ull;
   }();
   return ns;
@@ -880,7 +887,7 @@ void tma_ring(int M, int V, int* stages, int* per_sm) {
   const bool two = red <= 16 * 1024;
   *per_sm = two ? 2 : 1;
   *stages = two ? 3 : (M <= 4 ? 5 : 4);
-  static const int env_stages = tma_env_int("PJRTX_B200_TMA_STAGES", 0);
+  static const int env_stages = env_int("PJRTX_B200_TMA_STAGES", 0);
   if (env_stages >= 2 && env_stages <= 6) *stages = env_stages;
 }
 }  // namespace
@@ -909,11 +916,15 @@ DotScratch dot_group_plan(const DotShape* shapes, int count, int sm_count, bool 
     // 4 x 16 x 48 f32 6.5 / 4.4 us (a launch with nothing in it is about 2).
     int64_t small_tiles = 0;
     for (int g = 0; g < count; g++) small_tiles += (shapes[g].n + kSmallCols - 1) / kSmallCols;
-    p.small = s.k <= small_max_k(esize) && small_tiles <= sm_count ? 1 : 0;
     // Persistent TMA kernel: equal shares of (column tile, row chunk) units per CTA, two CTAs per SM with a ring of
     // 32 KiB stages each. Measured on the 8B-shape decode step (ms per step): two CTAs x 3 stages 3.50; one CTA x 5
     // stages 3.67; two CTAs x 6 stages of 16 KiB 3.94; one CTA x 6 stages of 16 KiB 4.95.
     p.tma = 1;
+    if (allow_tensor && s.k <= small_max_k(esize) && small_tiles <= sm_count) {
+      p.small = 1;
+      p.grid = (int)small_tiles;
+      return p;
+    }
     const int chunks = (int)((s.k + tma::kUnitRows - 1) / tma::kUnitRows);
     const int64_t units = tiles * chunks;
     int per_sm = 1;
@@ -1027,7 +1038,7 @@ int launch_tma_params(tma::Params& p, const tma::Maps& maps, int m, int grid, in
   p.timeout_ns = wait_timeout_ns();
   p.stages = stages;
   p.early_rhs = early_rhs ? 1 : 0;
-  static const int env_evict = tma_env_int("PJRTX_B200_TMA_EVICT_FIRST", 1);
+  static const int env_evict = env_int("PJRTX_B200_TMA_EVICT_FIRST", 1);
   p.evict_first = env_evict;
   const int M = m <= 1 ? 1 : m <= 2 ? 2 : m <= 4 ? 4 : 8;
   // The plain contraction (one segment, untransformed lhs, no residual) runs the kernel without the segment machinery.
@@ -1084,11 +1095,6 @@ int launch_chain(const DotChainSegment* segs, const DotChainArgs* args, int n, c
 
 
 // ---- tensor-core stream (umma_gemm.cuh) ---------------------------------------------------------------------------
-
-int env_int(const char* name, int fallback) {
-  const char* v = getenv(name);
-  return v && *v ? atoi(v) : fallback;
-}
 
 // 0: not eligible, 1: rhs[K,N] with N contiguous, 2: rhs[N,K] with K contiguous, 3: rhs[K,N] with N contiguous whose rows
 // the tensor maps cannot describe. Tensor maps need 16-byte multiples for every row stride; lhs must be k-contiguous.
@@ -1387,7 +1393,6 @@ int launch_umma(const DotShape* shapes, int count, const DotScratch& plan, const
   if (plan.pair) {
     umma::PairParams q{};
     q.m = p.m;
-    q.k = p.k;
     q.m_tile = p.m_tile;
     q.m_tiles = p.m_tiles;
     q.count = count;
@@ -1404,7 +1409,6 @@ int launch_umma(const DotShape* shapes, int count, const DotScratch& plan, const
     q.is_bf16 = s.dtype == kBF16;
     q.rhs_k_major = k_major ? 1 : 0;
     q.rhs_3d = p.rhs_3d;
-    q.early_rhs = early_rhs ? 1 : 0;
     q.error_flag = error_flag;
     q.timeout_ns = wait_timeout_ns();
     return launch_umma_pair(q, maps, plan, stream);
@@ -1572,6 +1576,8 @@ DotScratch dot_plan(const DotShape& s, int sm_count) {
   const bool few = s.lhs_k == 1 && s.rhs_n == 1 && s.k >= 64 && s.n >= 64;
   if ((s.m > 8 || few) && batches_fit && (s.m + kTile - 1) / kTile <= 65535) {
     p.path = 3;
+    p.wide = wide_tiles_fill(s, batch, sm_count) ? 1 : 0;
+    p.ksplit = split_tile_parts(s, batch, sm_count);
     return p;
   }
   p.path = 0;

@@ -95,6 +95,9 @@ struct DotScratch {
   int tma = 0;
   // ... or, for a k that a CTA's registers hold, the kernel without rings and folds.
   int small = 0;
+  // Path 3: 128 x 64 tiles fill the chip; otherwise (and where their 16-byte rows do not apply) `ksplit` CTAs of a cluster
+  // share a tile of 64 x 64.
+  int wide = 0;
   // Paths 1 and 4 for 16-bit floats without batch axes can run on the tensor cores (tcgen05, accumulator in TMEM); path 5
   // always does. `ksplit` CTAs of a cluster then share a tile of 128 columns x m_tile rows, contracting 1/ksplit of k each;
   // nothing goes through scratch memory.
@@ -247,7 +250,8 @@ int attn_decode_launch(const AttnDecodeShape& s, const AttnDecodePlan& plan, con
 
 // Causal self-attention over whole sequences (prefill) as one tensor-core kernel. q / out: [batch, kv_heads, seq, rep,
 // head_dim] contiguous (query head = kv head * rep + r); k / v: [batch, seq, kv_heads, head_dim] through the strides;
-// position s sees keys 0..s. q.k is rounded to the element type before it is scaled, as the explicit dot_general does.
+// position s sees keys 0..s. Scores stay in f32, where the written program rounds q.k to the element type before it scales.
+// The launch is always ordered after its predecessor.
 struct AttnPrefillShape {
   int dtype = 0;
   long long batch = 1, kv_heads = 1, rep = 1, seq = 1, head_dim = 1;
@@ -255,7 +259,7 @@ struct AttnPrefillShape {
   float scale = 1.f;
 };
 bool attn_prefill_supported(const AttnPrefillShape& s);
-int attn_prefill_launch(const AttnPrefillShape& s, const void* q, const void* k, const void* v, void* out, bool pdl,
+int attn_prefill_launch(const AttnPrefillShape& s, const void* q, const void* k, const void* v, void* out,
                         cudaStream_t stream, int* error_flag = nullptr);
 
 // All-reduce (sum) over peer-mapped regions, one launch per rank (kernels/peer_reduce.cu). `regions[r]` is rank r's

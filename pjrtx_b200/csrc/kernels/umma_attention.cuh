@@ -27,7 +27,7 @@
 // cycle), which overlap between the two tiles. Measured for 4 x 2048 positions, 32 query heads of 128 over 8 KV heads: the
 // warp-level kernel before this one (mma.sync, 64 rows per CTA) 627 us, this one 241 us; 1 x 517 positions 24 and 14 us.
 //
-// Row tiles are scheduled longest first. Waits are bounded by time (code 8 is reported); dependents are released after the
+// Row tiles are scheduled longest first. Waits are bounded by time (code 8 is reported). The launch is ordered after its predecessor; dependents are released after the
 // tensor-memory allocation, and a CTA asks for so much of the shared memory that nothing else that allocates tensor memory
 // fits beside it (least_smem).
 #pragma once
@@ -45,7 +45,6 @@ struct AttnParams {
   int rep, kv_heads;
   float scale_log2;  // |scale| * log2(e) (1 where scale is zero)
   float sign;        // 1, -1 or 0: what the scores are multiplied by first, so that the largest score has the largest exponent
-  int is_bf16;
   int* error_flag;
   unsigned long long timeout_ns;
 };
@@ -169,7 +168,6 @@ umma_attention_kernel(const AttnParams p, const __grid_constant__ CUtensorMap qm
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
   const uint32_t tmem_base = *tmem_slot;
   // Columns: S of every tile, then O of every tile.
   auto s_col = [&](int t) { return tmem_base + (uint32_t)(t * kAttnKeys); };

@@ -6,7 +6,7 @@
 // the same kernel; a small m costs a narrow MMA instead of a padded 128-row one, and no CUDA-core FMA work is left on
 // the SM, so for small m the kernel is a pure HBM stream: TMA in, tensor core, a tiny epilogue.
 //
-// Work decomposition: a thread-block cluster of `ksplit` CTAs (1..8, one CTA per SM) owns a tile of 128 columns x m_tile
+// Work decomposition: a thread-block cluster of `ksplit` CTAs (1..8, one or two CTAs per SM) owns a tile of 128 columns x m_tile
 // rows and walks tiles c, c + clusters, ...; each of its CTAs contracts 1/ksplit of k. The partial accumulators are
 // summed through distributed shared memory: every CTA sends the rows that CTA r finishes to CTA r, counts itself in on
 // r's mbarrier, and sums what it received itself in rank order (run-to-run identical results). Nothing goes through
@@ -630,7 +630,7 @@ __global__ void __launch_bounds__(threads_of(SRC), SRC == kLoose ? 1 : 2) umma_s
     } else if constexpr (SRC == kLoose) {
       // One column per thread, 16 * SUB rows per unit; the next unit's loads are in flight while this one is converted.
       constexpr int R = 16 * SUB;
-      if (!p.early_rhs) asm volatile("griddepcontrol.wait;" ::: "memory");
+      if (!p.early_rhs) asm volatile("griddepcontrol.wait;" ::: "memory");  // (returns at once: these launches are ordered)
       int tile = cluster, kb = kb_begin;
       Tile t = locate_tile(p, min(tile, p.tiles - 1));
       unsigned short next[R];

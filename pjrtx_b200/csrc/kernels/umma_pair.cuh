@@ -20,8 +20,8 @@
 // Measured, 8192 rows, bf16, before (one SM per tile) and now: 4096 x 28672 2030 / 1340 us (1433 TFLOP/s), 14336 x 4096
 // 880 / 648 us, 4096 x 6144 429 / 310 us, 4096 x 4096 291 / 211 us.
 //
-// No copy is multicast. Waits are bounded by time as in umma_gemm.cuh; dependents are released after the tensor-memory
-// allocation, and the weights of the first ring are requested before the preceding kernel has finished (`early_rhs`).
+// No copy is multicast. Waits are bounded by time as in umma_gemm.cuh. The launch is ordered after its predecessor; its
+// dependents are released after the tensor-memory allocation.
 #pragma once
 
 #include "umma_gemm.cuh"
@@ -33,7 +33,7 @@ constexpr int kPairN = 256;   // weight columns of a tile (128 per CTA)
 constexpr int kBand = 8;      // weight tiles of a band
 
 struct PairParams {
-  int m, k;
+  int m;
   int m_tile;                      // multiple of 32, 32..256
   int m_tiles, n_tiles;            // n_tiles over the whole group
   int count;
@@ -44,7 +44,7 @@ struct PairParams {
   int kblocks;                     // ceil(k / 64)
   int stages;
   int is_bf16;
-  int rhs_k_major, rhs_3d, early_rhs;
+  int rhs_k_major, rhs_3d;
   int* error_flag;
   unsigned long long timeout_ns;
 };
@@ -173,28 +173,20 @@ __global__ void __launch_bounds__(kBaseThreads, 1) umma_pair_kernel(const PairPa
         pair_load_2d(base + (uint32_t)stage * per_stage + 16384u, &maps.lhs, kb * kSubK, t.m_idx * p.m_tile + rank * (int)lhs_rows,
                      cluster_address(smem_u32(&full[stage]), 0));
       };
-      const int first = p.early_rhs ? min(min(count, p.stages), p.kblocks) : 0;
       PairTile t = locate_pair_tile(p, pair);
-      for (int i = 0; i < first; i++) {
-        if (rank == 0) mbar_expect_tx(&full[i], 2 * per_stage);
-        load_rhs(t, i, i);
-      }
-      asm volatile("griddepcontrol.wait;" ::: "memory");
       int seg = 0, kb = 0, stage = 0;
       unsigned phase = 0;
       for (int i = 0; i < count; i++) {
-        if (i >= first) {
-          if (i >= p.stages && !mbar_wait(&empty[stage], phase ^ 1, budget)) {
-            atomicExch(p.error_flag, 17);
-            // The copies in flight get time to land before the pair leaves.
-            const unsigned long long until = global_timer_ns() + 50000;
-            while (global_timer_ns() < until) {
-            }
-            break;
+        if (i >= p.stages && !mbar_wait(&empty[stage], phase ^ 1, budget)) {
+          atomicExch(p.error_flag, 17);
+          // The copies in flight get time to land before the pair leaves.
+          const unsigned long long until = global_timer_ns() + 50000;
+          while (global_timer_ns() < until) {
           }
-          if (rank == 0) mbar_expect_tx(&full[stage], 2 * per_stage);
-          load_rhs(t, kb, stage);
+          break;
         }
+        if (rank == 0) mbar_expect_tx(&full[stage], 2 * per_stage);
+        load_rhs(t, kb, stage);
         load_lhs(t, kb, stage);
         if (++kb == p.kblocks) {
           kb = 0;
@@ -249,7 +241,6 @@ __global__ void __launch_bounds__(kBaseThreads, 1) umma_pair_kernel(const PairPa
     }
   } else {
     // ---- epilogue warps 0..3 of each CTA: TMEM lane = weight column ------------------------------------------------------
-    asm volatile("griddepcontrol.wait;" ::: "memory");
     for (int seg = 0; seg < my_tiles; seg++) {
       const PairTile t = locate_pair_tile(p, pair + seg * pairs);
       const int buf = seg & 1;
