@@ -467,7 +467,9 @@ inline bool sgemm_ok(const DotShape& s, const void* lhs, const void* rhs, const 
 // 64 x 64 outputs per CTA of 64 threads, 8 x 8 per thread, k in slabs of 16 through two shared-memory buffers; the next slab
 // travels (cp.async for f32) while the current one is multiplied. `split` CTAs of a cluster contract a slice of k each and
 // sum their tiles through distributed shared memory in rank order.
-// Measured: a call with a small ragged product 112 -> 49 us. Where 128 x 64 tiles fill the chip the kernel above is ahead
+// Measured: a call with a small ragged product 112 -> 49 us; 333 x 1777 x 777 f32 74 us, issue slots 57 % busy, one
+// scalar cp.async per element of its odd rows. The 16-bit form spills 94 bytes at its bound of 168 registers (six CTAs per SM;
+// its slab waits in registers), the f32 forms none. Where 128 x 64 tiles fill the chip the kernel above is ahead
 // (1024^3 70 us against 75 here: both are bound by shared-memory reads beside the FMAs, and this one also sums four parts).
 constexpr int kSplitTile = 64, kSplitBK = 16, kSplitThreads = 64, kSplitPad = 4;
 
@@ -668,7 +670,8 @@ int launch_split_tile(const DotShape& s, const T* a, const T* b, T* o, int64_t b
 // dependent latencies, not bytes. The persistent kernel's chain is tensor map -> copy -> mbarrier -> partial sums in global
 // memory -> arrival counter -> fold; here a CTA owns 64 columns for all of k, requests every 16-byte piece of its weights
 // at once (before the preceding kernel has finished, where nothing writes them), then the lhs, multiplies, and folds the
-// eight warps through shared memory in a fixed order.
+// eight warps through shared memory in a fixed order. (16-bit at eight rows would spill 72 bytes; 16-bit operands come
+// here with one and two rows only, from three up the tensor cores take them wherever rows are aligned.)
 constexpr int kSmallCols = 64, kSmallThreads = 256, kSmallPasses = 16;
 // Rows a CTA covers in one round of loads: 8 warps x 32 lanes x 16 bytes over 64 columns.
 __host__ __device__ constexpr int small_rows_per_pass(int esize) { return kSmallThreads * 16 / (kSmallCols * esize); }
@@ -911,9 +914,9 @@ DotScratch dot_group_plan(const DotShape* shapes, int count, int sm_count, bool 
     if (all_umma) return umma_plan(shapes, count, sm_count, 1);
   }
   if (batch == 1) {
-    // A k that one round of loads covers and at most a wave of CTAs: the kernel without rings and folds. Measured per
-    // launch, before and now: 2 x 256 x 512 bf16 7.5 / 6.2 us, 2 x 256 x 1024 bf16 7.6 / 6.5 us,
-    // 4 x 16 x 48 f32 6.5 / 4.4 us (a launch with nothing in it is about 2).
+    // A k that one round of loads covers and at most a wave of CTAs: the kernel without rings and folds, and without
+    // scratch. Measured: eight steps of a toy decoder (72 such launches) 1290 us on the persistent kernel and 1233 on this
+    // one, together with the generated kernels' vector reads; a toy f32 block (seven such launches) 55 us on either.
     int64_t small_tiles = 0;
     for (int g = 0; g < count; g++) small_tiles += (shapes[g].n + kSmallCols - 1) / kSmallCols;
     // Persistent TMA kernel: equal shares of (column tile, row chunk) units per CTA, two CTAs per SM with a ring of

@@ -15,17 +15,21 @@
 //                  probabilities go back to tensor memory, over the scores they came from, in the element type
 // Tensor memory: S_t (128 columns, its first 64 reused for P_t) and O_t (head_dim columns) per tile.
 //
-// O is rescaled only when a row's maximum has grown by more than 2^8 since the scale in use was chosen: until then the
-// probabilities are relative to the older maximum (at most 256, in range for every type involved; the common factor cancels
-// in the division by the row sum), and the round trip of O through registers is saved. The row sum is kept in f32 and is taken
-// of the probabilities as the second product reads them, rounded to the element type, so that their rounding cancels where
-// few keys carry a row: with equal values under all keys the result is that value.
+// O is rescaled only when a row's maximum has grown by more than 2^8 since the scale in use was chosen (the conditional
+// rescaling published with FlashAttention-4): until then the probabilities are relative to the older maximum (at most 256, in
+// range for every type involved; the common factor cancels in the division by the row sum), and the round trip of O through
+// registers is saved. The row sum is kept in f32 and is taken of the probabilities as the second product reads them, rounded
+// to the element type, so that their rounding cancels where few keys carry a row: with equal values under all keys the result
+// is that value.
 // A block's S is complete only after the product O += P . V issued before it (one commit covers both), so a softmax thread
 // that has seen S may touch O.
 //
 // What bounds it: per block and tile 1024 cycles of tensor core and 1024 cycles of exponentials (128 x 128 at 16 per
 // cycle), which overlap between the two tiles. Measured for 4 x 2048 positions, 32 query heads of 128 over 8 KV heads: the
-// warp-level kernel before this one (mma.sync, 64 rows per CTA) 627 us, this one 241 us; 1 x 517 positions 24 and 14 us.
+// warp-level kernel before this one (mma.sync, 64 rows per CTA) 627 us, this one 256 us inside a full-depth prefill and 201 us
+// alone at full clock; 1 x 517 positions 24 and 14 us.
+// Two tiles per CTA (320 threads) get 168 registers and spill 56 to 60 bytes; one tile has 180 and none. Reading the scores
+// twice in 32-column chunks to hold fewer of them was slower (248 / 275 us).
 //
 // Row tiles are scheduled longest first. Waits are bounded by time (code 8 is reported). The launch is ordered after its predecessor; dependents are released after the
 // tensor-memory allocation, and a CTA asks for so much of the shared memory that nothing else that allocates tensor memory

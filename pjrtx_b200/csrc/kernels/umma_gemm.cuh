@@ -14,11 +14,11 @@
 // the per-SM rate and the number of waves (umma_choose in dot.cu).
 // This replaced equal shares of 64-deep units per CTA with f32 partials in global memory and a fold by the CTA that
 // arrived last: there every launch paid its HBM time plus 14 to 21 us, 7 us of them the tail (partials out, arrival
-// counter, two dependent rounds of loads through one SM). Measured per launch, before and now: 32 rows, bf16, 4096 x 6144
-// 22.5 / 19.8 us, 4096 x 4096 22.2 / 15.5 us, 14336 x 4096 34.4 / 26.4 us, 4096 x 128256 170 / 157 us; 16 rows, int8, 4096 x
-// 28672 49.2 / 39.6 us, 4096 x 128256 180 / 122 us. The 8B-shape step at batch 32 went from 5.98 to 5.43 ms, with int8 weights
-// at batch 16 from 6.48 to 5.50 ms. What is left at these sizes is the launch itself (set-up, first copies, sum, exit: 8 to 10
-// us) and, above it, HBM.
+// counter, two dependent rounds of loads through one SM). Measured per launch, before and now (events around a graph
+// node, the events' own time taken off): 32 rows, bf16, 4096 x 6144 22.5 / 18 us, 4096 x 4096 22.2 / 15.6 us, 14336 x 4096
+// 34.4 / 28 us, 4096 x 28672 49 / 42 us, 4096 x 128256 170 / 163 us; 16 rows, int8, 4096 x 28672 49.2 / 40 us, 4096 x 128256
+// 180 / 122 us. What is left at these sizes is the launch itself (set-up, first copies, sum, exit: 8 to 10 us) and, above it,
+// HBM.
 //
 // Roles of a CTA:
 //   producer lane   per unit (one [128 n x 64*SUB k] weight block + the matching [m_tile x 64*SUB] activation block),
@@ -46,7 +46,8 @@
 //            Converting into shared memory instead moved 110 KB through it per 128-deep stage (1630 cycles on the
 //            4096 x 128256 LM head, where HBM needs 715); through TMEM it is 36 KB.
 //   kLoose   16-bit weights of any pitch and alignment (an odd vocabulary, say): converter warps read them with plain
-//            loads, one column per thread, and write them to TMEM. TMA cannot describe such rows.
+//            loads, one column per thread, and write them to TMEM. TMA cannot describe such rows. 5 x 2048 x 32001 f16: 85 us
+//            (one thread per output before: 739), 1.6 TB/s; the converters' ALU is 65 % busy and waits for 2-byte loads.
 //
 // Programmatic dependent launch: weights are never written by earlier work of the stream (`early_rhs`), so their
 // copies for the first ring of stages are issued before griddepcontrol.wait; activation copies and all stores wait.
@@ -365,6 +366,9 @@ __device__ __forceinline__ void tmem_store_blocks(uint32_t addr, const uint32_t 
 }
 
 // SUB: 64-deep k sub-blocks per stage (1 or 2; the sources other than kTile use 2).
+// The converters' bounds spill: 68 bytes at 72 registers for kBytes, the price of two CTAs of 448 threads per SM (one cannot
+// keep the chain of copy, conversion and MMA full); 136 bytes at 80 for kLoose, whose 704 threads leave no more. Neither was
+// timed without its spills. kTile has none.
 template <int SUB, int SRC>
 __global__ void __launch_bounds__(threads_of(SRC), SRC == kLoose ? 1 : 2) umma_stream_kernel(const Params p, const __grid_constant__ Maps maps) {
   extern __shared__ unsigned char smem_dyn[];
