@@ -634,10 +634,28 @@ inline int split_tile_parts(const DotShape& s, int64_t batch, int sm_count) {
   while (split < 8 && tiles * split < (int64_t)sm_count * 4 && s.k / (2 * split) >= 64) split *= 2;
   return split;
 }
-// 128 x 64 tiles (sgemm_kernel, where its 16-byte rows apply) for more than three quarters of the SMs: they run one CTA per
-// SM. One point was measured, 1024^3 with 128 tiles: 70 us against 75 on split tiles; where the two cross was not.
-inline bool wide_tiles_fill(const DotShape& s, int64_t batch, int sm_count) {
-  return (s.n + kSgBN - 1) / kSgBN * ((s.m + kSgBM - 1) / kSgBM) * batch > sm_count * 3 / 4;
+// 128 x 64 tiles (sgemm_kernel, where its 16-byte rows apply): for a k of up to 128, where a split buys nothing (64 x 64
+// x 64 and 200 x 64 x 1024 10.8 us, split tiles 12.8; 500 x 128 x 1024 15.1 / 16.8, 500 x 256 x 1024 23 / 19), and where they give more than three
+// quarters of the SMs a CTA (1024^3 70 us, split tiles 75; 500 x 1024 x 1024, 64 CTAs, 70 / 44).
+inline bool wide_tiles_pay(const DotShape& s, int64_t batch, int sm_count) {
+  return s.k <= 128 || (s.n + kSgBN - 1) / kSgBN * ((s.m + kSgBM - 1) / kSgBM) * batch > sm_count * 3 / 4;
+}
+// Whether split tiles pay against what runs otherwise: one thread per output (up to eight rows) or tile_kernel (16-bit, more
+// rows; f32 always splits there: 9 x 77 x 96 of cold weights 17 us against 23, 500 x 4099 x 256 60 / 70, both near equal at k = 16).
+// A tile costs its 64 rows whatever m is, so few rows of many tiles belong to the threads, whose time hardly depends on n up
+// to 64000 outputs. Measured, threads / split tiles, us, weights in L2 and cold where that differs: f32 1 x 257 x 8001 33 / 25,
+// x 16001 33 / 40 and 83 / 40, x 32001 34 / 64, x 64001 35 / 109; 1 x 2049 x 32001 594 / 400, x 40001 596 / 592, x 64001 592 /
+// 777; 4 x 513 x 32001 76 / 113, 4 x 1025 x 64001 549 / 394, 8 x 2049 x 64001 1589 / 776. 16-bit, where a slab waits in
+// registers: 5 x 65 x 1001 17 / 21, 4 x 129 x 8001 27 / 25, 4 x 257 x 16001 50 / 56, 4 x 513 x 16001 92 / 89, 2 x 129 x 32001
+// 29 / 56, 2 x 2049 x 64001 848 / 1392, 8 x 513 x 32001 167 / 154; tile_kernel / split tiles 64 x 97 x 1001 21 / 29, 64 x 193
+// x 1001 34 / 31, 1000 x 257 x 1001 52 / 58, 1000 x 513 x 1001 95 / 93, 500 x 513 x 4001 141 / 158, 1000 x 2049 x 4001 868 / 1078.
+inline bool split_tiles_pay(const DotShape& s, int64_t batch, int sm_count) {
+  const int64_t tiles = (s.m + kSplitTile - 1) / kSplitTile * ((s.n + kSplitTile - 1) / kSplitTile) * batch;
+  if (dtype_size(s.dtype) == 2)
+    return s.k >= 128 && (tiles <= sm_count || (tiles <= 2 * sm_count && s.k >= 512) || (s.m > 6 && s.m <= 8 && s.k >= 512));
+  if (s.m > 8) return true;
+  if (s.k < 64) return false;
+  return tiles <= 2 * sm_count || s.m > 6 || (s.m > 3 && s.k >= 768) || (s.k >= 1024 && 2 * tiles <= 7 * sm_count);
 }
 
 template <typename T>
@@ -851,7 +869,7 @@ int launch_typed(const DotShape& s, const DotScratch& plan, const void* lhs, con
       dim3 grid((unsigned)((s.n + kSgBN - 1) / kSgBN), (unsigned)((s.m + kSgBM - 1) / kSgBM), (unsigned)batch);
       return launch_kernel(sgemm_kernel, grid, dim3(256), 0, stream, pdl, s, (const float*)lhs, (const float*)rhs, (float*)out) == cudaSuccess ? 1 : 0;
     }
-    if (split_tile_ok(s)) return launch_split_tile<T>(s, a, b, o, batch, plan.ksplit, pdl, stream);
+    if (plan.ksplit > 0 && split_tile_ok(s)) return launch_split_tile<T>(s, a, b, o, batch, plan.ksplit, pdl, stream);
     dim3 grid((unsigned)((s.n + kTile - 1) / kTile), (unsigned)((s.m + kTile - 1) / kTile), (unsigned)batch);
     return launch_kernel(tile_kernel<T>, grid, dim3(256), 0, stream, pdl, s, a, b, o) == cudaSuccess ? 1 : 0;
   }
@@ -914,7 +932,7 @@ DotScratch dot_group_plan(const DotShape* shapes, int count, int sm_count, bool 
     if (all_umma) return umma_plan(shapes, count, sm_count, 1);
   }
   if (batch == 1) {
-    // A k that one round of loads covers and at most a wave of CTAs: the kernel without rings and folds, and without
+    // A k that one round of loads covers and few CTAs: the kernel without rings and folds, and without
     // scratch. Measured: eight steps of a toy decoder (72 such launches) 1290 us on the persistent kernel and 1233 on this
     // one, together with the generated kernels' vector reads; a toy f32 block (seven such launches) 55 us on either.
     int64_t small_tiles = 0;
@@ -923,7 +941,11 @@ DotScratch dot_group_plan(const DotShape* shapes, int count, int sm_count, bool 
     // 32 KiB stages each. Measured on the 8B-shape decode step (ms per step): two CTAs x 3 stages 3.50; one CTA x 5
     // stages 3.67; two CTAs x 6 stages of 16 KiB 3.94; one CTA x 6 stages of 16 KiB 4.95.
     p.tma = 1;
-    if (allow_tensor && s.k <= small_max_k(esize) && small_tiles <= sm_count) {
+    // Where the persistent kernel's launch is as short, it stays: five to eight rows of a k up to 64 (8 x 64 x 1024 f32 8.9
+    // us, 10.9 here) or of many tiles (8 x 256 x 4736 11 / 13 of cold weights), three and four rows of a wave (4 x 256 x 9472
+    // 10.8 / 12.9).
+    const int64_t most = s.m > 4 ? sm_count / 8 : s.m > 2 ? sm_count * 3 / 4 : sm_count;
+    if (allow_tensor && s.k <= small_max_k(esize) && small_tiles <= most && (s.m <= 4 || s.k > 64)) {
       p.small = 1;
       p.grid = (int)small_tiles;
       return p;
@@ -1575,12 +1597,12 @@ DotScratch dot_plan(const DotShape& s, int sm_count) {
     p.path = 2;
     return p;
   }
-  // Few rows of pitches the streaming kernels cannot take: tiles, unless there is too little work for one to matter.
-  const bool few = s.lhs_k == 1 && s.rhs_n == 1 && s.k >= 64 && s.n >= 64;
+  const bool split = s.k >= 1 && s.n >= 1 && split_tile_ok(s) && split_tiles_pay(s, batch, sm_count);
+  const bool few = split && s.n >= 64;  // few rows of pitches the streaming kernels cannot take
   if ((s.m > 8 || few) && batches_fit && (s.m + kTile - 1) / kTile <= 65535) {
     p.path = 3;
-    p.wide = wide_tiles_fill(s, batch, sm_count) ? 1 : 0;
-    p.ksplit = split_tile_parts(s, batch, sm_count);
+    p.wide = wide_tiles_pay(s, batch, sm_count) ? 1 : 0;
+    p.ksplit = split ? split_tile_parts(s, batch, sm_count) : 0;
     return p;
   }
   p.path = 0;

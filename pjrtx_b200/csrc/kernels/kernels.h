@@ -95,8 +95,8 @@ struct DotScratch {
   int tma = 0;
   // ... or, for a k that a CTA's registers hold, the kernel without rings and folds.
   int small = 0;
-  // Path 3: 128 x 64 tiles fill the chip; otherwise (and where their 16-byte rows do not apply) `ksplit` CTAs of a cluster
-  // share a tile of 64 x 64.
+  // Path 3: 128 x 64 tiles where their 16-byte rows apply; otherwise `ksplit` CTAs of a cluster share a tile of 64 x 64, or
+  // (ksplit 0) one CTA of tile_kernel has it.
   int wide = 0;
   // Paths 1 and 4 for 16-bit floats without batch axes can run on the tensor cores (tcgen05, accumulator in TMEM); path 5
   // always does. `ksplit` CTAs of a cluster then share a tile of 128 columns x m_tile rows, contracting 1/ksplit of k each;

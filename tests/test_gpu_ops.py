@@ -750,10 +750,12 @@ def test_row_argmax_with_row_maximum_edge_values(gpu_backend, cols):
     (P.F32, 9, 64, 64),        # one tile
     (P.F32, 65, 130, 68),      # ragged in every direction, 16-byte pitches for rhs only
     (P.F32, 100, 2048, 256),   # k shared by eight CTAs
+    (P.F32, 9, 132, 64),       # one tile, k shared by two CTAs
     (P.F32, 64, 1000, 101),    # odd pitch: 4-byte copies
     (P.F32, 3, 200, 77),       # few rows of an odd pitch
     (P.F16, 40, 333, 129),     # 16-bit operands whose rows the tensor cores cannot take
     (P.BF16_CODE, 5, 1001, 65),
+    (P.F16, 64, 97, 130),      # 16-bit operands of a k too short to share: plain tiles
 ])
 def test_register_blocked_contractions_against_f64(gpu_backend, dtype, m, k, n):
     """f32 (and loosely pitched 16-bit) contractions in 64 x 64 tiles with k split over a cluster: f32 sums, one rounding of

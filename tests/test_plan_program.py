@@ -444,3 +444,30 @@ def test_every_device_side_wait_takes_its_budget_from_the_launch():
         budgets += [(name, b) for b in re.findall(r"WaitBudget budget\{[\w:]*global_timer_ns\(\) \+ ([\w.]+),", text)]
         assert not re.search(r"imeout_?ns\w* = \d", text, re.I), name
     assert len(budgets) == 5 and all(b.endswith("timeout_ns") for _, b in budgets), budgets
+
+
+@pytest.mark.parametrize("dtype,m,k,n,path,split", [
+    # few rows of a pitch nothing streams: split tiles while they are few or the threads have much to do
+    (P.F32, 1, 63, 1001, 0, False), (P.F32, 1, 257, 8001, 3, True), (P.F32, 2, 257, 32001, 0, False), (P.F32, 2, 2049, 32001, 3, True),
+    (P.F32, 2, 2049, 40001, 0, False), (P.F32, 4, 513, 32001, 0, False), (P.F32, 4, 1025, 64001, 3, True), (P.F32, 8, 257, 32001, 3, True),
+    (P.F16, 5, 65, 1001, 0, False), (P.F16, 4, 129, 8001, 3, True), (P.F16, 4, 257, 16001, 0, False), (P.F16, 2, 2049, 64001, 0, False),
+    (P.F16, 8, 513, 32001, 3, True),
+    # more rows: a k too short or too many tiles for a split in 16 bits
+    (P.F16, 64, 97, 1001, 3, False), (P.F16, 64, 193, 1001, 3, True), (P.F16, 1000, 257, 1001, 3, False), (P.F16, 1000, 513, 1001, 3, True),
+    (P.F16, 500, 513, 4001, 3, False), (P.F32, 500, 257, 4099, 3, True),
+])
+def test_kernel_choice_of_loosely_pitched_contractions(backend, dtype, m, k, n, path, split):
+    """The measured lines between one thread per output, split tiles and plain tiles."""
+    b = PlanBuilder()
+    b.set_outputs([b.dot_general(b.parameter(dtype, [m, k]), b.parameter(dtype, [k, n]), [1], [0])])
+    (st,) = backend.describe_kernels(b)["steps"]
+    assert st["path"] == path and (path == 0 or (st["ksplit"] > 0) == split), st
+
+
+@pytest.mark.parametrize("m,k,n,small", [(2, 256, 9472, 1), (4, 256, 7104, 1), (4, 256, 9472, 0), (8, 64, 256, 0), (8, 96, 1024, 1),
+                                         (8, 256, 4736, 0)])
+def test_small_contractions_keep_to_where_they_are_shorter(backend, m, k, n, small):
+    b = PlanBuilder()
+    b.set_outputs([b.dot_general(b.parameter(P.F32, [m, k]), b.parameter(P.F32, [k, n]), [1], [0])])
+    (st,) = backend.describe_kernels(b)["steps"]
+    assert st["path"] == 1 and st["small"] == small, st
