@@ -1193,11 +1193,15 @@ int launch_prefill(const AttnPrefillShape& s, const umma::AttnParams& p, const v
       !encode_kv_map(&vmap, v, !BF16, view, HD))
     return 0;
   // Two row tiles per CTA share every key block and let one tile's softmax overlap the other's products; one tile per CTA
-  // where that would leave SMs without work.
+  // where that would leave SMs without work. Of 64 elements a row an SM holds two CTAs of one tile, which overlap the same way
+  // and divide more evenly; over more than five blocks of keys the shared ones count for more. Measured, two tiles / two CTAs of
+  // one, us, sequences x KV heads x query heads each x positions: 16 x 8 x 1 x 300 25.4 / 23.3, x 513 45.6 / 37.8, x 700 49.6 /
+  // 48.0; 8 x 8 x 4 x 400 39.7 / 37.4, x 513 53.1 / 51.4, x 700 68.4 / 71.8; 1 x 8 x 4 x 2048 65.6 / 70.5 (the warp-level kernel
+  // before: 20.5, 39.1, 52.0; 39.9, 57.9, 87.7; 95.6).
   int device = 0, sms = 148;
   if (cudaGetDevice(&device) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
   const long long pairs = (p.rows + 2 * umma::kAttnRows - 1) / (2 * umma::kAttnRows) * s.kv_heads * s.batch;
-  return pairs >= sms ? launch_prefill_tiles<BF16, HD, 2>(s, p, qmap, kmap, vmap, out, stream)
+  return pairs >= sms && (HD == 128 || s.seq > 5 * umma::kAttnKeys) ? launch_prefill_tiles<BF16, HD, 2>(s, p, qmap, kmap, vmap, out, stream)
                       : launch_prefill_tiles<BF16, HD, 1>(s, p, qmap, kmap, vmap, out, stream);
 }
 

@@ -28,12 +28,12 @@
 // cycle), which overlap between the two tiles. Measured for 4 x 2048 positions, 32 query heads of 128 over 8 KV heads: the
 // warp-level kernel before this one (mma.sync, 64 rows per CTA) 627 us, this one 256 us inside a full-depth prefill and 201 us
 // alone at full clock; 1 x 517 positions 24 and 14 us.
-// Two tiles per CTA (320 threads) get 168 registers and spill 56 to 60 bytes; one tile has 180 and none. Reading the scores
+// Two tiles per CTA (320 threads) get 168 registers and spill 56 to 60 bytes, one tile of 64 elements a row with two CTAs per
+// SM the same and 68 bytes; one of 128 has 180 and none. Reading the scores
 // twice in 32-column chunks to hold fewer of them was slower (248 / 275 us).
 //
 // Row tiles are scheduled longest first. Waits are bounded by time (code 8 is reported). The launch is ordered after its predecessor; dependents are released after the
-// tensor-memory allocation, and a CTA asks for so much of the shared memory that nothing else that allocates tensor memory
-// fits beside it (least_smem).
+// tensor-memory allocation. The allocations of CTAs that share an SM fit its tensor memory (least_smem).
 #pragma once
 
 #include "umma_gemm.cuh"
@@ -54,9 +54,11 @@ struct AttnParams {
 };
 
 __host__ __device__ constexpr int attn_slot_bytes(int hd) { return kAttnKeys * hd * 2; }
+// CTAs an SM holds: two of one tile of 64 elements a row (98 KiB and 256 tensor-memory columns each), else one.
+__host__ __device__ constexpr int attn_per_sm(int hd, int tiles) { return hd == 64 && tiles == 1 ? 2 : 1; }
 __host__ __device__ constexpr size_t attn_smem_bytes(int hd, int tiles) {
   const size_t bytes = (size_t)tiles * kAttnRows * hd * 2 + (size_t)kAttnSlots * attn_slot_bytes(hd) + 512 + 1024;
-  const size_t least = least_smem(512);
+  const size_t least = least_smem(attn_per_sm(hd, tiles) == 2 ? 256 : 512);
   return bytes < least ? least : bytes;
 }
 
@@ -120,7 +122,7 @@ __device__ __forceinline__ void add_pair(uint32_t pair, float& lo, float& hi) {
 }
 
 template <bool BF16, int HD, int TILES>
-__global__ void __launch_bounds__(128 * TILES + 64, 1)
+__global__ void __launch_bounds__(128 * TILES + 64, attn_per_sm(HD, TILES))
 umma_attention_kernel(const AttnParams p, const __grid_constant__ CUtensorMap qmap, const __grid_constant__ CUtensorMap kmap,
                       const __grid_constant__ CUtensorMap vmap, void* __restrict__ out) {
   static_assert(HD == 64 || HD == 128, "");

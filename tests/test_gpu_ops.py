@@ -440,12 +440,13 @@ def test_prefill_attention_matches_oracle(gpu_backend, dtype, kv_heads, rep, seq
 
 @pytest.mark.parametrize("dtype,batch,kv_heads,rep,seq,hd,spread", [
     (P.BF16_CODE, 2, 8, 4, 700, 128, 1.0),  # two row tiles per CTA, six key blocks: the copy ring wraps
-    (P.F16, 5, 8, 4, 257, 64, 1.0),         # two row tiles, a third block that holds one key
+    (P.F16, 5, 8, 4, 257, 64, 1.0),         # two CTAs of one row tile per SM, a third block that holds one key
+    (P.F16, 4, 8, 4, 649, 64, 1.0),         # two row tiles per CTA, a sixth block
     (P.F16, 1, 2, 1, 385, 64, 8.0),         # scores in the hundreds: maxima grow by more than 2^8 between blocks
     (P.BF16_CODE, 2, 37, 1, 300, 128, 8.0),  # the same with two row tiles; a row tile spans a whole key block
 ])
 def test_prefill_attention_against_f64(gpu_backend, dtype, batch, kv_heads, rep, seq, hd, spread):
-    """Two row tiles per CTA and rescaled outputs, against the exact attention. The probabilities enter the second product
+    """One and two row tiles per CTA and rescaled outputs, against the exact attention. The probabilities enter the second product
     in the element type (half a unit in the last place of the largest value) and the result is rounded once more; a score's
     f32 error moves its probability by less than that."""
     b, args = cases.prefill_attention(dtype=dtype, batch=batch, kv_heads=kv_heads, rep=rep, seq=seq, head_dim=hd)
