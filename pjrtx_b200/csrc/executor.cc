@@ -2018,17 +2018,18 @@ bool execute_executable(Executable* exe, size_t device_index, Buffer* const* arg
     // Small parameters are staged into fixed slots; the graph reads the slots.
     std::vector<void*> graph_ptrs = param_ptrs;
     uint64_t dynamic_inputs = 0;
+    std::vector<CopyEntry> staged;
     for (size_t p = 0; p < nargs; p++)
       if (kp.param_slot[p] != UINT64_MAX) {
         void* slot = (char*)ds.arena + kp.param_slot[p];
-        if (args[p]->bytes &&
-            !check_cuda(cudaMemcpyAsync(slot, args[p]->ptr, args[p]->bytes, cudaMemcpyDeviceToDevice, dev->stream), "stage argument")) {
-          *error = last_error();
-          return false;
-        }
+        staged.push_back({args[p]->ptr, slot, args[p]->bytes});
         graph_ptrs[p] = slot;
         dynamic_inputs++;
       }
+    if (!copy_batch_launch(staged.data(), staged.size(), dev->stream)) {
+      *error = std::string("stage arguments: ") + cudaGetErrorString(cudaGetLastError());
+      return false;
+    }
     if (exe->profiling) {
       // Profiled replay: the same steps captured with an event record between them, so the step times are those of
       // graph nodes (no host launch gap) running one after the other; instantiated for this call only.
@@ -2129,6 +2130,7 @@ bool execute_executable(Executable* exe, size_t device_index, Buffer* const* arg
 
   // Wrap outputs.
   std::vector<char> param_taken(nargs, 0);
+  std::vector<CopyEntry> results;
   for (size_t o = 0; o < plan.output_ids.size(); o++) {
     const Value& ov = plan.values[plan.output_ids[o]];
     uint32_t r = kp.root[ov.id];
@@ -2168,14 +2170,13 @@ bool execute_executable(Executable* exe, size_t device_index, Buffer* const* arg
       for (size_t q = 0; q < o; q++)
         if (kp.root[plan.output_ids[q]] == r) src = outs[q]->ptr;
     }
-    if (b->bytes && src &&
-        !check_cuda(cudaMemcpyAsync(b->ptr, src, b->bytes, cudaMemcpyDeviceToDevice, dev->stream), "output copy")) {
-      *error = last_error();
-      buffer_free(b);
-      cleanup();
-      return false;
-    }
+    if (src) results.push_back({src, b->ptr, b->bytes});
     outs[o] = b;
+  }
+  if (!copy_batch_launch(results.data(), results.size(), dev->stream)) {
+    *error = std::string("output copy: ") + cudaGetErrorString(cudaGetLastError());
+    cleanup();
+    return false;
   }
   *outputs = outs;
 

@@ -207,6 +207,17 @@ struct SliceUpdateShape {
 int dus_launch(const SliceUpdateShape& s, void* dst, const void* update, const void* const* start_ptrs, bool pdl,
                cudaStream_t stream);
 
+// Several device-to-device copies as one launch for every kCopyBatchMax of them. A source is not written by another
+// entry of the same call; any addresses and sizes are taken (16 bytes at a time where both ends are aligned). The launch
+// is ordered after its predecessor and before its successor. False: a launch failed.
+struct CopyEntry {
+  const void* src;
+  void* dst;
+  uint64_t bytes;
+};
+constexpr int kCopyBatchMax = 120;  // 24 bytes each and a 4-byte block count: below the 4 KiB of kernel parameters
+bool copy_batch_launch(const CopyEntry* entries, size_t count, cudaStream_t stream);
+
 // Scaled dot-product attention custom call (src/backend/mlx_metal/custom_call.zig:120-152,
 // src/backend/mlx_metal/api.cc:4929-5043): q [b,]q,h,hd ; k,v [b,]kv,g,hd ; scalar token index.
 struct SdpaShape {

@@ -777,3 +777,27 @@ def test_register_blocked_contractions_against_f64(gpu_backend, dtype, m, k, n):
     mag = np.abs(x.astype(np.float64)) @ np.abs(w.astype(np.float64))
     ulp = {P.F32: 2.0 ** -24, P.BF16_CODE: 2.0 ** -9, P.F16: 2.0 ** -12}[dtype]
     assert np.all(np.abs(got.astype(np.float64) - want) <= 2 * ulp * np.abs(want) + k * 2.0 ** -24 * mag + 2.0 ** -24)
+
+
+@pytest.mark.parametrize("count", [3, 16, 17, 140])
+def test_arguments_and_results_of_a_captured_program_are_copied_whole(gpu_backend, count):
+    """Small arguments reach their slots and results leave the arena in batches of copies: every size around 16 bytes and
+    around a block's piece (32 KiB), more entries than one launch takes, byte for byte, twice with other values."""
+    sizes = [1, 15, 16, 17, 255, 1000, 4095, 4096]
+    b = PlanBuilder()
+    small = [b.parameter(P.U8, (sizes[i % len(sizes)],)) for i in range(count)]
+    x = y = b.parameter(P.F32, (2, 2))
+    for _ in range(4):  # enough steps for a graph
+        y = b.matmul(y, x)
+    wide = b.parameter(P.U8, (3, 32768 // 3 * 4 + 7))
+    b.set_outputs(small + [b.binary("add", wide, wide), y])
+    exe = gpu_backend.compile_executable(b, [0])
+    for seed in range(2):
+        rng = np.random.default_rng(seed)
+        args = [rng.integers(0, 256, v.dims, dtype=np.uint8) for v in small]
+        args += [rng.integers(-2, 3, (2, 2)).astype(np.float32), rng.integers(0, 256, wide.dims, dtype=np.uint8)]
+        got = run_backend(gpu_backend, b, args, exe=exe)
+        for g, w in zip(got, args[:count] + [args[-1] + args[-1], np.linalg.matrix_power(args[-2], 5)]):
+            assert g.dtype == w.dtype and np.array_equal(g, w)
+    assert exe.stats()["graph_launch_count"] == 2
+    exe.destroy()
