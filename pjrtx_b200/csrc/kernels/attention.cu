@@ -686,8 +686,20 @@ attn_decode_staged_kernel(DecodeArgs a, const T* __restrict__ q, const T* __rest
 //                                           V fragments by ldmatrix.trans
 // After the last stage the four warps' (max, sum, out) are merged through shared memory and the split is published
 // like in the CUDA-core kernel.
+//
+// One or two query heads per KV head leave most of the 16 rows empty, and the CUDA-core kernel, which they ran on before,
+// keeps the probabilities in f32. Here such a head has three rows with the same query: the rows' scores and probabilities
+// are equal, and row j multiplies the j-th 16-bit part of the probability (p = hi + mid + lo, each part the rounding of
+// what the ones before it leave), so that the three products add up to that of the f32 probability. The sum of the
+// probabilities is that of the f32 values. f16 has no exponents for the small parts of a probability at most 1: its
+// probabilities are 2^12 times as large, their sum with them. Against the CUDA-core kernel (8 KV heads of 128, two query
+// heads each, us, both with the same distance from 64-bit results to four digits): 5 sequences of 777 keys 18.8 -> 14.7,
+// of 4096 41 -> 24.7; 16 of 2048 53.5 -> 31; 32 of 4096 129 -> 82 (6.5 TB/s); up to 256 keys the two take the same.
 constexpr int kMmaWarps = 4;
 constexpr int kMmaStageKeys = 16 * kMmaWarps;
+// Parts of a probability (rows per query head) and rows of Q.
+__host__ __device__ constexpr int mma_parts(int rep) { return rep <= 2 ? 3 : 1; }
+__host__ __device__ constexpr int mma_rows(int rep) { return rep * mma_parts(rep); }
 
 template <typename T> struct MmaOps;
 template <> struct MmaOps<__nv_bfloat16> {
@@ -732,6 +744,9 @@ attn_decode_mma_kernel(DecodeArgs a, const T* __restrict__ q, const __grid_const
   constexpr int HALVES = HD / 64;                     // 128-byte column blocks per row
   constexpr int TILE_BYTES = kMmaStageKeys * HD * 2;  // one of K or V for one stage
   constexpr int STAGE_BYTES = 2 * TILE_BYTES;
+  constexpr int PARTS = mma_parts(REP), ROWS = mma_rows(REP);
+  constexpr int HALF_ROWS = ROWS <= 8 ? 1 : 2;        // rows 8 to 15 of the fragments are used only beyond eight
+  constexpr float P_SCALE = PARTS > 1 && std::is_same<T, __half>::value ? 4096.f : 1.f;
   // The swizzle of a tiled copy follows the absolute shared-memory address: tiles start on 1024-byte boundaries.
   extern __shared__ unsigned char smem_attn_raw[];
   unsigned char* smem_attn = smem_attn_raw + ((1024u - (attn_smem_u32(smem_attn_raw) & 1023u)) & 1023u);
@@ -811,16 +826,17 @@ attn_decode_mma_kernel(DecodeArgs a, const T* __restrict__ q, const __grid_const
   unsigned qa[HD / 16][4];
   {
     const int r0 = lane >> 2, c0 = (lane & 3) * 2;
-    const T* qrow0 = q + b * a.q_batch_stride + (g * REP + r0) * a.q_head_stride;
-    const T* qrow1 = q + b * a.q_batch_stride + (g * REP + r0 + 8) * a.q_head_stride;
+    const T* qrow0 = q + b * a.q_batch_stride + (g * REP + r0 % REP) * a.q_head_stride;
+    const T* qrow1 = q + b * a.q_batch_stride + (g * REP + (r0 + 8) % REP) * a.q_head_stride;
 #pragma unroll
     for (int ks = 0; ks < HD / 16; ks++) {
-      qa[ks][0] = r0 < REP ? __ldg(reinterpret_cast<const unsigned*>(qrow0 + ks * 16 + c0)) : 0u;
-      qa[ks][1] = r0 + 8 < REP ? __ldg(reinterpret_cast<const unsigned*>(qrow1 + ks * 16 + c0)) : 0u;
-      qa[ks][2] = r0 < REP ? __ldg(reinterpret_cast<const unsigned*>(qrow0 + ks * 16 + c0 + 8)) : 0u;
-      qa[ks][3] = r0 + 8 < REP ? __ldg(reinterpret_cast<const unsigned*>(qrow1 + ks * 16 + c0 + 8)) : 0u;
+      qa[ks][0] = r0 < ROWS ? __ldg(reinterpret_cast<const unsigned*>(qrow0 + ks * 16 + c0)) : 0u;
+      qa[ks][1] = r0 + 8 < ROWS ? __ldg(reinterpret_cast<const unsigned*>(qrow1 + ks * 16 + c0)) : 0u;
+      qa[ks][2] = r0 < ROWS ? __ldg(reinterpret_cast<const unsigned*>(qrow0 + ks * 16 + c0 + 8)) : 0u;
+      qa[ks][3] = r0 + 8 < ROWS ? __ldg(reinterpret_cast<const unsigned*>(qrow1 + ks * 16 + c0 + 8)) : 0u;
     }
   }
+  const int part = (lane >> 2) / REP;  // which part of the probability this thread's row multiplies
   float m_run[2] = {-INFINITY, -INFINITY}, l_part[2] = {0.f, 0.f};
   float o[HD / 8][4];
 #pragma unroll
@@ -902,9 +918,9 @@ attn_decode_mma_kernel(DecodeArgs a, const T* __restrict__ q, const __grid_const
         sc[nt][e] = d;
         mx[e >> 1] = fmaxf(mx[e >> 1], d);
       }
-    unsigned pa[4];
+    unsigned pa[4] = {0u, 0u, 0u, 0u};
 #pragma unroll
-    for (int h = 0; h < 2; h++) {  // row lane / 4 (h = 0) and row lane / 4 + 8 (h = 1)
+    for (int h = 0; h < HALF_ROWS; h++) {  // row lane / 4 (h = 0) and row lane / 4 + 8 (h = 1)
       mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], 1));
       mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], 2));
       const float m_new = fmaxf(m_run[h], mx[h]);
@@ -924,12 +940,21 @@ attn_decode_mma_kernel(DecodeArgs a, const T* __restrict__ q, const __grid_const
 #pragma unroll
         for (int e = 0; e < 2; e++) {
           const float sv = sc[nt][2 * h + e];
-          p[nt * 2 + e] = sv == -INFINITY ? 0.f : __expf(sv - m_new);
+          p[nt * 2 + e] = sv == -INFINITY ? 0.f : __expf(sv - m_new) * P_SCALE;
         }
-      // The probabilities enter the second contraction in the element type; the row sum uses the same rounded values.
+      if (PARTS == 1) {
+        // The probabilities enter the second contraction in the element type; the row sum uses the same rounded values.
+        l_part[h] += Elem<T>::round(p[0]) + Elem<T>::round(p[1]) + Elem<T>::round(p[2]) + Elem<T>::round(p[3]);
+      } else {
+        l_part[h] += (p[0] + p[1]) + (p[2] + p[3]);
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+          const float rest = p[e] - Elem<T>::round(p[e]);
+          p[e] = part == 0 ? p[e] : part == 1 ? rest : rest - Elem<T>::round(rest);
+        }
+      }
       pa[h] = MmaOps<T>::pack(p[0], p[1]);       // keys 0-7 block
       pa[2 + h] = MmaOps<T>::pack(p[2], p[3]);   // keys 8-15 block
-      l_part[h] += Elem<T>::round(p[0]) + Elem<T>::round(p[1]) + Elem<T>::round(p[2]) + Elem<T>::round(p[3]);
     }
     // O += P . V: B fragments from V[key][hd] by transposing loads, two 8-column tiles per ldmatrix.
 #pragma unroll
@@ -967,27 +992,27 @@ attn_decode_mma_kernel(DecodeArgs a, const T* __restrict__ q, const __grid_const
 
   // Row sums over the quad, then per-warp (max, sum, out) to shared memory.
 #pragma unroll
-  for (int h = 0; h < 2; h++) {
+  for (int h = 0; h < HALF_ROWS; h++) {
     l_part[h] += __shfl_xor_sync(0xffffffffu, l_part[h], 1);
     l_part[h] += __shfl_xor_sync(0xffffffffu, l_part[h], 2);
   }
   float* sm_m = reinterpret_cast<float*>(smem_attn);                 // [warps][16]
   float* sm_l = sm_m + kMmaWarps * 16;                               // [warps][16]
-  float* sm_o = sm_l + kMmaWarps * 16;                               // [warps][REP][HD]
+  float* sm_o = sm_l + kMmaWarps * 16;                               // [warps][ROWS][HD]
   {
     const int r0 = lane >> 2, c0 = (lane & 3) * 2;
 #pragma unroll
-    for (int h = 0; h < 2; h++) {
+    for (int h = 0; h < HALF_ROWS; h++) {
       const int r = r0 + 8 * h;
-      if (r < REP) {
+      if (r < ROWS) {
         if ((lane & 3) == 0) {
           sm_m[warp * 16 + r] = m_run[h];
           sm_l[warp * 16 + r] = l_part[h];
         }
 #pragma unroll
         for (int nt = 0; nt < HD / 8; nt++) {
-          sm_o[(warp * REP + r) * HD + nt * 8 + c0] = o[nt][2 * h];
-          sm_o[(warp * REP + r) * HD + nt * 8 + c0 + 1] = o[nt][2 * h + 1];
+          sm_o[(warp * ROWS + r) * HD + nt * 8 + c0] = o[nt][2 * h];
+          sm_o[(warp * ROWS + r) * HD + nt * 8 + c0 + 1] = o[nt][2 * h + 1];
         }
       }
     }
@@ -1005,7 +1030,11 @@ attn_decode_mma_kernel(DecodeArgs a, const T* __restrict__ q, const __grid_const
     for (int w = 0; w < kMmaWarps; w++) {
       const float mw = sm_m[w * 16 + r];
       const float wgt = mw == -INFINITY ? 0.f : __expf(mw - mm);
-      oo = fmaf(sm_o[(w * REP + r) * HD + d], wgt, oo);
+      float ow = sm_o[(w * ROWS + r) * HD + d];
+      // The smaller parts' products; of an infinite V element the largest part's alone is what the sum would be (the others
+      // may be 0 * infinity).
+      if (PARTS > 1 && fabsf(ow) <= 3.402823466e38f) ow += sm_o[(w * ROWS + REP + r) * HD + d] + sm_o[(w * ROWS + 2 * REP + r) * HD + d];
+      oo = fmaf(ow, wgt, oo);
       ll = fmaf(sm_l[w * 16 + r], wgt, ll);
     }
     if (a.splits == 1) {
@@ -1059,7 +1088,7 @@ template <typename T, int REP, int HD, int STAGES>
 int launch_decode_mma_stages(const DecodeArgs& args, dim3 grid, const void* q, const void* k, const void* v, const void* token, void* out,
                       bool pdl, cudaStream_t stream) {
   constexpr size_t stage_smem = (size_t)STAGES * 2 * kMmaStageKeys * HD * 2;
-  constexpr size_t merge_smem = (size_t)(2 * kMmaWarps * 16 + kMmaWarps * REP * HD) * sizeof(float);
+  constexpr size_t merge_smem = (size_t)(2 * kMmaWarps * 16 + kMmaWarps * mma_rows(REP) * HD) * sizeof(float);
   constexpr size_t scratch_smem = (size_t)64 * REP * 2 * sizeof(float);
   constexpr size_t smem = 1024 + (stage_smem > merge_smem ? (stage_smem > scratch_smem ? stage_smem : scratch_smem)
                                                           : (merge_smem > scratch_smem ? merge_smem : scratch_smem));
@@ -1093,7 +1122,7 @@ int dispatch_decode_mma(int rep, int hd, const DecodeArgs& a, dim3 grid, const v
                         const void* token, void* out, bool pdl, cudaStream_t stream) {
 #define CASE(R, H) \
   if (rep == R && hd == H) return launch_decode_mma<T, R, H>(a, grid, q, k, v, token, out, pdl, stream);
-  CASE(4, 128) CASE(8, 128) CASE(4, 64) CASE(8, 64)
+  CASE(1, 128) CASE(2, 128) CASE(4, 128) CASE(8, 128) CASE(4, 64) CASE(8, 64)
 #undef CASE
   return 0;
 }
@@ -1224,10 +1253,10 @@ AttnDecodePlan attn_decode_plan(const AttnDecodeShape& s, int sm_count) {
   AttnDecodePlan p;
   const long long tiles = s.batch * s.kv_heads;
   const long long rep = s.heads / s.kv_heads;
-  // Tensor-core kernel: 16-bit caches with four or eight query heads per KV head and 16-byte aligned rows; everything else
-  // (f32, other head ratios) runs on the CUDA-core kernel. PJRTX_B200_ATTENTION_MMA=0 / 1 forces the choice wherever
+  // Tensor-core kernel: 16-bit caches with four or eight query heads per KV head, one or two where heads are 128 wide, and
+  // 16-byte aligned rows; everything else (f32, one or two heads of 64) runs on the CUDA-core kernel. PJRTX_B200_ATTENTION_MMA=0 / 1 forces the choice wherever
   // the tensor-core kernel applies.
-  const bool mma_ok = (s.dtype == kF16 || s.dtype == kBF16) && (rep == 4 || rep == 8) && (s.head_dim == 64 || s.head_dim == 128) &&
+  const bool mma_ok = (s.dtype == kF16 || s.dtype == kBF16) && (((rep == 4 || rep == 8) && s.head_dim == 64) || s.head_dim == 128) &&
                       s.kv_len >= kMmaStageKeys &&  // the copies' box is a whole stage of keys
                       s.kv_row_stride % 8 == 0 && s.kv_head_stride % 8 == 0 && s.kv_batch_stride % 8 == 0;  // 16-byte pitches
   const char* force = getenv("PJRTX_B200_ATTENTION_MMA");
@@ -1261,7 +1290,9 @@ AttnDecodePlan attn_decode_plan(const AttnDecodeShape& s, int sm_count) {
     if (const char* w = getenv("PJRTX_B200_ATTENTION_SPLITS")) want = std::max(1, atoi(w));  // experiments
     // No split shorter than two stages (splits of one stage measured slower at 2.1 K keys and 8 KV heads: 3.30 ms per
     // 8B-shape step with 37, 3.31 with 30, 3.23 with 24 against 3.21 with 18).
-    long long max_splits = std::max<long long>(1, s.kv_len / (2 * kMmaStageKeys));
+    // Up to six stages one CTA is done before several have merged (one, two and three splits at 256 keys 11.7 / 12.4 / - us,
+    // at 384 keys 12.0 / 12.6 / 12.4 for one to five sequences; at 16 sequences 12.0 / 14.5, 12.5 / 15.5 / 19.6).
+    long long max_splits = s.kv_len <= 6 * kMmaStageKeys ? 1 : s.kv_len / (2 * kMmaStageKeys);
     p.splits = (int)std::max<long long>(1, std::min<long long>(std::min(want, max_splits), 64));
     p.workspace_bytes = (uint64_t)tiles * p.splits * rep * (s.head_dim + 2) * sizeof(float);
     p.counter_bytes = (uint64_t)tiles * 2 * sizeof(unsigned);

@@ -801,3 +801,39 @@ def test_arguments_and_results_of_a_captured_program_are_copied_whole(gpu_backen
             assert g.dtype == w.dtype and np.array_equal(g, w)
     assert exe.stats()["graph_launch_count"] == 2
     exe.destroy()
+
+
+@pytest.mark.parametrize("dtype", [P.BF16_CODE, P.F16])
+@pytest.mark.parametrize("heads,kv_heads,kv_len", [(16, 8, 64), (4, 4, 65), (16, 8, 777), (2, 1, 1200)])
+def test_decode_attention_of_one_and_two_heads_per_kv_head(gpu_backend, dtype, heads, kv_heads, kv_len):
+    """Tensor-core decode attention whose probabilities go through the contraction in three 16-bit parts, against f64: one
+    split and several, a buffer of exactly one stage of keys, spread-out scores. Bound: the rounding of the result (half a unit
+    in the last of 8 or 11 significant bits: at most 2^-8 or 2^-11 of its value) and f32 sums and exponentials (2e-5 of the largest value); also with an infinite value."""
+    hd, batch = 128, 3
+    rng = np.random.default_rng(kv_len)
+    dt = P.np_dtype(dtype)
+    q = (3 * rng.standard_normal((batch, 1, heads, hd))).astype(np.float32).astype(dt)
+    k = rng.standard_normal((batch, kv_len, kv_heads, hd)).astype(np.float32).astype(dt)
+    v = rng.standard_normal((batch, kv_len, kv_heads, hd)).astype(np.float32).astype(dt)
+    b = PlanBuilder()
+    pq, pk, pv = b.parameter(dtype, q.shape), b.parameter(dtype, k.shape), b.parameter(dtype, v.shape)
+    pt = b.parameter(P.S32, [])
+    b.set_outputs([b.custom_call("pjrtx.b200.scaled_dot_product_attention", [pq, pk, pv, pt], dtype, q.shape)])
+    exe = gpu_backend.compile_executable(b, [0])
+    assert exe.describe()["kernel_plan"]["steps"][0]["mma"] == 1
+    kk, vv = (np.repeat(x.astype(np.float64), heads // kv_heads, axis=2) for x in (k, v))
+    scores = np.einsum("bqhd,bkhd->bhk", q.astype(np.float64), kk) / np.sqrt(hd)
+    bits = 2.0 ** -8 if dtype == P.BF16_CODE else 2.0 ** -11
+    for token in {0, 15, 16, 63, min(64, kv_len - 1), kv_len // 2, kv_len - 1, kv_len + 5}:
+        seen = min(token + 1, kv_len)
+        p = np.exp(scores[:, :, :seen] - scores[:, :, :seen].max(axis=2, keepdims=True))
+        want = np.einsum("bhk,bkhd->bhd", p / p.sum(axis=2, keepdims=True), vv[:, :seen])[:, None]
+        got = run_backend(gpu_backend, b, [q, k, v, np.array(token, np.int32)], exe=exe)[0].astype(np.float64)
+        assert (np.abs(got - want) <= bits * np.abs(want) + 2e-5 * np.abs(vv).max()).all(), (token, np.abs(got - want).max())
+    w = v.copy()
+    w[1, 0, 0, 5] = np.inf  # seen by the heads of that KV head only, in one column
+    got = run_backend(gpu_backend, b, [q, k, w, np.array(kv_len, np.int32)], exe=exe)[0].astype(np.float64)
+    hit = np.zeros(got.shape, bool)
+    hit[1, 0, :heads // kv_heads, 5] = True
+    assert np.isfinite(got[~hit]).all() and np.isin(got[hit], [np.inf]).all()
+    exe.destroy()
