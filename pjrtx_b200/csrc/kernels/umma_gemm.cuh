@@ -14,17 +14,20 @@
 // the per-SM rate and the number of waves (umma_choose in dot.cu).
 // This replaced equal shares of 64-deep units per CTA with f32 partials in global memory and a fold by the CTA that
 // arrived last: there every launch paid its HBM time plus 14 to 21 us, 7 us of them the tail (partials out, arrival
-// counter, two dependent rounds of loads through one SM). Measured per launch, before and now (events around a graph
-// node, the events' own time taken off): 32 rows, bf16, 4096 x 6144 22.5 / 18 us, 4096 x 4096 22.2 / 15.6 us, 14336 x 4096
-// 34.4 / 28 us, 4096 x 28672 49 / 42 us, 4096 x 128256 170 / 163 us; 16 rows, int8, 4096 x 28672 49.2 / 40 us, 4096 x 128256
-// 180 / 122 us. What is left at these sizes is the launch itself (set-up, first copies, sum, exit: 8 to 10 us) and, above it,
-// HBM.
+// counter, two dependent rounds of loads through one SM). What is left at the decode sizes is the launch itself (set-up,
+// first copies, sum, exit: 7 to 9 us) and, above it, HBM.
+//
+// Who issues: the copy warp and the MMA warp run their loops converged and let one elected thread issue (elect_one). With a
+// single thread in those loops every operand of an issued instruction went through a vector register: the MMA lane
+// needed 1380 cycles per 128-deep unit beside busy converters, of which the products take 370, and 570 per 64-deep unit
+// without them. Launches one after the other, us, before and now: 32 rows bf16 4096 x 4096 16.5 / 14.8, 4096 x 6144 18.6 /
+// 16.9, 14336 x 4096 30.2 / 27.4, 2048 x 14336 20.5 / 18.5, 7168 x 2048 16.8 / 14.7, 4096 x 28672 43.3 / 42.8 (HBM).
 //
 // Roles of a CTA:
-//   producer lane   per unit (one [128 n x 64*SUB k] weight block + the matching [m_tile x 64*SUB] activation block),
+//   copy warp       per unit (one [128 n x 64*SUB k] weight block + the matching [m_tile x 64*SUB] activation block),
 //                   tiled TMA copies with the 128-byte swizzle into a ring of shared-memory stages; completion is
 //                   counted on the stage's `full` mbarrier
-//   MMA lane        4*SUB tcgen05.mma.cta_group::1.kind::f16 (M=128, N=m_tile, K=16) per stage, operands read through
+//   MMA warp        4*SUB tcgen05.mma.cta_group::1.kind::f16 (M=128, N=m_tile, K=16) per stage, operands read through
 //                   shared-memory descriptors, accumulator in TMEM (two accumulators, so the epilogue of one tile
 //                   overlaps the MMAs of the next); tcgen05.commit releases the stage (`empty`) and, after a
 //                   tile's last MMA, publishes the accumulator (`acc_full`)
@@ -44,7 +47,10 @@
 //            weight at bf16), so the two agree to rounding, not bit for bit, and a product w * s that overflows f16 in
 //            the written program stays finite here.
 //            Converting into shared memory instead moved 110 KB through it per 128-deep stage (1630 cycles on the
-//            4096 x 128256 LM head, where HBM needs 715); through TMEM it is 36 KB.
+//            4096 x 128256 LM head, where HBM needs 715); through TMEM it is 36 KB. The warps of a quarter take units in
+//            turn, read them transposed (ldmatrix) and share the arithmetic out between the ALU and the packed units
+//            (widen_byte_pair). 16 rows, us, before these and the issue above, and now: 4096 x 28672 40.9 / 33.3, 14336 x
+//            4096 30.8 / 26.1, 8192 x 57344 114 / 94.5, 4096 x 128256 119.5 / 102 (5.2 TB/s).
 //   kLoose   16-bit weights of any pitch and alignment (an odd vocabulary, say): converter warps read them with plain
 //            loads, one column per thread, and write them to TMEM. TMA cannot describe such rows. 5 x 2048 x 32001 f16: 85 us
 //            (one thread per output before: 739), 1.6 TB/s; the converters' ALU is 65 % busy and waits for 2-byte loads.
@@ -210,6 +216,25 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t smem_addr, uint32_t leadi
   return d;
 }
 
+// Advanced by a number of bytes (a multiple of 16) inside shared memory: the start address is the descriptor's lowest field
+// and does not run over into the next one.
+__device__ __forceinline__ uint64_t desc_advance(uint64_t desc, uint32_t bytes) {
+  return (desc & 0xffffffff00000000ull) | (uint32_t)((uint32_t)desc + (bytes >> 4));
+}
+// One thread of a converged warp. The MMA warps run their loops as a whole and let this thread issue: addresses and
+// descriptors are then the same for the whole warp and sit in uniform registers, which the tcgen05 instructions want.
+// With one thread of the warp in the loop an instruction took 120 cycles to issue and a 128-deep unit 1380 (its products
+// take 370).
+__device__ __forceinline__ bool elect_one() {
+  unsigned one;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(one));
+  return one != 0;
+}
+
 // Instruction descriptor for kind::f16: f32 accumulate, B (activations) K-major.
 __host__ __device__ inline uint32_t instr_desc(int is_bf16, int mma_n, int a_mn_major) {
   uint32_t d = 0;
@@ -226,9 +251,9 @@ __device__ __forceinline__ void mma_f16(uint32_t tmem_d, uint64_t a_desc, uint64
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
       :
-      : "r"(tmem_d), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(0u)
+      : "r"(tmem_d), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
 // The same with the A operand (128 rows x 16 k: eight 32-bit columns, one row per lane) in tensor memory.
@@ -236,9 +261,9 @@ __device__ __forceinline__ void mma_f16_tmem_a(uint32_t tmem_d, uint32_t tmem_a,
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n\t}"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
       :
-      : "r"(tmem_d), "r"(tmem_a), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(0u)
+      : "r"(tmem_d), "r"(tmem_a), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
@@ -321,30 +346,33 @@ __device__ __forceinline__ Tile locate_tile(const Params& p, int tile) {
   return Tile{g, n_tile, t - n_tile * p.m_tiles};
 }
 
-// Four signed bytes -> four integers in the 16-bit type, two per word, exactly.
-__device__ __forceinline__ void widen_bytes(uint32_t word, int is_bf16, uint32_t* packed) {
-  if (is_bf16) {
-    // b = low7 - 128 * sign. {0x43, low7} is the bf16 128 + low7 and {0x43, sign << 7} is 128 or 256: their difference
-    // is b, exactly.
-    const uint32_t low7 = word & 0x7f7f7f7fu, sign = word & 0x80808080u;
-#pragma unroll
-    for (int e = 0; e < 2; e++) {
-      const uint32_t sel = e ? 0x4342 : 0x4140;
-      const uint32_t x = __byte_perm(low7, 0x43434343u, sel), y = __byte_perm(sign, 0x43434343u, sel);
-      const __nv_bfloat162 v = __hsub2(*reinterpret_cast<const __nv_bfloat162*>(&x), *reinterpret_cast<const __nv_bfloat162*>(&y));
-      packed[e] = *reinterpret_cast<const uint32_t*>(&v);
-    }
-  } else {
-    // {0x64, b + 128} is the f16 1024 + 128 + b.
-    const uint32_t flipped = word ^ 0x80808080u;
-    const __half2 bias = __float2half2_rn(1152.0f);
-#pragma unroll
-    for (int e = 0; e < 2; e++) {
-      const uint32_t x = __byte_perm(flipped, 0x64646464u, e ? 0x4342 : 0x4140);
-      const __half2 v = __hsub2(*reinterpret_cast<const __half2*>(&x), bias);
-      packed[e] = *reinterpret_cast<const uint32_t*>(&v);
-    }
+// Bytes J and J + 2 of a word of signed bytes -> the two integers in the 16-bit type, exactly, byte J in the low half.
+// f16: with its top bit flipped a byte is u = b + 128, and {0x64, u} is 1024 + u: one three-input logic operation masks,
+// flips and adds the exponent (behind a shift for J = 1), one packed subtraction takes the constant away.
+// bf16 has seven fraction bits, and two ways that load the ALU and the packed multiply-add units differently (both issue every
+// second cycle): J = 0 takes one logic operation and three packed, J = 1 a shift, two and one, which balances the two (16 x
+// 4096 x 128256: 103 us; the first way for both 120, the second 117; f16 101).
+//   J = 0: {0x43, u} is v = 128 + u below 128 and 2 * u from there on; with r = v / 2 - 128, b is r where r >= 0 and 2 * r
+//          below: r - max(-r, 0). Every step is exact in eight significant bits.
+//   J = 1: {0x43, low seven bits} is 128 + low and {0x43, top bit} is 128 or 256: their difference is b.
+template <int J, bool BF16>
+__device__ __forceinline__ uint32_t widen_byte_pair(uint32_t word) {
+  if (!BF16) {
+    const uint32_t x = ((J ? word >> 8 : word) & 0x00ff00ffu) ^ 0x64806480u;
+    const __half2 b = __hsub2(*reinterpret_cast<const __half2*>(&x), __float2half2_rn(1152.0f));
+    return *reinterpret_cast<const uint32_t*>(&b);
   }
+  __nv_bfloat162 b;
+  if (J == 0) {
+    const uint32_t x = (word & 0x00ff00ffu) ^ 0x43804380u;
+    const __nv_bfloat162 v = *reinterpret_cast<const __nv_bfloat162*>(&x);
+    const __nv_bfloat162 half = __float2bfloat162_rn(0.5f), bias = __float2bfloat162_rn(128.0f);
+    b = __hsub2(__hfma2(v, half, __hneg2(bias)), __hfma2_relu(v, __hneg2(half), bias));
+  } else {
+    const uint32_t high = word >> 8, x = (high & 0x007f007fu) | 0x43004300u, y = (high & 0x00800080u) | 0x43004300u;
+    b = __hsub2(*reinterpret_cast<const __nv_bfloat162*>(&x), *reinterpret_cast<const __nv_bfloat162*>(&y));
+  }
+  return *reinterpret_cast<const uint32_t*>(&b);
 }
 
 // Sixteen registers per thread: 32 lanes (one per thread) x 16 columns.
@@ -355,19 +383,47 @@ __device__ __forceinline__ void tmem_store_rows(uint32_t addr, const uint32_t (&
       "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
       : "memory");
 }
-// Four 16-lane x 8-column blocks next to each other: of every four registers, 0 and 1 go to lane t/4, columns 2*(t%4) and
-// + 1; 2 and 3 to lane t/4 + 8.
+// Eight 16-lane x 4-column blocks next to each other: registers 2 * i and 2 * i + 1 of thread t go to lanes t / 4 and
+// t / 4 + 8, column 4 * i + t % 4.
 __device__ __forceinline__ void tmem_store_blocks(uint32_t addr, const uint32_t (&r)[16]) {
   asm volatile(
-      "tcgen05.st.sync.aligned.16x256b.x4.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(addr),
+      "tcgen05.st.sync.aligned.16x128b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(addr),
       "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]),
       "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
       : "memory");
 }
+// Four 8 x 8 blocks of 16-bit units, transposed: thread t gets units [2 * (t % 4)][t / 4] and [2 * (t % 4) + 1][t / 4] of each
+// block, whose rows start at the addresses of threads 8 * block .. + 7.
+__device__ __forceinline__ void load_blocks_transposed(uint32_t (&w)[4], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3])
+               : "r"(addr)
+               : "memory");
+}
+
+// One warp's share of a unit of 128 k x 128 columns of signed bytes: the 32 columns of its quarter. `row`: shared-memory
+// address of the lane's row among the first 32.
+template <bool BF16>
+__device__ __forceinline__ void convert_unit(uint32_t row, int quarter, int lane, uint32_t dst) {
+  uint32_t w[8][4];  // 32 rows each; the first four are of lanes 0-15 of the quarter, the others of 16-31
+#pragma unroll
+  for (int i = 0; i < 8; i++)
+    load_blocks_transposed(w[i], row + (((uint32_t)(quarter * 2 + (i >> 2)) ^ (uint32_t)(lane & 7)) << 4) + (uint32_t)(i & 3) * 4096u);
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    uint32_t v[16];
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+      v[2 * i] = widen_byte_pair<0, BF16>(w[2 * q + (i >> 2)][i & 3]);
+      v[2 * i + 1] = widen_byte_pair<1, BF16>(w[2 * q + (i >> 2)][i & 3]);
+    }
+    tmem_store_blocks(dst + (uint32_t)((q & 1) * 32) + (q >> 1 ? 16u << 16 : 0u), v);
+  }
+}
 
 // SUB: 64-deep k sub-blocks per stage (1 or 2; the sources other than kTile use 2).
-// The converters' bounds spill: 68 bytes at 72 registers for kBytes, the price of two CTAs of 448 threads per SM (one cannot
-// keep the chain of copy, conversion and MMA full); 136 bytes at 80 for kLoose, whose 704 threads leave no more. Neither was
+// The bounds make the epilogue spill: 52 bytes at 72 registers for kBytes, the price of two CTAs of 448 threads per SM (one cannot
+// keep the chain of copy, conversion and MMA full); 102 bytes at 80 for kLoose, whose 704 threads leave no more. Neither was
 // timed without its spills. kTile has none.
 template <int SUB, int SRC>
 __global__ void __launch_bounds__(threads_of(SRC), SRC == kLoose ? 1 : 2) umma_stream_kernel(const Params p, const __grid_constant__ Maps maps) {
@@ -399,7 +455,8 @@ __global__ void __launch_bounds__(threads_of(SRC), SRC == kLoose ? 1 : 2) umma_s
   const int count = my_tiles * (kb_end - kb_begin);  // units of this CTA
   const uint32_t tmem_cols = tmem_columns(p.m_tile, SUB, SRC);
 
-  if (threadIdx.x == 4 * 32) {
+  const bool leader = elect_one();  // of every warp; the copy and the MMA warp issue through theirs
+  if (warp == 4 && leader) {
     for (int g = 0; g < p.count && (SRC == kTile || SRC == kBytes); g++) asm volatile("prefetch.tensormap [%0];" ::"l"(&maps.rhs[g]) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&maps.lhs) : "memory");
     for (int s = 0; s < p.stages; s++) {
@@ -407,7 +464,7 @@ __global__ void __launch_bounds__(threads_of(SRC), SRC == kLoose ? 1 : 2) umma_s
       mbar_init(&empty[s], 1);
     }
     for (int s = 0; s < kOperandSlots; s++) {
-      mbar_init(&ready[s], kTmemA ? converter_warps(SRC) : 1);
+      mbar_init(&ready[s], SRC == kBytes ? 4 : kTmemA ? converter_warps(SRC) : 1);  // the warps of a unit
       mbar_init(&slot_empty[s], 1);
     }
     for (int b = 0; b < 2; b++) {
@@ -442,17 +499,21 @@ __global__ void __launch_bounds__(threads_of(SRC), SRC == kLoose ? 1 : 2) umma_s
   };
   // The weights of the first ring are requested before anything else: they depend on nothing.
   const int first = p.early_rhs ? min(count, p.stages) : 0;
-  if (threadIdx.x == 4 * 32) {
+  if (warp == 4) {
     int tile = cluster, kb = kb_begin;
+    Tile t = locate_tile(p, min(tile, p.tiles - 1));
     for (int i = 0; i < first; i++) {
-      const Tile t = locate_tile(p, tile);
-      mbar_expect_tx(&full[i], per_stage);
-      load_rhs(t, kb, i);
+      if (leader) {
+        mbar_expect_tx(&full[i], per_stage);
+        load_rhs(t, kb, i);
+      }
       if (++kb == kb_end) {
         kb = kb_begin;
         tile += clusters;
+        t = locate_tile(p, min(tile, p.tiles - 1));
       }
     }
+    __syncwarp();
   }
   if (warp == 5) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(tmem_cols) : "memory");
@@ -469,98 +530,97 @@ __global__ void __launch_bounds__(threads_of(SRC), SRC == kLoose ? 1 : 2) umma_s
 
   if (warp == 4) {
     // ---- TMA producer ------------------------------------------------------------------------------------------
-    if (lane == 0 && count > 0) {
-      auto load_lhs = [&](const Tile& t, int kb, int stage) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    int tile = cluster, kb = kb_begin, stage = 0;
+    unsigned phase = 0;
+    Tile t = locate_tile(p, min(tile, p.tiles - 1));
+    for (int i = 0; i < count; i++) {
+      if (i >= p.stages && !__all_sync(0xffffffffu, mbar_wait(&empty[stage], phase ^ 1, budget))) {
+        if (leader) {
+          atomicExch(p.error_flag, 11);
+          // Nothing more is requested; the copies in flight get a bounded time to land before the CTA leaves.
+          for (int b = 1; b <= p.stages; b++) {
+            const int j = i - b;  // the last unit requested into each stage
+            for (unsigned spin = 0; spin < (1u << 16) && !mbar_try_wait(&full[j % p.stages], (unsigned)(j / p.stages) & 1u); spin++) {
+            }
+          }
+        }
+        break;
+      }
+      if (leader) {
+        if (i >= first) {
+          mbar_expect_tx(&full[stage], per_stage);
+          load_rhs(t, kb, stage);
+        }
         const uint32_t st = base + (uint32_t)stage * per_stage + w_bytes;
 #pragma unroll
         for (int s = 0; s < SUB; s++)
           tma_load_2d(st + (uint32_t)s * p.m_tile * 128u, &maps.lhs, kb * kDepth + s * kSubK, t.m_idx * p.m_tile, &full[stage]);
-      };
-      asm volatile("griddepcontrol.wait;" ::: "memory");
-      int tile = cluster, kb = kb_begin, stage = 0;
-      unsigned phase = 0;
-      Tile t = locate_tile(p, tile);
-      for (int i = 0; i < count; i++) {
-        if (i >= first) {
-          if (i >= p.stages && !mbar_wait(&empty[stage], phase ^ 1, budget)) {
-            atomicExch(p.error_flag, 11);
-            // Nothing more is requested; the copies in flight get a bounded time to land before the CTA leaves.
-            for (int b = 1; b <= p.stages; b++) {
-              const int j = i - b;  // the last unit requested into each stage
-              for (unsigned spin = 0; spin < (1u << 16) && !mbar_try_wait(&full[j % p.stages], (unsigned)(j / p.stages) & 1u); spin++) {
-              }
-            }
-            break;
-          }
-          mbar_expect_tx(&full[stage], per_stage);
-          load_rhs(t, kb, stage);
+      }
+      __syncwarp();
+      if (++kb == kb_end) {
+        kb = kb_begin;
+        tile += clusters;
+        t = locate_tile(p, min(tile, p.tiles - 1));
+      }
+      if (++stage == p.stages) {
+        stage = 0;
+        phase ^= 1;
+      }
+    }
+    __syncwarp();
+  } else if (warp == 5) {
+    // ---- MMA issuer ----------------------------------------------------------------------------------------------
+    const uint32_t idesc = instr_desc(p.is_bf16, p.m_tile, !kTmemA && !p.rhs_k_major);
+    // Operands of stage 0. Weights K-major like the activations: 64-k sub-blocks 16 KiB apart, 32 bytes per 16-k step inside
+    // the swizzled row. MN-major: 16 k rows = two 1024-byte swizzle atoms further down; the two 64-column boxes are
+    // SUB * 8192 bytes apart (leading offset), 8-row groups 1024 bytes apart (stride offset).
+    const uint64_t a_first = p.rhs_k_major ? smem_desc(base, 16, 1024) : smem_desc(base, SUB * 8192u, 1024);
+    const uint64_t b_first = smem_desc(base + w_bytes, 16, 1024);
+    int stage = 0, slot = 0;
+    unsigned phase = 0, slot_phase = 0;
+    bool ok = true;
+    for (int seg = 0; seg < my_tiles && ok; seg++) {
+      // Take the next accumulator once the epilogue has drained its previous use.
+      const int buf = seg & 1;
+      ok = seg < 2 || __all_sync(0xffffffffu, mbar_wait(&acc_empty[buf], ((seg >> 1) & 1) ^ 1, budget));
+      if (!ok) {
+        if (leader) atomicExch(p.error_flag, 14);
+        break;
+      }
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const uint32_t acc = tmem_base + (uint32_t)(buf * p.m_tile);
+      for (int kb = kb_begin; kb < kb_end; kb++) {
+        // The copies of the stage have landed; the converters have also filled the slot.
+        ok = __all_sync(0xffffffffu, mbar_wait(&full[stage], phase, budget) && (!kTmemA || mbar_wait(&ready[slot], slot_phase, budget)));
+        if (!ok) {
+          if (leader) atomicExch(p.error_flag, 12);
+          break;
         }
-        load_lhs(t, kb, stage);
-        if (++kb == kb_end) {
-          kb = kb_begin;
-          tile += clusters;
-          if (tile < p.tiles) t = locate_tile(p, tile);
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint64_t a = desc_advance(a_first, (uint32_t)stage * per_stage), b = desc_advance(b_first, (uint32_t)stage * per_stage);
+        const uint32_t operand = operand_base + (uint32_t)(slot * 32 * SUB);
+        if (leader) {
+#pragma unroll
+          for (int kk = 0; kk < 4 * SUB; kk++) {
+            const uint64_t b_desc = desc_advance(b, (uint32_t)(kk >> 2) * p.m_tile * 128u + (kk & 3) * 32u);
+            const uint32_t accumulate = (kb == kb_begin && kk == 0) ? 0u : 1u;
+            if (kTmemA) mma_f16_tmem_a(acc, operand + (uint32_t)(kk * 8), b_desc, idesc, accumulate);
+            else mma_f16(acc, desc_advance(a, p.rhs_k_major ? (kk >> 2) * 16384u + (kk & 3) * 32u : kk * 2048u), b_desc, idesc, accumulate);
+          }
+          mma_commit(&empty[stage]);  // the stage is free once these MMAs have read it
+          if (kTmemA) mma_commit(&slot_empty[slot]);  // and so is the operand slot
+          if (kb + 1 == kb_end) mma_commit(&acc_full[buf]);
+        }
+        __syncwarp();
+        if (kTmemA && ++slot == kOperandSlots) {
+          slot = 0;
+          slot_phase ^= 1;
         }
         if (++stage == p.stages) {
           stage = 0;
           phase ^= 1;
         }
-      }
-    }
-  } else if (warp == 5) {
-    // ---- MMA issuer ----------------------------------------------------------------------------------------------
-    if (lane == 0 && count > 0) {
-      const uint32_t idesc = instr_desc(p.is_bf16, p.m_tile, !kTmemA && !p.rhs_k_major);
-      int stage = 0, slot = 0;
-      unsigned phase = 0, slot_phase = 0;
-      bool ok = true;
-      for (int seg = 0; seg < my_tiles && ok; seg++) {
-        // Take the next accumulator once the epilogue has drained its previous use.
-        const int buf = seg & 1;
-        if (seg >= 2 && !mbar_wait(&acc_empty[buf], ((seg >> 1) & 1) ^ 1, budget)) {
-          atomicExch(p.error_flag, 14);
-          break;
-        }
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t acc = tmem_base + (uint32_t)(buf * p.m_tile);
-        for (int kb = kb_begin; kb < kb_end; kb++) {
-          // The copies of the stage have landed; the converters have also filled the slot.
-          if (!mbar_wait(&full[stage], phase, budget) || (kTmemA && !mbar_wait(&ready[slot], slot_phase, budget))) {
-            atomicExch(p.error_flag, 12);
-            ok = false;
-            break;
-          }
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint32_t st = base + (uint32_t)stage * per_stage;
-#pragma unroll
-          for (int kk = 0; kk < 4 * SUB; kk++) {
-            const uint64_t b_desc = smem_desc(st + w_bytes + (uint32_t)(kk >> 2) * p.m_tile * 128u + (kk & 3) * 32u, 16, 1024);
-            const uint32_t accumulate = (kb == kb_begin && kk == 0) ? 0u : 1u;
-            if (kTmemA) {
-              mma_f16_tmem_a(acc, operand_base + (uint32_t)(slot * 32 * SUB + kk * 8), b_desc, idesc, accumulate);
-            } else if (p.rhs_k_major) {
-              // A K-major like B: 64-k sub-blocks 16 KiB apart, 32 bytes per 16-k step inside the swizzled row.
-              mma_f16(acc, smem_desc(st + (kk >> 2) * 16384u + (kk & 3) * 32u, 16, 1024), b_desc, idesc, accumulate);
-            } else {
-              // A MN-major: 16 k rows = two 1024-byte swizzle atoms further down; the two 64-column boxes are
-              // SUB * 8192 bytes apart (leading offset), 8-row groups 1024 bytes apart (stride offset).
-              mma_f16(acc, smem_desc(st + kk * 2048u, SUB * 8192u, 1024), b_desc, idesc, accumulate);
-            }
-          }
-          mma_commit(&empty[stage]);  // the stage is free once these MMAs have read it
-          if (kTmemA) {
-            mma_commit(&slot_empty[slot]);  // and so is the operand slot
-            if (++slot == kOperandSlots) {
-              slot = 0;
-              slot_phase ^= 1;
-            }
-          }
-          if (++stage == p.stages) {
-            stage = 0;
-            phase ^= 1;
-          }
-        }
-        if (ok) mma_commit(&acc_full[buf]);
       }
     }
   } else if (kTmemA && warp >= 6) {
@@ -582,54 +642,43 @@ __global__ void __launch_bounds__(threads_of(SRC), SRC == kLoose ? 1 : 2) umma_s
       }
     };
     if constexpr (SRC == kBytes) {
-      // A thread owns the 4 adjacent columns 4 * (lane / 4) .. + 3 of its warp's 32 and, of every 16-row step, the rows
-      // 4 * (lane % 4) .. + 3: four 32-bit reads; byte permutes pair up the bytes of rows 0 and 1, 2 and 3 of a column,
-      // and each column's four k values are the two words the 16-lane store wants from this thread. Column 4 * c + j of the
-      // warp lands in TMEM lane 8 * j + c. (The bytes are in the 128-byte swizzle, 16-byte chunk ^= row % 8: lanes of
-      // rows 8 apart share a bank, two reads per request. Reading those rows in another order avoids that, but the selects it
-      // takes cost more than the reads: the ALU, 28 permutes and masks per 16 bytes, is what limits the converters.)
-      const int c = lane >> 2, q = lane & 3;
-      const int word = quarter * 8 + c;  // of the 32 words of a row
-      const uint32_t chunk = (uint32_t)(word >> 2), in_chunk = (uint32_t)(word & 3) * 4u;
-      for (int i = 0; i < count; i++) {
+      // 16 columns of 8 rows are a block of 8 x 8 16-bit units: read transposed, a thread gets columns 2 * c and 2 * c + 1
+      // (c = lane / 4) of rows 2 * (lane % 4) and + 1 in one word, which is two k values of each column, and those are the
+      // 32-bit columns that the 16-lane store wants from this thread for lanes c and c + 8. (The 128-byte swizzle spreads
+      // the block's eight rows over all banks.) The two warps of a quarter take units in turn: one waits, reads and stores
+      // while the other converts.
+      static_assert(SRC != kBytes || SUB == 2, "128 rows per unit");
+      auto next_unit = [&]() {
+        if (++stage == p.stages) {
+          stage = 0;
+          phase ^= 1;
+        }
+      };
+      auto next_slot = [&]() {
+        if (++slot == kOperandSlots) {
+          slot = 0;
+          slot_phase ^= 1;
+        }
+      };
+      if (part) {
+        next_unit();
+        next_slot();
+      }
+      for (int i = part; i < count; i += 2) {
         const bool ok = mbar_wait(&full[stage], phase, budget) && slot_free(i);
         if (!__all_sync(0xffffffffu, ok)) {
           if (lane == 0) atomicExch(p.error_flag, 15);
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const unsigned char* raw = base_ptr + (size_t)stage * per_stage;
         const uint32_t dst = operand_base + quarter_addr + (uint32_t)(slot * 32 * SUB);
-        uint32_t w[2 * SUB][4];  // every word of this thread is requested before the first is converted
-#pragma unroll
-        for (int s = 0; s < 2 * SUB; s++)
-#pragma unroll
-          for (int e = 0; e < 4; e++) {
-            const int row = (part * 2 * SUB + s) * 16 + 4 * q + e;
-            w[s][e] = *reinterpret_cast<const uint32_t*>(raw + row * 128 + ((chunk ^ (uint32_t)(row & 7)) << 4) + in_chunk);
-          }
-        static_assert(SRC != kBytes || SUB == 2, "four 16-row steps per warp and unit");
-        const uint32_t at = dst + (uint32_t)(part * 16 * SUB);
-#pragma unroll
-        for (int half = 0; half < 2; half++) {  // lanes 0-15 and 16-31 of the quarter
-          uint32_t v[16];
-#pragma unroll
-          for (int s = 0; s < 2 * SUB; s++) {
-            uint32_t lo[2], hi[2];  // rows 0, 1 and rows 2, 3 of two columns
-            widen_bytes(__byte_perm(w[s][0], w[s][1], half ? 0x7362 : 0x5140), p.is_bf16, lo);
-            widen_bytes(__byte_perm(w[s][2], w[s][3], half ? 0x7362 : 0x5140), p.is_bf16, hi);
-            v[4 * s] = lo[0];
-            v[4 * s + 1] = hi[0];
-            v[4 * s + 2] = lo[1];
-            v[4 * s + 3] = hi[1];
-          }
-          tmem_store_blocks(at + (half ? 16u << 16 : 0u), v);
-        }
+        const uint32_t row = base + (uint32_t)stage * per_stage + (uint32_t)lane * 128u;
+        if (p.is_bf16) convert_unit<true>(row, quarter, lane, dst);
+        else convert_unit<false>(row, quarter, lane, dst);
         publish();
-        if (++stage == p.stages) {
-          stage = 0;
-          phase ^= 1;
-        }
+        next_slot();
+        next_unit();
+        next_unit();
       }
     } else if constexpr (SRC == kLoose) {
       // One column per thread, 16 * SUB rows per unit; the next unit's loads are in flight while this one is converted.
@@ -677,16 +726,10 @@ __global__ void __launch_bounds__(threads_of(SRC), SRC == kLoose ? 1 : 2) umma_s
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if (ksplit > 1) asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
     // The tile column whose values are in this thread's TMEM lane (kBytes writes its operand in that order).
-    const int n_local = warp * 32 + (SRC == kBytes ? 4 * (lane & 7) + (lane >> 3) : lane);
+    const int n_local = warp * 32 + (SRC == kBytes ? (lane & 16) + 2 * (lane & 7) + ((lane >> 3) & 1) : lane);
     for (int seg = 0; seg < my_tiles; seg++) {
       const Tile t = locate_tile(p, cluster + seg * clusters);
       const int buf = seg & 1;
-      // One decision for all four warps: tcgen05.ld is warp-collective.
-      if (!epilogue_all(mbar_wait(&acc_full[buf], (seg >> 1) & 1, budget))) {
-        if (threadIdx.x == 0) atomicExch(p.error_flag, 13);
-        break;
-      }
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const long long n = (long long)t.n_tile * kTileN + n_local;
       const bool in = n < p.n[t.group];
       const int m0 = t.m_idx * p.m_tile;
@@ -695,6 +738,12 @@ __global__ void __launch_bounds__(threads_of(SRC), SRC == kLoose ? 1 : 2) umma_s
       constexpr bool int8 = SRC == kBytes;
       // Int8 weights: the tensor core contracted the integers; this thread's column scale finishes the product.
       const float scale = int8 && in ? __half2float(static_cast<const __half*>(p.scale[t.group])[n]) : 1.f;
+      // One decision for all four warps: tcgen05.ld is warp-collective.
+      if (!epilogue_all(mbar_wait(&acc_full[buf], (seg >> 1) & 1, budget))) {
+        if (threadIdx.x == 0) atomicExch(p.error_flag, 13);
+        break;
+      }
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       auto store = [&](int row, float v) {
         if (int8) v *= scale;
         const long long at = (long long)(m0 + row) * ldo + n;
@@ -704,6 +753,7 @@ __global__ void __launch_bounds__(threads_of(SRC), SRC == kLoose ? 1 : 2) umma_s
       const uint32_t taddr = tmem_base + ((uint32_t)(warp * 32) << 16) + (uint32_t)(buf * p.m_tile);
       const int sum_buf = p.sum_buffers == 2 ? buf : 0;
       float* received = sums + (size_t)sum_buf * ksplit * p.rows_per_rank * kTileN;
+      int owner = 0, owner_row = 0;  // the CTA that finishes the next four rows, and their place among its rows
       for (int c0 = 0; c0 < m_rows; c0 += 16) {
         uint32_t r[16];
         asm volatile(
@@ -717,10 +767,14 @@ __global__ void __launch_bounds__(threads_of(SRC), SRC == kLoose ? 1 : 2) umma_s
           // Rows past m up to the tile's height are delivered too and not used.
 #pragma unroll
           for (int j = 0; j < 16; j += 4) {
-            const int owner = (c0 + j) / p.rows_per_rank, row = c0 + j - owner * p.rows_per_rank;
-            const uint32_t at = cluster_address(smem_u32(received + ((size_t)rank * p.rows_per_rank + row) * kTileN + threadIdx.x * 4), (uint32_t)owner);
+            const uint32_t at =
+                cluster_address(smem_u32(received + ((size_t)rank * p.rows_per_rank + owner_row) * kTileN + threadIdx.x * 4), (uint32_t)owner);
             asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(r[j]), "r"(r[j + 1]), "r"(r[j + 2]), "r"(r[j + 3])
                          : "memory");
+            if ((owner_row += 4) == p.rows_per_rank) {
+              owner_row = 0;
+              owner++;
+            }
           }
         } else if (in) {
 #pragma unroll
@@ -735,8 +789,7 @@ __global__ void __launch_bounds__(threads_of(SRC), SRC == kLoose ? 1 : 2) umma_s
       if (ksplit > 1) {
         // A receive buffer is written again two tiles later, after its writer has seen this CTA's arrivals for the tile
         // in between, which follow the reads below.
-        if (lane == 0)
-          for (int q = 0; q < ksplit; q++) cluster_arrive(cluster_address(smem_u32(&sum_full[buf]), (uint32_t)q));
+        if (lane < ksplit) cluster_arrive(cluster_address(smem_u32(&sum_full[buf]), (uint32_t)lane));
         if (!epilogue_all(cluster_wait(&sum_full[buf], (seg >> 1) & 1, budget))) {
           if (threadIdx.x == 0) atomicExch(p.error_flag, 16);
           break;
