@@ -123,6 +123,7 @@ __global__ void __launch_bounds__(kBaseThreads, 1) umma_pair_kernel(const PairPa
   const int my_tiles = pair < tiles ? (tiles - 1 - pair) / pairs + 1 : 0;
   const int count = my_tiles * p.kblocks;
   const uint32_t tmem_cols = tmem_columns(p.m_tile, 1, kTile);  // two accumulators, as there
+  const bool leader = elect_one();  // of the warp: the copy and the MMA warp issue through theirs
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < p.stages; s++) {
@@ -155,12 +156,26 @@ __global__ void __launch_bounds__(kBaseThreads, 1) umma_pair_kernel(const PairPa
 
   if (warp == 4) {
     // ---- TMA producer (each CTA its own half of both operands) -----------------------------------------------------
-    if (lane == 0 && count > 0) {
-      const uint32_t lhs_rows = (uint32_t)p.m_tile / 2;
-      auto load_rhs = [&](const PairTile& t, int kb, int stage) {
+    const int lhs_rows = p.m_tile / 2;
+    PairTile t = locate_pair_tile(p, min(pair, tiles - 1));
+    int seg = 0, kb = 0, stage = 0;
+    unsigned phase = 0;
+    for (int i = 0; i < count; i++) {
+      if (i >= p.stages && !__all_sync(0xffffffffu, mbar_wait(&empty[stage], phase ^ 1, budget))) {
+        if (leader) {
+          atomicExch(p.error_flag, 17);
+          // The copies in flight get time to land before the pair leaves.
+          const unsigned long long until = global_timer_ns() + 50000;
+          while (global_timer_ns() < until) {
+          }
+        }
+        break;
+      }
+      if (leader) {
         const uint32_t st = base + (uint32_t)stage * per_stage;
         const uint32_t bar = cluster_address(smem_u32(&full[stage]), 0);
         const int k0 = kb * kSubK, n0 = t.n0 + rank * 128;
+        if (rank == 0) mbar_expect_tx(&full[stage], 2 * per_stage);
         if (p.rhs_3d) {
           pair_load_3d(st, &maps.rhs[t.group], 0, k0, n0 / 64, bar);
         } else if (p.rhs_k_major) {
@@ -169,77 +184,65 @@ __global__ void __launch_bounds__(kBaseThreads, 1) umma_pair_kernel(const PairPa
           pair_load_2d(st, &maps.rhs[t.group], n0, k0, bar);
           pair_load_2d(st + 8192u, &maps.rhs[t.group], n0 + 64, k0, bar);
         }
-      };
-      auto load_lhs = [&](const PairTile& t, int kb, int stage) {
-        pair_load_2d(base + (uint32_t)stage * per_stage + 16384u, &maps.lhs, kb * kSubK, t.m_idx * p.m_tile + rank * (int)lhs_rows,
-                     cluster_address(smem_u32(&full[stage]), 0));
-      };
-      PairTile t = locate_pair_tile(p, pair);
-      int seg = 0, kb = 0, stage = 0;
-      unsigned phase = 0;
-      for (int i = 0; i < count; i++) {
-        if (i >= p.stages && !mbar_wait(&empty[stage], phase ^ 1, budget)) {
-          atomicExch(p.error_flag, 17);
-          // The copies in flight get time to land before the pair leaves.
-          const unsigned long long until = global_timer_ns() + 50000;
-          while (global_timer_ns() < until) {
-          }
-          break;
-        }
-        if (rank == 0) mbar_expect_tx(&full[stage], 2 * per_stage);
-        load_rhs(t, kb, stage);
-        load_lhs(t, kb, stage);
-        if (++kb == p.kblocks) {
-          kb = 0;
-          if (++seg < my_tiles) t = locate_pair_tile(p, pair + seg * pairs);
-        }
-        if (++stage == p.stages) {
-          stage = 0;
-          phase ^= 1;
-        }
+        pair_load_2d(st + 16384u, &maps.lhs, k0, t.m_idx * p.m_tile + rank * lhs_rows, bar);
+      }
+      __syncwarp();
+      if (++kb == p.kblocks) {
+        kb = 0;
+        if (++seg < my_tiles) t = locate_pair_tile(p, pair + seg * pairs);
+      }
+      if (++stage == p.stages) {
+        stage = 0;
+        phase ^= 1;
       }
     }
+    __syncwarp();
   } else if (warp == 5) {
     // ---- MMA issuer (leader) -----------------------------------------------------------------------------------------
     asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
     __syncwarp();
-    if (rank == 0 && lane == 0) {
+    if (rank == 0) {
       // M = 256: twice the single-CTA instruction's.
       const uint32_t idesc = instr_desc(p.is_bf16, p.m_tile, !p.rhs_k_major) + ((uint32_t)(kTileN >> 4) << 24);
+      const uint64_t a_first = p.rhs_k_major ? smem_desc(base, 16, 1024) : smem_desc(base, 8192u, 1024);
+      const uint64_t b_first = smem_desc(base + 16384u, 16, 1024);
+      const uint32_t a_step = p.rhs_k_major ? 32u : 2048u;
       int stage = 0;
       unsigned phase = 0;
       bool ok = true;
       for (int seg = 0; seg < my_tiles && ok; seg++) {
         const int buf = seg & 1;
-        if (seg >= 2 && !cluster_wait(&acc_empty[buf], ((seg >> 1) & 1) ^ 1, budget)) {
-          atomicExch(p.error_flag, 20);
+        ok = seg < 2 || __all_sync(0xffffffffu, cluster_wait(&acc_empty[buf], ((seg >> 1) & 1) ^ 1, budget));
+        if (!ok) {
+          if (leader) atomicExch(p.error_flag, 20);
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t acc = tmem_base + (uint32_t)(buf * p.m_tile);
         for (int kb = 0; kb < p.kblocks; kb++) {
-          if (!cluster_wait(&full[stage], phase, budget)) {
-            atomicExch(p.error_flag, 18);
-            ok = false;
+          ok = __all_sync(0xffffffffu, cluster_wait(&full[stage], phase, budget));
+          if (!ok) {
+            if (leader) atomicExch(p.error_flag, 18);
             break;
           }
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint32_t st = base + (uint32_t)stage * per_stage;
+          const uint64_t a = desc_advance(a_first, (uint32_t)stage * per_stage), b = desc_advance(b_first, (uint32_t)stage * per_stage);
+          if (leader) {
 #pragma unroll
-          for (int kk = 0; kk < 4; kk++) {
-            const uint64_t a_desc = p.rhs_k_major ? smem_desc(st + kk * 32u, 16, 1024) : smem_desc(st + kk * 2048u, 8192u, 1024);
-            const uint64_t b_desc = smem_desc(st + 16384u + kk * 32u, 16, 1024);
-            pair_mma_f16(acc, a_desc, b_desc, idesc, (kb == 0 && kk == 0) ? 0u : 1u);
+            for (int kk = 0; kk < 4; kk++)
+              pair_mma_f16(acc, desc_advance(a, kk * a_step), desc_advance(b, kk * 32u), idesc, (kb == 0 && kk == 0) ? 0u : 1u);
+            pair_commit(&empty[stage]);
+            if (kb + 1 == p.kblocks) pair_commit(&acc_full[buf]);
           }
-          pair_commit(&empty[stage]);
+          __syncwarp();
           if (++stage == p.stages) {
             stage = 0;
             phase ^= 1;
           }
         }
-        if (ok) pair_commit(&acc_full[buf]);
       }
     }
+    __syncwarp();
   } else {
     // ---- epilogue warps 0..3 of each CTA: TMEM lane = weight column ------------------------------------------------------
     for (int seg = 0; seg < my_tiles; seg++) {
