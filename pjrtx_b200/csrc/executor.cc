@@ -409,6 +409,7 @@ struct AttnMatch {
   uint32_t q = 0, k = 0, v = 0, pos = 0, out = 0;
   float scale = 1.f;
   bool prefill = false;
+  bool positions_first = false;  // prefill: the result is stored as its only reader, a transpose, would
 };
 
 AttnPrefillShape prefill_shape(const Value& q, const Value& k, float scale) {
@@ -591,6 +592,13 @@ void fuse_decode_attention(Plan* plan) {
       if (k.dims[0] != q.dims[0] || k.dims[2] != q.dims[1] || k.dims[1] != q.dims[2] || k.dims[3] != q.dims[4] ||
           !attn_prefill_supported(prefill_shape(q, k, 1.f)))
         continue;
+      // [B, G, S, rep, hd] read only as [B, S, G, rep, hd]: the kernel stores that.
+      if ((u = sole_user(m.out)) >= 0 && plan->instructions[u].kind == Kind::transpose &&
+          is_list(plan->instructions[u].list("permutation"), {0, 2, 1, 3, 4})) {
+        m.positions_first = true;
+        m.out = plan->instructions[u].outputs[0];
+        m.consumed.push_back(u);
+      }
       bool clash = false;
       for (size_t c : m.consumed) clash |= taken[c] != 0;
       if (clash) continue;
@@ -633,6 +641,7 @@ void fuse_decode_attention(Plan* plan) {
     memcpy(&bits, &m.scale, 4);
     call.attrs["scale_bits"] = {(int64_t)bits};
     call.attrs["dims"] = plan->values[m.out].dims;
+    if (m.prefill) call.attrs["positions_first"] = {m.positions_first ? 1 : 0};
     plan->instructions[m.d1] = call;
   }
   std::vector<Instruction> kept;
@@ -992,6 +1001,7 @@ bool plan_kernels(const Plan& original, int sm_count, KernelPlan* kp, std::strin
           uint32_t bits = (uint32_t)ins.scalar("scale_bits", 0);
           memcpy(&scale, &bits, 4);
           st.attn_prefill = prefill_shape(plan.values[ins.inputs[0]], plan.values[ins.inputs[1]], scale);
+          st.attn_prefill.positions_first = (int)ins.scalar("positions_first", 0);
           if (!attn_prefill_supported(st.attn_prefill)) {
             *error = format_issue(plan, Issue{(long)i, -1, "internal attention call has an unsupported shape", "b200-attention"});
             return false;

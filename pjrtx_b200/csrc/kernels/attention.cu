@@ -1393,6 +1393,9 @@ int attn_prefill_launch(const AttnPrefillShape& s, const void* q, const void* k,
   p.rows = s.seq * s.rep;
   p.rep = (int)s.rep;
   p.kv_heads = (int)s.kv_heads;
+  p.out_batch = s.kv_heads * p.rows * s.head_dim;
+  p.out_head = (s.positions_first ? s.rep : p.rows) * s.head_dim;
+  p.out_pos = (s.positions_first ? s.kv_heads * s.rep : s.rep) * s.head_dim;
   p.sign = s.scale > 0.f ? 1.f : s.scale < 0.f ? -1.f : 0.f;
   p.scale_log2 = s.scale == 0.f ? 1.f : fabsf(s.scale) * 1.4426950408889634f;
   p.error_flag = error_flag;

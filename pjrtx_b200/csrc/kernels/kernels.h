@@ -259,8 +259,9 @@ int attn_decode_launch(const AttnDecodeShape& s, const AttnDecodePlan& plan, con
                        bool early_kv = false, int* error_flag = nullptr, const void* prefetch = nullptr,
                        uint64_t prefetch_bytes = 0);
 
-// Causal self-attention over whole sequences (prefill) as one tensor-core kernel. q / out: [batch, kv_heads, seq, rep,
-// head_dim] contiguous (query head = kv head * rep + r); k / v: [batch, seq, kv_heads, head_dim] through the strides;
+// Causal self-attention over whole sequences (prefill) as one tensor-core kernel. q: [batch, kv_heads, seq, rep,
+// head_dim] contiguous (query head = kv head * rep + r); out: the same, or with `positions_first` [batch, seq, kv_heads, rep,
+// head_dim]; k / v: [batch, seq, kv_heads, head_dim] through the strides;
 // position s sees keys 0..s. Scores stay in f32, where the written program rounds q.k to the element type before it scales.
 // The launch is always ordered after its predecessor.
 struct AttnPrefillShape {
@@ -268,6 +269,7 @@ struct AttnPrefillShape {
   long long batch = 1, kv_heads = 1, rep = 1, seq = 1, head_dim = 1;
   long long kv_batch_stride = 0, kv_row_stride = 0, kv_head_stride = 0;
   float scale = 1.f;
+  int positions_first = 0;
 };
 bool attn_prefill_supported(const AttnPrefillShape& s);
 int attn_prefill_launch(const AttnPrefillShape& s, const void* q, const void* k, const void* v, void* out,

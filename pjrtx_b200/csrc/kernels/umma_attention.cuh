@@ -2,14 +2,15 @@
 // and outputs in tensor memory:
 //   out[b, g, s, r, :] = softmax_j( q[b, g, s, r, :] . k[b, j, g, :] * scale  for j <= s ) . v[b, j, g, :]
 //
-// q and out are [batch, kv_heads, seq, rep, head_dim] (the operand and result layout of the recognised
-// dot_general -> masked softmax -> dot_general form), so the `seq * rep` query rows that share one KV head are one
-// contiguous row-major matrix; row `x` belongs to position x / rep. Scores and probabilities never leave the SM.
+// q is [batch, kv_heads, seq, rep, head_dim] (the operand layout of the recognised dot_general -> masked softmax ->
+// dot_general form), so the `seq * rep` query rows that share one KV head are one contiguous row-major matrix; row `x`
+// belongs to position x / rep. out has that layout too, or [batch, seq, kv_heads, rep, head_dim] where the program only reads
+// it transposed so (a launch of its own before: 26 us for 4 x 2048 positions of 32 heads, 4 us for 517). Scores and probabilities never leave the SM.
 //
 // A CTA owns TILES (1 or 2) tiles of 128 query rows and walks the keys 0..(its last position) in blocks of 128:
-//   copy lane      q once, then K and V blocks into a ring of shared-memory slots (tiled tensor-map copies, 128-byte
+//   copy warp      q once, then K and V blocks into a ring of shared-memory slots (tiled tensor-map copies, 128-byte
 //                  swizzle)
-//   MMA lane       S_t = Q_t . K^T (M = 128 rows, N = 128 keys) and O_t += P_t . V (A operand P_t in tensor memory) for the
+//   MMA warp       S_t = Q_t . K^T (M = 128 rows, N = 128 keys) and O_t += P_t . V (A operand P_t in tensor memory) for the
 //                  tiles in turn: while the softmax warps of one tile work, the tensor core runs the other tile's products
 //   softmax warps  four per tile, one query row per thread (TMEM lane = row): the block's row maximum needs no shuffle;
 //                  probabilities go back to tensor memory, over the scores they came from, in the element type
@@ -47,6 +48,7 @@ constexpr int kAttnSlots = 5;
 struct AttnParams {
   long long rows;  // seq * rep query rows per (sequence, KV head)
   int rep, kv_heads;
+  long long out_batch, out_head, out_pos;  // element strides of the result; a position's `rep` heads are contiguous
   float scale_log2;  // |scale| * log2(e) (1 where scale is zero)
   float sign;        // 1, -1 or 0: what the scores are multiplied by first, so that the largest score has the largest exponent
   int* error_flag;
@@ -146,6 +148,7 @@ umma_attention_kernel(const AttnParams p, const __grid_constant__ CUtensorMap qm
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   constexpr int kMmaWarp = 4 * TILES, kCopyWarp = 4 * TILES + 1;
+  const bool leader = elect_one();  // of the warp: the copy and the MMA warp issue through theirs
   const int g = blockIdx.y, b = blockIdx.z;
   const long long row0 = (long long)(gridDim.x - 1 - blockIdx.x) * (kAttnRows * TILES);  // longest first
   const long long last_row = min(row0 + kAttnRows * TILES, p.rows) - 1;
@@ -180,95 +183,110 @@ umma_attention_kernel(const AttnParams p, const __grid_constant__ CUtensorMap qm
   auto o_col = [&](int t) { return tmem_base + (uint32_t)(TILES * kAttnKeys + t * HD); };
 
   if (warp == kCopyWarp) {
-    if (lane == 0) {
+    if (leader) {
       mbar_expect_tx(q_full, TILES * kTileBytes);
       for (int t = 0; t < TILES; t++)
         for (int c = 0; c < kHalves; c++)
           tma_load_2d(base + t * kTileBytes + c * kBlock, &qmap, c * 64, (int)(matrix_row + t * kAttnRows), q_full);
-      // K0 V0 K1 V1 ...; a block is two boxes of 64 keys per 64 elements. Keys past a row's position are masked, keys past
-      // the sequence arrive as zeros.
-      int slot = 0;
-      unsigned phase = 0;
-      for (int i = 0; i < 2 * blocks; i++) {
-        if (i >= kAttnSlots && !mbar_wait(&slot_empty[slot], phase ^ 1, budget)) {
-          // The copies in flight get a bounded time to land before the CTA leaves.
-          for (int r = 1; r <= kAttnSlots; r++) {
-            const int j = i - r;
-            for (unsigned spin = 0; spin < (1u << 16) && !mbar_try_wait(&slot_full[j % kAttnSlots], (unsigned)(j / kAttnSlots) & 1u); spin++) {
-            }
+    }
+    __syncwarp();
+    // K0 V0 K1 V1 ...; a block is two boxes of 64 keys per 64 elements. Keys past a row's position are masked, keys past
+    // the sequence arrive as zeros.
+    int slot = 0;
+    unsigned phase = 0;
+    for (int i = 0; i < 2 * blocks; i++) {
+      if (i >= kAttnSlots && !__all_sync(0xffffffffu, mbar_wait(&slot_empty[slot], phase ^ 1, budget))) {
+        // The copies in flight get a bounded time to land before the CTA leaves.
+        for (int r = 1; r <= kAttnSlots && leader; r++) {
+          const int j = i - r;
+          for (unsigned spin = 0; spin < (1u << 16) && !mbar_try_wait(&slot_full[j % kAttnSlots], (unsigned)(j / kAttnSlots) & 1u); spin++) {
           }
-          break;
         }
+        break;
+      }
+      if (leader) {
         const CUtensorMap* map = (i & 1) ? &vmap : &kmap;
         const uint32_t dst = ring + (uint32_t)slot * kSlotBytes;
         const int key0 = (i >> 1) * kAttnKeys;
         mbar_expect_tx(&slot_full[slot], kSlotBytes);
         for (int c = 0; c < kHalves; c++)
           for (int h = 0; h < 2; h++) tma_load_4d(dst + c * kBlock + h * (kBlock / 2), map, c * 64, key0 + h * 64, g, b, &slot_full[slot]);
-        if (++slot == kAttnSlots) {
-          slot = 0;
-          phase ^= 1;
-        }
+      }
+      __syncwarp();
+      if (++slot == kAttnSlots) {
+        slot = 0;
+        phase ^= 1;
       }
     }
+    __syncwarp();
   } else if (warp == kMmaWarp) {
-    if (lane == 0) {
-      // N = 128 keys with K as a K-major B operand; N = head_dim with V as an MN-major one (bit 16).
-      const uint32_t idesc_s = instr_desc(BF16, kAttnKeys, 0);
-      const uint32_t idesc_o = instr_desc(BF16, HD, 0) | 1u << 16;
-      int slot = 0;
-      unsigned phase = 0;
-      auto next_slot = [&]() {
-        const int s = slot;
-        if (++slot == kAttnSlots) {
-          slot = 0;
-          phase ^= 1;
-        }
-        return s;
-      };
-      auto scores = [&](int t, uint32_t k) {
+    // N = 128 keys with K as a K-major B operand; N = head_dim with V as an MN-major one (bit 16).
+    const uint32_t idesc_s = instr_desc(BF16, kAttnKeys, 0);
+    const uint32_t idesc_o = instr_desc(BF16, HD, 0) | 1u << 16;
+    const uint64_t q_first = smem_desc(base, 16, 1024), k_first = smem_desc(ring, 16, 1024), v_first = smem_desc(ring, kBlock, 1024);
+    int slot = 0;
+    unsigned phase = 0;
+    auto next_slot = [&]() {
+      const int s = slot;
+      if (++slot == kAttnSlots) {
+        slot = 0;
+        phase ^= 1;
+      }
+      return s;
+    };
+    auto wait = [&](uint64_t* bar, unsigned parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity, budget)) != 0; };
+    // Issued by the elected thread.
+    auto scores = [&](int t, int k_slot) {
+      const uint64_t q = desc_advance(q_first, t * kTileBytes), k = desc_advance(k_first, (uint32_t)k_slot * kSlotBytes);
 #pragma unroll
-        for (int kk = 0; kk < HD / 16; kk++) {
-          const uint32_t at = (uint32_t)(kk >> 2) * kBlock + (uint32_t)(kk & 3) * 32u;
-          mma_f16(s_col(t), smem_desc(base + t * kTileBytes + at, 16, 1024), smem_desc(k + at, 16, 1024), idesc_s, kk ? 1u : 0u);
-        }
-        mma_commit(&s_full[t]);
-      };
-      auto values = [&](int t, uint32_t v, bool accumulate) {
+      for (int kk = 0; kk < HD / 16; kk++) {
+        const uint32_t at = (uint32_t)(kk >> 2) * kBlock + (uint32_t)(kk & 3) * 32u;
+        mma_f16(s_col(t), desc_advance(q, at), desc_advance(k, at), idesc_s, kk ? 1u : 0u);
+      }
+      mma_commit(&s_full[t]);
+    };
+    auto values = [&](int t, int v_slot, bool accumulate) {
+      const uint64_t v = desc_advance(v_first, (uint32_t)v_slot * kSlotBytes);
 #pragma unroll
-        for (int kk = 0; kk < kAttnKeys / 16; kk++)
-          mma_f16_tmem_a(o_col(t), s_col(t) + (uint32_t)kk * 8u, smem_desc(v + (uint32_t)kk * 2048u, kBlock, 1024), idesc_o,
-                         (accumulate || kk) ? 1u : 0u);
-      };
-      bool ok = mbar_wait(q_full, 0, budget) && mbar_wait(&slot_full[0], 0, budget);
-      if (ok) {
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        for (int t = 0; t < TILES; t++) scores(t, ring);
+      for (int kk = 0; kk < kAttnKeys / 16; kk++)
+        mma_f16_tmem_a(o_col(t), s_col(t) + (uint32_t)kk * 8u, desc_advance(v, (uint32_t)kk * 2048u), idesc_o, (accumulate || kk) ? 1u : 0u);
+    };
+    bool ok = wait(q_full, 0) && wait(&slot_full[0], 0);
+    if (ok) {
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      if (leader) {
+        for (int t = 0; t < TILES; t++) scores(t, 0);
         mma_commit(&slot_empty[0]);
-        next_slot();
       }
-      for (int j = 0; j < blocks && ok; j++) {
-        const unsigned v_phase = phase;
-        const int v_slot = next_slot();
-        const unsigned k_phase = phase;
-        const bool more = j + 1 < blocks;
-        const int k_slot = more ? next_slot() : 0;
-        ok = mbar_wait(&slot_full[v_slot], v_phase, budget);
-        for (int t = 0; t < TILES && ok; t++) {
-          ok = mbar_wait(&p_ready[t], (unsigned)j & 1u, budget) && (!more || t > 0 || mbar_wait(&slot_full[k_slot], k_phase, budget));
-          if (!ok) break;
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          values(t, ring + (uint32_t)v_slot * kSlotBytes, j > 0);
-          if (more) scores(t, ring + (uint32_t)k_slot * kSlotBytes);
-          else mma_commit(&o_full[t]);
-        }
-        if (ok) {
-          mma_commit(&slot_empty[v_slot]);
-          if (more) mma_commit(&slot_empty[k_slot]);
-        }
-      }
-      if (!ok && p.error_flag) atomicExch(p.error_flag, 8);
+      __syncwarp();
+      next_slot();
     }
+    for (int j = 0; j < blocks && ok; j++) {
+      const unsigned v_phase = phase;
+      const int v_slot = next_slot();
+      const unsigned k_phase = phase;
+      const bool more = j + 1 < blocks;
+      const int k_slot = more ? next_slot() : 0;
+      ok = wait(&slot_full[v_slot], v_phase);
+#pragma unroll
+      for (int t = 0; t < TILES; t++) {
+        ok = ok && wait(&p_ready[t], (unsigned)j & 1u) && (!more || t > 0 || wait(&slot_full[k_slot], k_phase));
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if (leader) {
+          values(t, v_slot, j > 0);
+          if (more) scores(t, k_slot);
+          else mma_commit(&o_full[t]);
+          if (t + 1 == TILES) {
+            mma_commit(&slot_empty[v_slot]);
+            if (more) mma_commit(&slot_empty[k_slot]);
+          }
+        }
+        __syncwarp();
+      }
+    }
+    if (!ok && leader && p.error_flag) atomicExch(p.error_flag, 8);
+    __syncwarp();
   } else {
     const int t = warp >> 2;
     const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
@@ -343,7 +361,8 @@ umma_attention_kernel(const AttnParams p, const __grid_constant__ CUtensorMap qm
     if (ok) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const float inv = sum > 0.f ? 1.f / sum : sum != sum ? sum : 0.f;
-      uint4* dst = reinterpret_cast<uint4*>(static_cast<unsigned short*>(out) + (((long long)b * p.kv_heads + g) * p.rows + row) * HD);
+      const long long at = b * p.out_batch + g * p.out_head + row / p.rep * p.out_pos + row % p.rep * HD;
+      uint4* dst = reinterpret_cast<uint4*>(static_cast<unsigned short*>(out) + at);
 #pragma unroll
       for (int c = 0; c < HD; c += 32) {
         float o[32];

@@ -837,3 +837,20 @@ def test_decode_attention_of_one_and_two_heads_per_kv_head(gpu_backend, dtype, h
     hit[1, 0, :heads // kv_heads, 5] = True
     assert np.isfinite(got[~hit]).all() and np.isin(got[hit], [np.inf]).all()
     exe.destroy()
+
+
+@pytest.mark.parametrize("dtype,kv_heads,rep,seq,hd", [(P.BF16_CODE, 8, 4, 517, 128), (P.F16, 3, 1, 130, 64), (P.BF16_CODE, 37, 3, 300, 128)])
+def test_prefill_attention_stores_what_a_transpose_would(gpu_backend, dtype, kv_heads, rep, seq, hd):
+    """A result that is only read as [batch, seq, kv_heads, rep, head_dim] is stored so, bit for bit what the transpose of the
+    other layout gives; one that is an output itself keeps its layout and its transpose."""
+    b, args = cases.prefill_attention(dtype=dtype, batch=2, kv_heads=kv_heads, rep=rep, seq=seq, head_dim=hd)
+    plain = run_backend(gpu_backend, b, args)[0]
+    out = P.Val(b, b.output_ids[0])
+    turned = b.transpose(out, [0, 2, 1, 3, 4])
+    for outputs, steps in (([turned], 1), ([out, turned], 2)):
+        b.set_outputs(outputs)
+        exe = gpu_backend.compile_executable(b, [0])
+        assert len(exe.describe()["kernel_plan"]["steps"]) == steps
+        got = run_backend(gpu_backend, b, args, exe=exe)
+        assert np.array_equal(got[-1].view(np.uint16), np.ascontiguousarray(plain.transpose(0, 2, 1, 3, 4)).view(np.uint16))
+        assert len(got) == 1 or np.array_equal(got[0].view(np.uint16), plain.view(np.uint16))
