@@ -1546,8 +1546,8 @@ std::string describe_steps(const KernelPlan& kp, bool with_source) {
         n_total = 0;
         for (const DotShape& d : st.dot_group) n_total += d.n;
       }
-      s += strfmt(",\"path\":%d,\"tma\":%d,\"umma\":%d,\"pair\":%d,\"small\":%d,\"m_tile\":%d,\"stages\":%d,\"smem\":%llu,\"tmem\":%d,\"ordered\":%d,\"grid\":%d,\"ksplit\":%d,\"b0\":%lld,\"b1\":%lld,\"m\":%lld,\"n\":%lld,\"k\":%lld,\"group\":%zu",
-                  st.dot_scratch.path, st.dot_scratch.tma, st.dot_scratch.umma, st.dot_scratch.pair, st.dot_scratch.small, st.dot_scratch.m_tile, st.dot_scratch.stages, (unsigned long long)st.dot_scratch.smem, st.dot_scratch.tmem, st.dot_scratch.ordered, st.dot_scratch.grid, st.dot_scratch.ksplit, (long long)st.dot.b0, (long long)st.dot.b1, (long long)st.dot.m,
+      s += strfmt(",\"path\":%d,\"tma\":%d,\"umma\":%d,\"pair\":%d,\"shift\":%d,\"small\":%d,\"m_tile\":%d,\"stages\":%d,\"smem\":%llu,\"tmem\":%d,\"ordered\":%d,\"grid\":%d,\"ksplit\":%d,\"b0\":%lld,\"b1\":%lld,\"m\":%lld,\"n\":%lld,\"k\":%lld,\"group\":%zu",
+                  st.dot_scratch.path, st.dot_scratch.tma, st.dot_scratch.umma, st.dot_scratch.pair, st.dot_scratch.shift, st.dot_scratch.small, st.dot_scratch.m_tile, st.dot_scratch.stages, (unsigned long long)st.dot_scratch.smem, st.dot_scratch.tmem, st.dot_scratch.ordered, st.dot_scratch.grid, st.dot_scratch.ksplit, (long long)st.dot.b0, (long long)st.dot.b1, (long long)st.dot.m,
                   n_total, (long long)st.dot.k, std::max<size_t>(st.dot_group.size(), 1));
       long long weight_elems = 0;
       if (st.segs.empty()) {

@@ -101,8 +101,9 @@ struct DotScratch {
   // Paths 1 and 4 for 16-bit floats without batch axes can run on the tensor cores (tcgen05, accumulator in TMEM); path 5
   // always does. `ksplit` CTAs of a cluster then share a tile of 128 columns x m_tile rows, contracting 1/ksplit of k each;
   // nothing goes through scratch memory.
-  // `pair`: CTA pairs work on tiles of 256 columns (umma_pair.cuh).
-  int umma = 0, m_tile = 0, sub = 1, pair = 0;
+  // `pair`: CTA pairs work on tiles of 256 columns (umma_pair.cuh). `shift`: path 5 by residues of the rows (umma_shift.cuh),
+  // so many of them; the rearranged lhs takes `partial_bytes`.
+  int umma = 0, m_tile = 0, sub = 1, pair = 0, shift = 0;
   // Tensor-memory columns of a CTA, and whether the launch waits for its predecessor to complete whatever the stream's
   // setting for programmatic dependent launch.
   int tmem = 0, ordered = 0;

@@ -854,3 +854,40 @@ def test_prefill_attention_stores_what_a_transpose_would(gpu_backend, dtype, kv_
         got = run_backend(gpu_backend, b, args, exe=exe)
         assert np.array_equal(got[-1].view(np.uint16), np.ascontiguousarray(plain.transpose(0, 2, 1, 3, 4)).view(np.uint16))
         assert len(got) == 1 or np.array_equal(got[0].view(np.uint16), plain.view(np.uint16))
+
+
+@pytest.mark.parametrize("dtype", [P.BF16_CODE, P.F16])
+@pytest.mark.parametrize("m,k,n,residues", [
+    (1, 64, 800 * 120 + 1, 8),    # one block of eight rows per residue, one result in the last tile
+    (16, 136, 44999, 8),          # residues of 17 rows
+    (5, 2048, 3001, 8),           # the fewest columns
+    (5, 2048, 36001, 8),          # more tiles than CTAs: both sets of accumulators
+    (17, 520, 12001, 8),          # 32 rows of activations, two blocks per residue, the second of one row
+    (32, 520, 12002, 4),
+    (3, 1000, 6004, 2),
+])
+def test_unaligned_weight_rows_by_residue_against_f64(gpu_backend, dtype, m, k, n, residues):
+    """Weight rows without a 16-byte pitch as matrices of every second, fourth or eighth row. Error bound as for the aligned
+    rows: f32 sums and one rounding of the output. An infinite weight shows in its own column only."""
+    rng = np.random.default_rng(m * 31 + n)
+    dt = P.np_dtype(dtype)
+    x = rng.standard_normal((m, k), dtype=np.float32).astype(dt)
+    w = rng.standard_normal((k, n), dtype=np.float32).astype(dt)
+    b = PlanBuilder()
+    b.set_outputs([b.dot_general(b.parameter(dtype, x.shape), b.parameter(dtype, w.shape), [1], [0])])
+    exe = gpu_backend.compile_executable(b, [0])
+    step = exe.describe()["kernel_plan"]["steps"][0]
+    assert step["path"] == 5 and step["shift"] == residues, step
+    got, again = (run_backend(gpu_backend, b, [x, w], exe=exe)[0] for _ in range(2))
+    assert np.array_equal(got.view(np.uint16), again.view(np.uint16))
+    want = x.astype(np.float64) @ w.astype(np.float64)
+    mag = np.abs(x.astype(np.float64)) @ np.abs(w.astype(np.float64))
+    ulp = 2.0 ** (-9 if dtype == P.BF16_CODE else -12)
+    assert np.all(np.abs(got.astype(np.float64) - want) <= 2 * ulp * np.abs(want) + k * 2.0 ** -24 * mag + 2.0 ** -24)
+    columns = [0, 7, 119, 120, 127, 128, 240, n - 1]
+    for i, c in enumerate(columns):
+        w[(i * 11) % k, c] = np.inf
+    got = run_backend(gpu_backend, b, [x, w], exe=exe)[0].astype(np.float64)
+    exe.destroy()
+    hit = np.isin(np.arange(n), columns)
+    assert not np.isfinite(got[:, hit]).any() and np.isfinite(got[:, ~hit]).all()
