@@ -52,8 +52,8 @@
 //            (widen_byte_pair). 16 rows, us, before these and the issue above, and now: 4096 x 28672 40.9 / 33.3, 14336 x
 //            4096 30.8 / 26.1, 8192 x 57344 114 / 94.5, 4096 x 128256 119.5 / 102 (5.2 TB/s).
 //   kLoose   16-bit weights of any pitch and alignment (an odd vocabulary, say): converter warps read them with plain
-//            loads, one column per thread, and write them to TMEM. TMA cannot describe such rows. 5 x 2048 x 32001 f16: 85 us
-//            (one thread per output before: 739), 1.6 TB/s; the converters' ALU is 65 % busy and waits for 2-byte loads.
+//            loads, one column per thread, and write them to TMEM, at 1.6 TB/s: the converters' ALU is 65 % busy and waits for
+//            2-byte loads. Few rows of large weights go by residues instead (umma_shift.cuh).
 //
 // Programmatic dependent launch: weights are never written by earlier work of the stream (`early_rhs`), so their
 // copies for the first ring of stages are issued before griddepcontrol.wait; activation copies and all stores wait.

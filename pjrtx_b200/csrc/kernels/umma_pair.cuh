@@ -8,16 +8,20 @@
 // tensor cores read the other half from the peer, so an SM moves 8 KiB in and 8 KiB out per 128 cycles.
 //
 // One persistent cluster of two CTAs per pair of SMs. Both CTAs run the same roles, CTA 0 leads:
-//   producer lane   (each CTA) copies its 128 weight columns and its m_tile / 2 activation rows into its own ring; the
+//   copy warp       (each CTA) copies its 128 weight columns and its m_tile / 2 activation rows into its own ring; the
 //                   bytes of both CTAs are counted on the leader's `full` mbarrier
-//   MMA lane        (leader) issues tcgen05.mma.cta_group::2 (M = 256, N = m_tile, K = 16); the commits release the stage
+//   MMA warp        (leader) issues tcgen05.mma.cta_group::2 (M = 256, N = m_tile, K = 16); the commits release the stage
 //                   (`empty`) and publish the accumulator (`acc_full`) in both CTAs
 //   epilogue warps  (each CTA) drain the CTA's own 128 rows of the accumulator (two accumulators: the next tile's MMAs
 //                   run meanwhile) and tell the leader (`acc_empty`)
 // Tiles are dealt out in bands of kBand weight tiles, activations fastest inside a band, so that the tiles in flight on the
 // chip form a compact block and share both operands through L2.
 //
-// Measured, 8192 rows, bf16, one SM per tile and pairs: 4096 x 28672 2030 / 1340 us (1433 TFLOP/s), 14336 x 4096 880 / 648 us,
+// Both warps run converged and let an elected thread issue (elect_one in umma_gemm.cuh); by a single thread a 64-deep unit took
+// 300 ns and 0.5 ns per row, now 195 and 0.57: 517 rows, us, before and now, 14336 x 4096 85 / 71.5, 4096 x 28672 120 / 109, 4096 x
+// 4096 35.5 / 31; 2048 rows, 4096 x 28672 332 / 315 (1527 TFLOP/s).
+//
+// Measured before that, 8192 rows, bf16, one SM per tile and pairs: 4096 x 28672 2030 / 1340 us (1433 TFLOP/s), 14336 x 4096 880 / 648 us,
 // 4096 x 6144 429 / 310 us, 4096 x 4096 291 / 211 us. Inside a full-depth prefill, under the power cap and with the launch
 // ordered after its predecessor: 1382, 675, 325 and 220 us.
 //
