@@ -1124,6 +1124,9 @@ int launch_chain(const DotChainSegment* segs, const DotChainArgs* args, int n, c
 
 // 0: not eligible, 1: rhs[K,N] with N contiguous, 2: rhs[N,K] with K contiguous, 3: rhs[K,N] with N contiguous whose rows
 // the tensor maps cannot describe. Tensor maps need 16-byte multiples for every row stride; lhs must be k-contiguous.
+// Int8 weights of a million and more have no lower bound on m: the alternative writes the dequantised weights out and reads
+// them again (one row, us, so and here: 1024 x 1024 17.3 / 12, 4096 x 1024 14.3 / 12.1, 4096 x 4096 22.6 / 16, 14336 x 4096 56 / 25,
+// 4096 x 32000 122 / 33).
 // Case 3 (odd vocabularies) has no lower bound on m: the alternative is one thread per output (path 0) or 64 x 64 tiles on
 // the CUDA cores (path 3). Measured, 5 x 2048 x 32001 f16: 739 us on path 0. Below 64 columns or a k of 64 a tile would be
 // mostly padding and the other paths stay.
@@ -1136,7 +1139,7 @@ int umma_eligible(const DotShape& s) {
   if (s.m > (1 << 20) || s.n > (1ll << 30) || s.k > (1ll << 30)) return 0;
   const bool pitch_ok = s.rhs_s8 ? s.rhs_k % 16 == 0 : s.rhs_k % 8 == 0;
   if (s.rhs_n == 1 && s.rhs_k >= s.n) {
-    if (pitch_ok) return s.m >= min_m ? 1 : 0;
+    if (pitch_ok) return s.m >= min_m || (s.rhs_s8 && s.k * s.n >= (1 << 20)) ? 1 : 0;
     return s.n >= 64 && s.k >= 64 && !s.rhs_s8 ? 3 : 0;
   }
   if (s.rhs_s8 || s.m < min_m) return 0;
