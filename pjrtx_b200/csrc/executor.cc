@@ -2176,8 +2176,9 @@ bool execute_executable(Executable* exe, size_t device_index, Buffer* const* arg
     }
     const void* src = st.kind == Storage::kParameter && param_taken[st.index] ? nullptr : ptr.of(ov.id);
     if (st.kind == Storage::kParameter && param_taken[st.index]) {
-      // A second output aliasing an already transferred argument: copy from the first one.
-      for (size_t q = 0; q < o; q++)
+      // Further outputs aliasing an already transferred argument copy from the one that took it over, the first with that
+      // root: the others are destinations of this very batch, whose copies have no order.
+      for (size_t q = 0; q < o && !src; q++)
         if (kp.root[plan.output_ids[q]] == r) src = outs[q]->ptr;
     }
     if (src) results.push_back({src, b->ptr, b->bytes});

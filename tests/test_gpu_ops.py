@@ -238,6 +238,39 @@ def test_donated_slice_update_is_in_place(gpu_backend):
     assert np.array_equal(got[:, 15].view(np.uint16), u[:, 0].view(np.uint16))
 
 
+@pytest.mark.parametrize("graph", [True, False])
+@pytest.mark.parametrize("shape", [(2, 16, 2, 8), (3, 40001)])  # one block's piece of a copy, and fifteen
+def test_results_that_share_one_donated_argument(gpu_backend, graph, shape):
+    """A donated argument (updated in place, and as it came) listed several times as a result, through reshapes too: the first
+    result takes the buffer over, every other one holds a copy of it, byte for byte, whatever order the copies run in."""
+    be = gpu_backend
+    rng = np.random.default_rng(len(shape))
+    b = PlanBuilder()
+    cache, kept = b.parameter(P.F32, shape), b.parameter(P.F32, shape)
+    upd, pos = b.parameter(P.F32, (1,) + shape[1:]), b.parameter(P.S32, [])
+    zero = b.constant(np.int32(0))
+    out = b.dynamic_update_slice(cache, upd, [pos] + [zero] * (len(shape) - 1))
+    flat = b.reshape(out, [int(np.prod(shape))])
+    x = y = b.parameter(P.F32, (2, 2))
+    for _ in range(4 if graph else 1):
+        y = b.matmul(y, x)
+    b.set_outputs([out, flat, out, kept, kept, b.reshape(out, shape), kept, flat, y], donate={0: 0, 3: 1})
+    exe = be.compile_executable(b, [0])
+    for row in (0, shape[0] - 1):
+        args = [rng.standard_normal(v.dims, dtype=np.float32) if v.dims else np.array(row, np.int32)
+                for v in (cache, kept, upd, pos)] + [rng.integers(-2, 3, (2, 2)).astype(np.float32)]
+        updated = args[0].copy()
+        updated[row] = args[2][0]
+        want = [updated, updated.ravel(), updated, args[1], args[1], updated, args[1], updated.ravel(),
+                np.linalg.matrix_power(args[4], 5 if graph else 2)]
+        got = run_backend(be, b, args, exe=exe)
+        for i, (g, w) in enumerate(zip(got, want)):
+            assert np.array_equal(g, w), i
+    stats = exe.stats()
+    assert stats["donation_alias_output_count"] == 4 and stats["graph_launch_count"] == (2 if graph else 0)
+    exe.destroy()
+
+
 def test_slice_updates_ride_in_the_producing_kernel(gpu_backend):
     """Two in-place updates of different donated buffers computed and stored by one generated kernel: one writes whole
     trailing rows (vector stores), the other a window inside the innermost axis (scalar stores); start indices clamp."""
