@@ -87,8 +87,13 @@ enum Source { kTile = 0, kBytes = 1, kLoose = 2 };
 // bytes in flight are theirs), two where TMA brings the bytes.
 __host__ __device__ constexpr int converter_warps(int src) { return src == kTile ? 0 : src == kBytes ? 8 : 16; }
 __host__ __device__ constexpr int threads_of(int src) { return kBaseThreads + 32 * converter_warps(src); }
-// Weight operand tiles in TMEM (sources other than kTile), 32 * SUB columns each.
+// Weight operand tiles in TMEM (sources other than kTile), 32 * SUB columns each. kBytes: a warp converts every second unit only
+// and therefore sees every second phase of the barriers that the units in between share with its own, where a parity that is
+// one phase behind counts as complete. What keeps it from that: unit i's slot is free once the products of unit i - kOperandSlots
+// are done, so all units up to there have landed, and those are all earlier users of its stage that the warp has not waited
+// for itself (a ring of two stages has its own units only). So a warp waits for the slot first, then for the stage.
 constexpr int kOperandSlots = 3;
+static_assert(kOperandSlots <= 3, "a ring of three stages relies on it");
 
 struct Params {
   int m, k;
@@ -668,7 +673,7 @@ __global__ void __launch_bounds__(threads_of(SRC), SRC == kLoose ? 1 : 2) umma_s
         next_slot();
       }
       for (int i = part; i < count; i += 2) {
-        const bool ok = mbar_wait(&full[stage], phase, budget) && slot_free(i);
+        const bool ok = slot_free(i) && mbar_wait(&full[stage], phase, budget);  // in this order (kOperandSlots)
         if (!__all_sync(0xffffffffu, ok)) {
           if (lane == 0) atomicExch(p.error_flag, 15);
           break;

@@ -598,6 +598,43 @@ def test_int8_contractions_of_tall_tiles_against_f64(gpu_backend, m, k, n, count
         assert np.all(np.abs(g.astype(np.float64) - want) <= 2 * ulp * np.abs(want) + k * 2.0 ** -24 * mag + 2.0 ** -24)
 
 
+@pytest.mark.parametrize("m,k,n,dtype", [(113, 4096, 6144, P.BF16_CODE), (97, 14336, 4096, P.F16), (192, 4096, 6144, P.F16)])
+def test_int8_rings_of_three_stages_repeat_exactly(gpu_backend, m, k, n, dtype):
+    """The two converter warps of a quarter take units in turn; in a ring of three stages a unit's stage was the other warp's
+    before. 320 launches on weights that come from HBM (more of them than L2 holds), queued forty at a time: every result is
+    the first one of its weights bit for bit, and that one is the exact product to the tall tiles' bound."""
+    rng = np.random.default_rng(m)
+    be, dt = gpu_backend, P.np_dtype(dtype)
+    x = rng.standard_normal((m, k), dtype=np.float32).astype(dt)
+    sc = (rng.uniform(0.5, 1.5, size=(n,)) / 127 / np.sqrt(k)).astype(np.float16)
+    b = PlanBuilder()
+    px, pw = b.parameter(dtype, x.shape), b.parameter(P.S8, (k, n))
+    wf = b.convert(pw, P.F16) * b.broadcast_in_dim(b.parameter(P.F16, sc.shape), [k, n], [1])
+    b.set_outputs([b.dot_general(px, wf if dtype == P.F16 else b.convert(wf, dtype), [1], [0])])
+    exe = be.compile_executable(b, [0])
+    (step,) = [s for s in exe.describe()["kernel_plan"]["steps"] if s["type"] == "dot"]
+    assert step["rhs_s8"] == 1 and step["stages"] == 3, step
+    weights = [rng.integers(-127, 128, size=(k, n), dtype=np.int8) for _ in range(2)]
+    held = [be.buffer_from_host(w) for w in weights]
+    copies = held + [be.clone_buffer(held[i % 2]) for i in range(2, 8)]
+    bx, bs = be.buffer_from_host(x), be.buffer_from_host(sc)
+    first = [None, None]
+    for _ in range(8):
+        outs = [be.execute_executable(exe, [bx, copies[i % 8], bs])[0] for i in range(40)]
+        for i, o in enumerate(outs):
+            got = o.to_numpy().view(np.uint16)
+            o.destroy()
+            if first[i % 2] is None:
+                first[i % 2] = got
+            assert np.array_equal(got, first[i % 2])
+    exe.destroy()
+    x64, ulp = x.astype(np.float64), 2.0 ** (-9 if dtype == P.BF16_CODE else -12)
+    for bits, w8 in zip(first, weights):
+        w = w8.astype(np.float64) * sc.astype(np.float64)
+        want, mag = x64 @ w, np.abs(x64) @ np.abs(w)
+        assert np.all(np.abs(bits.view(dt).astype(np.float64) - want) <= 2 * ulp * np.abs(want) + k * 2.0 ** -24 * mag + 2.0 ** -24)
+
+
 @pytest.mark.parametrize("dtype", [P.BF16_CODE, P.F16])
 @pytest.mark.parametrize("m,k,n,count", [
     (3, 128, 128, 1),      # one tile, two 64-deep blocks

@@ -1,6 +1,7 @@
 """Host logic on CPU: C-ABI exports, plan verifier, program graph counters, legalization, kernel planner, codegen."""
 import ctypes
 import os
+import random
 import re
 
 import numpy as np
@@ -420,6 +421,55 @@ def test_every_planned_contraction_fits_an_sm(backend, source):
         for k, n in widths + [(4096, 14336)]:
             for st in _contraction(backend, source, m, k, n, group=2 if n == 14336 else 1):
                 assert st["smem"] <= 227 * 1024 and st["stages"] >= 2 and st["ksplit"] <= (k + 127) // 128, st
+
+
+@pytest.mark.parametrize("stages", [2, 3, 4, 5, 7, 12])
+def test_int8_converters_never_read_a_stage_before_its_unit_has_landed(stages):
+    """The barriers of the int8 ring as counters, its copies landing in any order: a unit's copy, the two converters that take
+    units in turn, the products that release stage and operand slot. The order of a converter's two waits and the number of
+    slots are the kernel's own."""
+    kernels = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "pjrtx_b200", "csrc", "kernels")
+    with open(os.path.join(kernels, "umma_gemm.cuh")) as f:
+        text = f.read()
+    slots = int(re.search(r"constexpr int kOperandSlots = (\d+);", text).group(1))
+    waits = re.search(r"for \(int i = part; i < count; i \+= 2\) \{\s*const bool ok = (.*?) && (.*?);", text).groups()
+    waits = ["slot" if w.startswith("slot_free(i)") else "stage" if w.startswith("mbar_wait(&full[stage], phase, budget)") else w for w in waits]
+    assert sorted(waits) == ["slot", "stage"]
+    units = 24
+    complete = lambda phases, parity: phases & 1 != parity  # try_wait.parity: of the phase before, too
+    for seed in range(400):
+        rng = random.Random(seed)
+        full, empty, ready, released = [0] * stages, [0] * stages, [0] * slots, [0] * slots
+        requested, landed, in_flight, products, at, passed = 0, set(), [], 0, [0, 1], [0, 0]
+        while products < units:
+            can = [("land", u) for u in in_flight]
+            if requested < units and (requested < stages or complete(empty[requested % stages], (requested // stages & 1) ^ 1)):
+                can.append(("request", requested))
+            for part, i in enumerate(at):
+                free = i < slots or complete(released[i % slots], (i // slots & 1) ^ 1)
+                if i < units and (free if waits[passed[part]] == "slot" else complete(full[i % stages], i // stages & 1)):
+                    can.append(("convert", part))
+            if complete(full[products % stages], products // stages & 1) and complete(ready[products % slots], products // slots & 1):
+                can.append(("product", products))
+            what, which = rng.choice(can)  # an empty list would be a ring that is stuck
+            if what == "request":
+                in_flight.append(which)
+                requested += 1
+            elif what == "land":
+                in_flight.remove(which)
+                landed.add(which)
+                full[which % stages] += 1
+            elif what == "product":
+                empty[which % stages] += 1
+                released[which % slots] += 1
+                products += 1
+            elif passed[which] == 0:
+                passed[which] = 1
+            else:
+                assert at[which] in landed, (stages, seed, at[which])
+                ready[at[which] % slots] += 1
+                at[which] += 2
+                passed[which] = 0
 
 
 def test_error_word_codes_belong_to_one_kernel_each():
