@@ -692,14 +692,16 @@ attn_decode_staged_kernel(DecodeArgs a, const T* __restrict__ q, const T* __rest
 // are equal, and row j multiplies the j-th 16-bit part of the probability (p = hi + mid + lo, each part the rounding of
 // what the ones before it leave), so that the three products add up to that of the f32 probability. The sum of the
 // probabilities is that of the f32 values. f16 has no exponents for the small parts of a probability at most 1: its
-// probabilities are 2^12 times as large, their sum with them. Against the CUDA-core kernel (8 KV heads of 128, two query
+// probabilities are 2^12 times as large, their sum with them, and what is below 2^-37 of the warp's largest has no part left. A
+// fourth row with a one for every probability above zero stands in where V is not finite, since 0 * infinity would be NaN
+// there and p * infinity is infinity. Against the CUDA-core kernel (8 KV heads of 128, two query
 // heads each, us, both with the same distance from 64-bit results to four digits): 5 sequences of 777 keys 18.8 -> 14.7,
 // of 4096 41 -> 24.7; 16 of 2048 53.5 -> 31; 32 of 4096 129 -> 82 (6.5 TB/s); up to 256 keys the two take the same.
 constexpr int kMmaWarps = 4;
 constexpr int kMmaStageKeys = 16 * kMmaWarps;
-// Parts of a probability (rows per query head) and rows of Q.
-__host__ __device__ constexpr int mma_parts(int rep) { return rep <= 2 ? 3 : 1; }
-__host__ __device__ constexpr int mma_rows(int rep) { return rep * mma_parts(rep); }
+// Rows of Q: three parts of a probability and the row of ones per query head, or the head's alone.
+__host__ __device__ constexpr bool mma_in_parts(int rep) { return rep <= 2; }
+__host__ __device__ constexpr int mma_rows(int rep) { return mma_in_parts(rep) ? 4 * rep : rep; }
 
 template <typename T> struct MmaOps;
 template <> struct MmaOps<__nv_bfloat16> {
@@ -733,6 +735,11 @@ __device__ __forceinline__ void ldmatrix_x4_trans(unsigned* r, unsigned smem_add
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_addr));
 }
+__device__ __forceinline__ float min_or_nan(float a, float b) {
+  float r;
+  asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
 // STAGES = 3: two CTAs per SM, two stages in flight each. (A two-stage ring with three CTAs per SM and a third more
 // splits was measured on thirty-two (sequence, KV head) pairs of 4K keys: no faster.)
 template <typename T, int REP, int HD, int STAGES>
@@ -744,9 +751,10 @@ attn_decode_mma_kernel(DecodeArgs a, const T* __restrict__ q, const __grid_const
   constexpr int HALVES = HD / 64;                     // 128-byte column blocks per row
   constexpr int TILE_BYTES = kMmaStageKeys * HD * 2;  // one of K or V for one stage
   constexpr int STAGE_BYTES = 2 * TILE_BYTES;
-  constexpr int PARTS = mma_parts(REP), ROWS = mma_rows(REP);
+  constexpr bool IN_PARTS = mma_in_parts(REP);
+  constexpr int ROWS = mma_rows(REP);
   constexpr int HALF_ROWS = ROWS <= 8 ? 1 : 2;        // rows 8 to 15 of the fragments are used only beyond eight
-  constexpr float P_SCALE = PARTS > 1 && std::is_same<T, __half>::value ? 4096.f : 1.f;
+  constexpr float P_SCALE = IN_PARTS && std::is_same<T, __half>::value ? 4096.f : 1.f;
   // The swizzle of a tiled copy follows the absolute shared-memory address: tiles start on 1024-byte boundaries.
   extern __shared__ unsigned char smem_attn_raw[];
   unsigned char* smem_attn = smem_attn_raw + ((1024u - (attn_smem_u32(smem_attn_raw) & 1023u)) & 1023u);
@@ -836,7 +844,10 @@ attn_decode_mma_kernel(DecodeArgs a, const T* __restrict__ q, const __grid_const
       qa[ks][3] = r0 + 8 < ROWS ? __ldg(reinterpret_cast<const unsigned*>(qrow1 + ks * 16 + c0 + 8)) : 0u;
     }
   }
-  const int part = (lane >> 2) / REP;  // which part of the probability this thread's row multiplies
+  // Which part of the probability this thread's row multiplies, 3: the ones, min(2^126 * p, 1). As constants instead of selects.
+  const int part = (lane >> 2) / REP;
+  const float p_scale = IN_PARTS && part >= 3 ? 8.507059e37f : P_SCALE, p_most = IN_PARTS && part >= 3 ? 1.f : INFINITY;
+  const float minus_hi = part == 1 || part == 2 ? -1.f : 0.f, minus_mid = part == 2 ? -1.f : 0.f;
   float m_run[2] = {-INFINITY, -INFINITY}, l_part[2] = {0.f, 0.f};
   float o[HD / 8][4];
 #pragma unroll
@@ -940,17 +951,19 @@ attn_decode_mma_kernel(DecodeArgs a, const T* __restrict__ q, const __grid_const
 #pragma unroll
         for (int e = 0; e < 2; e++) {
           const float sv = sc[nt][2 * h + e];
-          p[nt * 2 + e] = sv == -INFINITY ? 0.f : __expf(sv - m_new) * P_SCALE;
+          p[nt * 2 + e] = sv == -INFINITY ? 0.f : __expf(sv - m_new);
         }
-      if (PARTS == 1) {
+      if (!IN_PARTS) {
         // The probabilities enter the second contraction in the element type; the row sum uses the same rounded values.
         l_part[h] += Elem<T>::round(p[0]) + Elem<T>::round(p[1]) + Elem<T>::round(p[2]) + Elem<T>::round(p[3]);
       } else {
+#pragma unroll
+        for (int e = 0; e < 4; e++) p[e] = min_or_nan(p[e] * p_scale, p_most);
         l_part[h] += (p[0] + p[1]) + (p[2] + p[3]);
 #pragma unroll
         for (int e = 0; e < 4; e++) {
-          const float rest = p[e] - Elem<T>::round(p[e]);
-          p[e] = part == 0 ? p[e] : part == 1 ? rest : rest - Elem<T>::round(rest);
+          const float rest = fmaf(minus_hi, Elem<T>::round(p[e]), p[e]);
+          p[e] = fmaf(minus_mid, Elem<T>::round(rest), rest);
         }
       }
       pa[h] = MmaOps<T>::pack(p[0], p[1]);       // keys 0-7 block
@@ -1031,9 +1044,13 @@ attn_decode_mma_kernel(DecodeArgs a, const T* __restrict__ q, const __grid_const
       const float mw = sm_m[w * 16 + r];
       const float wgt = mw == -INFINITY ? 0.f : __expf(mw - mm);
       float ow = sm_o[(w * ROWS + r) * HD + d];
-      // The smaller parts' products; of an infinite V element the largest part's alone is what the sum would be (the others
-      // may be 0 * infinity).
-      if (PARTS > 1 && fabsf(ow) <= 3.402823466e38f) ow += sm_o[(w * ROWS + REP + r) * HD + d] + sm_o[(w * ROWS + 2 * REP + r) * HD + d];
+      if (IN_PARTS) {
+        // A finite sum of the largest parts says that V is finite. Otherwise the sum over the ones is infinite or NaN as that of
+        // the probabilities is, unless V is finite and the sum has only grown too large.
+        const float* rest = sm_o + (w * ROWS + REP + r) * HD + d;
+        if (fabsf(ow) <= 3.402823466e38f) ow += rest[0] + rest[REP * HD];
+        else if (!(fabsf(rest[2 * REP * HD]) <= 3.402823466e38f)) ow = rest[2 * REP * HD];
+      }
       oo = fmaf(ow, wgt, oo);
       ll = fmaf(sm_l[w * 16 + r], wgt, ll);
     }

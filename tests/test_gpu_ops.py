@@ -909,6 +909,48 @@ def test_decode_attention_of_one_and_two_heads_per_kv_head(gpu_backend, dtype, h
     exe.destroy()
 
 
+@pytest.mark.parametrize("dtype", [P.BF16_CODE, P.F16])
+@pytest.mark.parametrize("heads,kv_heads", [(2, 2), (4, 2)])
+@pytest.mark.parametrize("kv_len", [80, 1200])  # one split and several
+def test_decode_attention_of_infinite_values_at_small_probabilities(gpu_backend, dtype, heads, kv_heads, kv_len):
+    """One key of every sixteen has score 0, the others -31: their probabilities, 2^-45, are f32 numbers without a 16-bit part
+    in f16. An infinite value there is an infinite result, infinities of both signs or a NaN are a NaN, and the finite
+    columns stay what they are (error as for other values)."""
+    hd, batch = 128, 2
+    rng = np.random.default_rng(kv_len)
+    dt = P.np_dtype(dtype)
+    q = np.zeros((batch, 1, heads, hd), np.float32)
+    q[..., 0] = 8
+    k = np.zeros((batch, kv_len, kv_heads, hd), np.float32)
+    k[..., 0] = -31 * np.sqrt(hd) / 8
+    k[:, 2::16, :, 0] = 0
+    q, k = q.astype(dt), k.astype(dt)
+    v = rng.standard_normal((batch, kv_len, kv_heads, hd)).astype(np.float32).astype(dt)
+    wide = np.abs(v.astype(np.float64)).max()
+    for key, column, value in [(5, 7, np.inf), (17, 9, -np.inf), (33, 11, np.inf), (77, 11, np.inf), (4, 13, np.inf), (70, 13, -np.inf),
+                               (40, 15, np.nan), (18, 17, np.inf)]:
+        v[1, key, 0, column] = value
+    b = PlanBuilder()
+    pq, pk, pv = b.parameter(dtype, q.shape), b.parameter(dtype, k.shape), b.parameter(dtype, v.shape)
+    pt = b.parameter(P.S32, [])
+    b.set_outputs([b.custom_call("pjrtx.b200.scaled_dot_product_attention", [pq, pk, pv, pt], dtype, q.shape)])
+    exe = gpu_backend.compile_executable(b, [0])
+    assert exe.describe()["kernel_plan"]["steps"][0]["mma"] == 1
+    got = run_backend(gpu_backend, b, [q, k, v, np.array(kv_len - 1, np.int32)], exe=exe)[0].astype(np.float64)
+    exe.destroy()
+    rep = heads // kv_heads
+    kk, vv = (np.repeat(x.astype(np.float64), rep, axis=2) for x in (k, v))
+    scores = np.einsum("bqhd,bkhd->bhk", q.astype(np.float64), kk) / np.sqrt(hd)
+    p = np.exp(scores - scores.max(axis=2, keepdims=True))
+    with np.errstate(invalid="ignore"):
+        want = np.einsum("bhk,bkhd->bhd", p / p.sum(axis=2, keepdims=True), vv)[:, None]
+    assert np.isinf(want).sum() == 4 * rep and np.isnan(want).sum() == 2 * rep
+    finite = np.isfinite(want)
+    assert np.array_equal(np.isnan(got), np.isnan(want)) and np.array_equal(got[np.isinf(want)], want[np.isinf(want)])
+    bits = 2.0 ** -8 if dtype == P.BF16_CODE else 2.0 ** -11
+    assert (np.abs(got[finite] - want[finite]) <= bits * np.abs(want[finite]) + 2e-5 * wide).all()
+
+
 @pytest.mark.parametrize("dtype,kv_heads,rep,seq,hd", [(P.BF16_CODE, 8, 4, 517, 128), (P.F16, 3, 1, 130, 64), (P.BF16_CODE, 37, 3, 300, 128)])
 def test_prefill_attention_stores_what_a_transpose_would(gpu_backend, dtype, kv_heads, rep, seq, hd):
     """A result that is only read as [batch, seq, kv_heads, rep, head_dim] is stored so, bit for bit what the transpose of the
