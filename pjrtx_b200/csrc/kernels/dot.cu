@@ -20,9 +20,10 @@
 //   0  generic   : one thread per output element, any strides, any m.
 // 16-bit floats without batch axes whose operands a TMA tensor map can describe run on the tensor cores instead
 // (umma_gemm.cuh, CTA pairs: umma_pair.cuh): rhs[K,N] as a variant of path 1 (so that q/k/v and gate/up still share one
-// launch), rhs[N,K] as path 4, rhs[K,N] rows that a tensor map cannot describe as path 5. PJRTX_B200_UMMA=0 turns that off; PJRTX_B200_UMMA_MIN_M (default 3: the CUDA-core
-// kernel was ahead for one and two rows on the 8B decode shapes, measured before the cluster-split stream and not again since)
-// keeps the CUDA-core streaming kernels below that m.
+// launch), rhs[N,K] as path 4, rhs[K,N] rows that a tensor map cannot describe as path 5. PJRTX_B200_UMMA=0 turns that off.
+// Paths 1 and 4 start at three rows (one row takes the same on either side; two are 7 % faster on the tensor cores over 8
+// layers of 8B widths, but f16 errors against 64 bits grow in the fourth digit there), large int8 weights at one;
+// PJRTX_B200_UMMA_MIN_M, where it is set, is the least m for both.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -1124,7 +1125,7 @@ int launch_chain(const DotChainSegment* segs, const DotChainArgs* args, int n, c
 
 // 0: not eligible, 1: rhs[K,N] with N contiguous, 2: rhs[N,K] with K contiguous, 3: rhs[K,N] with N contiguous whose rows
 // the tensor maps cannot describe. Tensor maps need 16-byte multiples for every row stride; lhs must be k-contiguous.
-// Int8 weights of a million and more have no lower bound on m: the alternative writes the dequantised weights out and reads
+// Int8 weights of a million and more have no lower bound on m unless the environment sets one: the alternative writes the dequantised weights out and reads
 // them again (one row, us, so and here: 1024 x 1024 17.3 / 12, 4096 x 1024 14.3 / 12.1, 4096 x 4096 22.6 / 16, 14336 x 4096 56 / 25,
 // 4096 x 32000 122 / 33).
 // Case 3 (odd vocabularies) has no lower bound on m: the alternative is one thread per output (path 0) or 64 x 64 tiles on
@@ -1132,14 +1133,16 @@ int launch_chain(const DotChainSegment* segs, const DotChainArgs* args, int n, c
 // mostly padding and the other paths stay.
 int umma_eligible(const DotShape& s) {
   static const int enabled = env_int("PJRTX_B200_UMMA", 1);
-  static const int min_m = env_int("PJRTX_B200_UMMA_MIN_M", 3);
+  static const int set_min_m = env_int("PJRTX_B200_UMMA_MIN_M", -1);
+  const int min_m = set_min_m < 0 ? 3 : set_min_m;
   if (!enabled || (s.dtype != kF16 && s.dtype != kBF16)) return 0;
   if (s.b0 * s.b1 != 1 || s.m < 1 || s.k < 1 || s.n < 1) return 0;
   if (s.lhs_k != 1 || (s.m > 1 && s.lhs_m % 8 != 0)) return 0;
   if (s.m > (1 << 20) || s.n > (1ll << 30) || s.k > (1ll << 30)) return 0;
   const bool pitch_ok = s.rhs_s8 ? s.rhs_k % 16 == 0 : s.rhs_k % 8 == 0;
   if (s.rhs_n == 1 && s.rhs_k >= s.n) {
-    if (pitch_ok) return s.m >= min_m || (s.rhs_s8 && s.k * s.n >= (1 << 20)) ? 1 : 0;
+    const bool few_rows = s.rhs_s8 && set_min_m < 0 && s.k * s.n >= (1 << 20);
+    if (pitch_ok) return s.m >= min_m || few_rows ? 1 : 0;
     return s.n >= 64 && s.k >= 64 && !s.rhs_s8 ? 3 : 0;
   }
   if (s.rhs_s8 || s.m < min_m) return 0;

@@ -1006,7 +1006,7 @@ def test_unaligned_weight_rows_by_residue_against_f64(gpu_backend, dtype, m, k, 
 
 
 @pytest.mark.parametrize("dtype", [P.BF16_CODE, P.F16])
-@pytest.mark.parametrize("m,k,n", [(1, 1024, 1024), (1, 4096, 1040), (2, 200, 5248), (2, 1024, 4112)])
+@pytest.mark.parametrize("m,k,n", [(1, 1024, 1024), (1, 4096, 1040), (2, 200, 5248), (2, 1024, 4112), (1, 1001, 1056)])
 def test_int8_contractions_of_one_and_two_rows(gpu_backend, m, k, n, dtype):
     """One and two rows of a million weights and more read the bytes themselves too: the bound of more rows."""
     test_int8_dequantising_contraction(gpu_backend, m, k, n, dtype)

@@ -3,6 +3,8 @@ import ctypes
 import os
 import random
 import re
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -470,6 +472,34 @@ def test_int8_converters_never_read_a_stage_before_its_unit_has_landed(stages):
                 ready[at[which] % slots] += 1
                 at[which] += 2
                 passed[which] = 0
+
+
+@pytest.mark.parametrize("setting,taken", [
+    ("", {(1, 1024, 1024), (2, 1024, 1024), (1, 1001, 1056), (3, 256, 256)}),
+    ("3", {(3, 256, 256)}),
+    ("2", {(2, 1024, 1024), (2, 1024, 1008), (3, 256, 256)}),
+    ("4", set()),
+])
+def test_least_rows_of_int8_contractions_on_the_tensor_cores(setting, taken):
+    """Int8 weights of 2^20 elements and more are read as bytes from one row up, smaller ones from three (below, the scaled weights
+    are written out and rounded); a minimum that the environment sets holds for both. Rows of a k that is no multiple of 8
+    have no pitch for the tensor map, but a single row needs none."""
+    sizes = [(1, 1024, 1024), (2, 1024, 1024), (2, 1024, 1008), (1, 1001, 1056), (2, 1001, 1056), (3, 256, 256)]
+    script = f"""
+import pjrtx_b200
+from pjrtx_b200 import plan as P
+from pjrtx_b200 import PlanBuilder
+for m, k, n in {sizes!r}:
+    b = PlanBuilder()
+    w = b.convert(b.parameter(P.S8, [k, n]), P.F16) * b.broadcast_in_dim(b.parameter(P.F16, [n]), [k, n], [1])
+    b.set_outputs([b.dot_general(b.parameter(P.F16, [m, k]), w, [1], [0])])
+    (dot,) = [s for s in pjrtx_b200.Backend().describe_kernels(b)["steps"] if s["type"] == "dot"]
+    print(m, k, n, dot["rhs_s8"])
+"""
+    env = {**os.environ, "PJRTX_B200_UMMA_MIN_M": setting}  # read once per process
+    out = subprocess.run([sys.executable, "-c", script], cwd=ROOT, env=env, capture_output=True, text=True, check=True).stdout
+    got = {tuple(map(int, line.split())) for line in out.splitlines()}
+    assert got == {(*size, int(size in taken)) for size in sizes}
 
 
 def test_error_word_codes_belong_to_one_kernel_each():
