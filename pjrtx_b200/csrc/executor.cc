@@ -669,8 +669,14 @@ void fuse_dequant_dots(Plan* plan) {
   auto made_by = [&](uint32_t v, Kind kind) -> const Instruction* {
     return producer[v] >= 0 && plan->instructions[producer[v]].kind == kind ? &plan->instructions[producer[v]] : nullptr;
   };
+  struct Candidate {
+    size_t dot;
+    uint32_t bytes, scale;
+    DotShape shape;
+  };
+  std::vector<Candidate> candidates;
   for (size_t i = 0; i < ni; i++) {
-    Instruction& dot = plan->instructions[i];
+    const Instruction& dot = plan->instructions[i];
     if (dot.kind != Kind::dot_general || dot.inputs.size() != 2) continue;
     const Value& x = plan->values[dot.inputs[0]];
     uint32_t w = dot.inputs[1];
@@ -717,8 +723,16 @@ void fuse_dequant_dots(Plan* plan) {
     shape.rhs_k = shape.n;
     shape.rhs_n = 1;
     shape.out_m = shape.n;
-    if (!dot_s8_supported(shape)) continue;
-    dot.inputs = {dot.inputs[0], bytes, scale};
+    if (dot_s8_supported(shape)) candidates.push_back({i, bytes, scale, shape});
+  }
+  // A narrow projection (k or v of few KV heads) rides along in the launch of a wider one that reads the same activations.
+  std::set<uint32_t> streamed;
+  for (const Candidate& c : candidates)
+    if (dot_s8_pays(c.shape, false)) streamed.insert(plan->instructions[c.dot].inputs[0]);
+  for (const Candidate& c : candidates) {
+    Instruction& dot = plan->instructions[c.dot];
+    if (!dot_s8_pays(c.shape, streamed.count(dot.inputs[0]) > 0)) continue;
+    dot.inputs = {dot.inputs[0], c.bytes, c.scale};
     dot.attrs["rhs_s8"] = {1};
   }
 }

@@ -22,7 +22,7 @@
 // (umma_gemm.cuh, CTA pairs: umma_pair.cuh): rhs[K,N] as a variant of path 1 (so that q/k/v and gate/up still share one
 // launch), rhs[N,K] as path 4, rhs[K,N] rows that a tensor map cannot describe as path 5. PJRTX_B200_UMMA=0 turns that off.
 // Paths 1 and 4 start at three rows (one row takes the same on either side; two are 7 % faster on the tensor cores over 8
-// layers of 8B widths, but f16 errors against 64 bits grow in the fourth digit there), large int8 weights at one;
+// layers of 8B widths, but f16 errors against 64 bits grow in the fourth digit there), large int8 weights, unless narrow or flat, at one;
 // PJRTX_B200_UMMA_MIN_M, where it is set, is the least m for both.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -1123,26 +1123,27 @@ int launch_chain(const DotChainSegment* segs, const DotChainArgs* args, int n, c
 
 // ---- tensor-core stream (umma_gemm.cuh) ---------------------------------------------------------------------------
 
+int least_rows_asked_for() {
+  static const int m = env_int("PJRTX_B200_UMMA_MIN_M", -1);
+  return m;
+}
+
 // 0: not eligible, 1: rhs[K,N] with N contiguous, 2: rhs[N,K] with K contiguous, 3: rhs[K,N] with N contiguous whose rows
 // the tensor maps cannot describe. Tensor maps need 16-byte multiples for every row stride; lhs must be k-contiguous.
-// Int8 weights of a million and more have no lower bound on m unless the environment sets one: the alternative writes the dequantised weights out and reads
-// them again (one row, us, so and here: 1024 x 1024 17.3 / 12, 4096 x 1024 14.3 / 12.1, 4096 x 4096 22.6 / 16, 14336 x 4096 56 / 25,
-// 4096 x 32000 122 / 33).
+// Int8 weights can start at one row (dot_s8_pays says where they do) unless the environment sets a least number.
 // Case 3 (odd vocabularies) has no lower bound on m: the alternative is one thread per output (path 0) or 64 x 64 tiles on
 // the CUDA cores (path 3). Measured, 5 x 2048 x 32001 f16: 739 us on path 0. Below 64 columns or a k of 64 a tile would be
 // mostly padding and the other paths stay.
 int umma_eligible(const DotShape& s) {
   static const int enabled = env_int("PJRTX_B200_UMMA", 1);
-  static const int set_min_m = env_int("PJRTX_B200_UMMA_MIN_M", -1);
-  const int min_m = set_min_m < 0 ? 3 : set_min_m;
+  const int set_min_m = least_rows_asked_for(), min_m = set_min_m < 0 ? 3 : set_min_m;
   if (!enabled || (s.dtype != kF16 && s.dtype != kBF16)) return 0;
   if (s.b0 * s.b1 != 1 || s.m < 1 || s.k < 1 || s.n < 1) return 0;
   if (s.lhs_k != 1 || (s.m > 1 && s.lhs_m % 8 != 0)) return 0;
   if (s.m > (1 << 20) || s.n > (1ll << 30) || s.k > (1ll << 30)) return 0;
   const bool pitch_ok = s.rhs_s8 ? s.rhs_k % 16 == 0 : s.rhs_k % 8 == 0;
   if (s.rhs_n == 1 && s.rhs_k >= s.n) {
-    const bool few_rows = s.rhs_s8 && set_min_m < 0 && s.k * s.n >= (1 << 20);
-    if (pitch_ok) return s.m >= min_m || few_rows ? 1 : 0;
+    if (pitch_ok) return s.m >= min_m || (s.rhs_s8 && set_min_m < 0) ? 1 : 0;
     return s.n >= 64 && s.k >= 64 && !s.rhs_s8 ? 3 : 0;
   }
   if (s.rhs_s8 || s.m < min_m) return 0;
@@ -1626,6 +1627,20 @@ bool dot_s8_supported(const DotShape& s) {
   DotShape probe = s;
   probe.rhs_s8 = 1;
   return umma_eligible(probe) == 1;
+}
+
+// Under one or two rows the alternative writes the scaled weights out and reads them again, five bytes per weight, while the
+// bytes' own way is a chain per 128 rows of k that at most eight CTAs share. Measured, us, written form and bytes, one row / two
+// rows: 1024 x 1024 10.9 10.2 / 11.1 10.3, 4096 x 4096 22.6 16.1 / 24.7 16.2, 14336 x 4096 56 25 and 4096 x 32000 122 33 at one; k
+// long against n: 4096 x 256 10.8 10.3 / 12.4 10.3, 16384 x 256 18.5 16.4 / 26.7 16.5, 32768 x 512 25.2 22.6 / 32.5 22.6, 24576 x 384
+// 18.5 18.8 / 25.1 18.9, 65536 x 256 28.8 34.9 / 39.2 34.9, 8192 x 192 12.0 12.5 / 16.3 12.4, 8192 x 128 11.7 12.4 / 16.3 12.4, 32768 x
+// 32 16.5 22.5 / 25.9 22.6, 65536 x 16 18.4 34.2 / 28.6 34.2; k short: 128 x 8192 9.4 8.7 / 9.6 8.6, 96 x 65536 16.5 12.4 / 18.5 12.4,
+// 64 x 65536 11.1 12.4 / 12.1 12.4, 16 x 65536 11.0 12.4 / 10.8 12.4. Below a million weights neither side was measured against
+// the other and the written rounding stays.
+bool dot_s8_pays(const DotShape& s, bool shared) {
+  if (s.m > 2 || least_rows_asked_for() >= 0) return true;  // (dot_s8_supported has looked at what was asked for)
+  if (s.k * s.n < (1 << 20)) return false;
+  return shared || (s.k >= 96 && (s.m == 1 ? s.n >= 256 && s.k <= 64 * s.n : s.k <= 1024 * s.n));
 }
 
 int dot_group_launch(const DotShape* shapes, int count, const DotScratch& plan, const void* lhs, const void* const* rhs,

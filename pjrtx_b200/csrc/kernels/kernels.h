@@ -178,6 +178,8 @@ int dot_launch(const DotShape& s, const DotScratch& plan, const void* lhs, const
                const void* scale = nullptr);
 // True when an int8-weight contraction of this shape has a kernel (the tensor-core stream with in-kernel dequantisation).
 bool dot_s8_supported(const DotShape& s);
+// Whether it is shorter than the written form; `shared`: another one that pays reads the same lhs.
+bool dot_s8_pays(const DotShape& s, bool shared);
 
 // out[m, n] = lhs[m, k] . rhs[k, n] (dense row-major device pointers) with split-K scratch taken from a fixed
 // array in the library image instead of an allocation. 1 on success, 0 with last_error set.

@@ -502,6 +502,31 @@ for m, k, n in {sizes!r}:
     assert got == {(*size, int(size in taken)) for size in sizes}
 
 
+@pytest.mark.parametrize("m,k,n,taken", [
+    (1, 4096, 256, 1), (1, 16384, 256, 1), (1, 16400, 256, 0), (1, 8192, 240, 0), (1, 8192, 128, 0), (1, 131072, 16, 0), (1, 65536, 1024, 1),
+    (2, 8192, 128, 1), (2, 32768, 32, 1), (2, 32800, 32, 0), (2, 65536, 16, 0), (2, 131072, 16, 0),
+    (1, 96, 65536, 1), (1, 64, 65536, 0), (2, 64, 65536, 0), (2, 16, 65536, 0), (3, 65536, 16, 1),
+])
+def test_int8_contractions_of_few_rows_keep_to_where_they_are_shorter(backend, m, k, n, taken):
+    """Narrow weights of a long k and flat ones keep the written form at one and two rows."""
+    b = PlanBuilder()
+    w = b.convert(b.parameter(P.S8, [k, n]), P.F16) * b.broadcast_in_dim(b.parameter(P.F16, [n]), [k, n], [1])
+    b.set_outputs([b.dot_general(b.parameter(P.F16, [m, k]), w, [1], [0])])
+    (st,) = [s for s in backend.describe_kernels(b)["steps"] if s["type"] == "dot"]
+    assert st["rhs_s8"] == taken, st
+
+
+def test_a_narrow_int8_projection_rides_along_with_a_wide_one(backend):
+    b = PlanBuilder()
+    x, outs = b.parameter(P.F16, [1, 8192]), []
+    for n in (8192, 128, 128):  # one KV head
+        w = b.convert(b.parameter(P.S8, [8192, n]), P.F16) * b.broadcast_in_dim(b.parameter(P.F16, [n]), [8192, n], [1])
+        outs.append(b.dot_general(x, w, [1], [0]))
+    b.set_outputs(outs)
+    (st,) = [s for s in backend.describe_kernels(b)["steps"] if s["type"] == "dot"]
+    assert st["rhs_s8"] == 1 and st["group"] == 3, st
+
+
 def test_error_word_codes_belong_to_one_kernel_each():
     """A caller drops its peers on code 21, so no local wait may raise it; the same for every other code."""
     kernels = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "pjrtx_b200", "csrc", "kernels")
