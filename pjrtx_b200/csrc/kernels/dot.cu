@@ -884,7 +884,7 @@ int launch_typed(const DotShape& s, const DotScratch& plan, const void* lhs, con
 
 namespace {
 int umma_eligible(const DotShape& s);
-DotScratch umma_plan(const DotShape* shapes, int count, int sm_count, int kind, bool by_residue = true);
+DotScratch umma_plan(const DotShape* shapes, int count, int sm_count, int kind);
 }  // namespace
 
 namespace {
@@ -1272,10 +1272,10 @@ DotScratch shift_plan(const DotShape& s, int sm_count) {
   return p;
 }
 
-DotScratch umma_plan(const DotShape* shapes, int count, int sm_count, int kind, bool by_residue) {
+DotScratch umma_plan(const DotShape* shapes, int count, int sm_count, int kind) {
   DotScratch p;
   const DotShape& s = shapes[0];
-  if (kind == 3 && by_residue && count == 1 && shift_pays(s)) return shift_plan(s, sm_count);
+  if (kind == 3 && count == 1 && shift_pays(s)) return shift_plan(s, sm_count);
   const int src = umma_source(s, kind == 3);
   p.path = kind == 1 ? 1 : kind == 2 ? 4 : 5;
   p.umma = 1;
@@ -1361,7 +1361,8 @@ int launch_umma_pair(const umma::PairParams& prm, const umma::Maps& maps, const 
 int launch_umma_shift(const DotShape& s, const DotScratch& plan, const void* lhs, const void* rhs, void* out, void* rearranged,
                       int* error_flag, bool early_rhs, bool pdl, cudaStream_t stream) {
   EncodeTiledFn enc = encode_tiled();
-  if (!enc || !rearranged) return 0;
+  // The residues' maps start at most 14 bytes before their first row: on a 16-byte boundary if the weights do.
+  if (!enc || !rearranged || (reinterpret_cast<uintptr_t>(rhs) & 15) != 0) return 0;
   const int residues = plan.shift;
   const int64_t depth = ((s.k + residues - 1) / residues + 63) / 64 * 64;
   umma::ShiftParams p{};
@@ -1647,14 +1648,7 @@ int dot_group_launch(const DotShape* shapes, int count, const DotScratch& plan, 
                      void* const* out, void* partials, void* counters, int* error_flag, bool early_rhs, bool pdl,
                      cudaStream_t stream, const void* const* scales) {
   if (count < 1 || count > kDotGroupMax) return 0;
-  if (plan.shift) {
-    if ((reinterpret_cast<uintptr_t>(rhs[0]) & 15) == 0)
-      return launch_umma_shift(shapes[0], plan, lhs, rhs[0], out[0], partials, error_flag, early_rhs, pdl, stream);
-    // Weights that do not start on a 16-byte boundary go through the converters.
-    int device = 0, sms = 0;
-    if (cudaGetDevice(&device) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return 0;
-    return launch_umma(shapes, count, umma_plan(shapes, count, sms, 3, false), lhs, rhs, out, error_flag, early_rhs, pdl, stream, scales);
-  }
+  if (plan.shift) return launch_umma_shift(shapes[0], plan, lhs, rhs[0], out[0], partials, error_flag, early_rhs, pdl, stream);
   if (plan.umma) return launch_umma(shapes, count, plan, lhs, rhs, out, error_flag, early_rhs, pdl, stream, scales);
   if (shapes[0].rhs_s8) return 0;  // int8 weights run on the tensor-core stream only
   if (plan.small) {

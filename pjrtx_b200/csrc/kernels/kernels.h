@@ -211,8 +211,8 @@ int dus_launch(const SliceUpdateShape& s, void* dst, const void* update, const v
                cudaStream_t stream);
 
 // Several device-to-device copies as one launch for every kCopyBatchMax of them. A source is not written by another
-// entry of the same call; any addresses and sizes are taken (16 bytes at a time where both ends are aligned). The launch
-// is ordered after its predecessor and before its successor. False: a launch failed.
+// entry of the same call; both ends start on 16-byte boundaries (buffers, slots and arena values start on 256-byte ones), any
+// size is taken. The launch is ordered after its predecessor and before its successor. False: a launch failed.
 struct CopyEntry {
   const void* src;
   void* dst;

@@ -93,25 +93,23 @@ __global__ void __launch_bounds__(kCopyThreads) copy_batch_kernel(const __grid_c
   const uint64_t begin = piece * kCopyPiece, end = min(e.bytes, begin + kCopyPiece);
   const unsigned char* src = static_cast<const unsigned char*>(e.src);
   unsigned char* dst = static_cast<unsigned char*>(e.dst);
-  uint64_t tail = begin;
-  if (((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15) == 0) {
-    const uint4* s = reinterpret_cast<const uint4*>(src + begin);
-    uint4* d = reinterpret_cast<uint4*>(dst + begin);
-    const int vectors = (int)((end - begin) / 16);
-    uint4 v[kCopyUnroll];
+  const uint4* s = reinterpret_cast<const uint4*>(src + begin);
+  uint4* d = reinterpret_cast<uint4*>(dst + begin);
+  const int vectors = (int)((end - begin) / 16);
+  uint4 v[kCopyUnroll];
 #pragma unroll
-    for (int i = 0; i < kCopyUnroll; i++) {
-      const int at = i * kCopyThreads + (int)threadIdx.x;
-      if (at < vectors) v[i] = s[at];
-    }
-#pragma unroll
-    for (int i = 0; i < kCopyUnroll; i++) {
-      const int at = i * kCopyThreads + (int)threadIdx.x;
-      if (at < vectors) d[at] = v[i];
-    }
-    tail = begin + (uint64_t)vectors * 16;
+  for (int i = 0; i < kCopyUnroll; i++) {
+    const int at = i * kCopyThreads + (int)threadIdx.x;
+    if (at < vectors) v[i] = s[at];
   }
-  for (uint64_t at = tail + threadIdx.x; at < end; at += kCopyThreads) dst[at] = src[at];
+#pragma unroll
+  for (int i = 0; i < kCopyUnroll; i++) {
+    const int at = i * kCopyThreads + (int)threadIdx.x;
+    if (at < vectors) d[at] = v[i];
+  }
+  // The last piece of an entry may end between two boundaries.
+  const uint64_t at = begin + (uint64_t)vectors * 16 + threadIdx.x;
+  if (at < end) dst[at] = src[at];
 }
 
 // ------------------------------------------------------------------ attention
@@ -185,6 +183,7 @@ static bool copy_batches(const CopyEntry* entries, size_t count, cudaStream_t st
       const uint64_t pieces = (entries[at].bytes + kCopyPiece - 1) / kCopyPiece;
       if (blocks && blocks + pieces > 0x7fffffffull) break;  // a grid's limit
       if (pieces == 0) continue;
+      if (((reinterpret_cast<uintptr_t>(entries[at].src) | reinterpret_cast<uintptr_t>(entries[at].dst)) & 15) != 0) return false;
       blocks += pieces;
       b.entry[b.count] = entries[at];
       b.end[b.count++] = (unsigned)blocks;

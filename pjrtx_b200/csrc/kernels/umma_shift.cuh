@@ -13,8 +13,8 @@
 // hundred KB), zeros where a residue has fewer rows.
 //
 // What bounds it: HBM, and above it 12 us for two launches, the first copies and the residues' sum. Before it, one 2-byte load
-// per weight through the converter warps of umma_stream_kernel<2, kLoose>, 1.6 TB/s, which remains for more rows, for small
-// weights (shift_pays in dot.cu) and for weights that do not start on a 16-byte boundary. 5 rows of f16, launches one after the
+// per weight through the converter warps of umma_stream_kernel<2, kLoose>, 1.6 TB/s, which remains for more rows and for small
+// weights (shift_pays in dot.cu). 5 rows of f16, launches one after the
 // other, us, before and now: 2048 x 32001 83 / 31.6, 4096 x 32001 156 / 54, 8192 x 32001 300 / 101 (5.2 TB/s); 32 rows 85 / 36,
 // 158 / 62.5, 302 / 106. Errors against 64 bits are equal to three digits (the rounding of the output), the fourth is smaller.
 //
