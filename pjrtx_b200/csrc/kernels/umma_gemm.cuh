@@ -159,9 +159,6 @@ struct WaitBudget {
   unsigned long long deadline;
   volatile int* abort;
 };
-__device__ __forceinline__ WaitBudget launch_budget(unsigned long long timeout_ns, int* abort) {
-  return WaitBudget{global_timer_ns() + timeout_ns, abort};
-}
 // Bounded by time: gives up when the launch's deadline has passed or another thread of the CTA already gave up.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity, const WaitBudget& w) {
   for (unsigned spin = 0;; spin++) {

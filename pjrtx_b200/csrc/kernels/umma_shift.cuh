@@ -88,7 +88,7 @@ __global__ void __launch_bounds__(kBaseThreads, MT == 16 ? 2 : 1) umma_shift_ker
   uint64_t* acc_empty = acc_full + 2;     // [2]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
   int* flags = reinterpret_cast<int*>(tmem_slot + 1);  // [0] abort
-  const WaitBudget budget = launch_budget(p.timeout_ns, flags);
+  const WaitBudget budget{global_timer_ns() + p.timeout_ns, flags};
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const bool leader = elect_one();

@@ -546,9 +546,11 @@ def test_every_device_side_wait_takes_its_budget_from_the_launch():
     for name in sorted(os.listdir(kernels)):
         with open(os.path.join(kernels, name)) as f:
             text = f.read()
-        budgets += [(name, b) for b in re.findall(r"WaitBudget budget\{[\w:]*global_timer_ns\(\) \+ ([\w.]+),", text)]
+        budgets += [(name, b) for b in re.findall(
+            r"(?:WaitBudget budget\{[\w:]*global_timer_ns\(\) \+|deadline = global_timer_ns\(\) \+|deadline \+=|t1 - t0 >) ([\w.]+)", text)]
+        assert len(re.findall(r"WaitBudget budget\b", text)) == len(re.findall(r"WaitBudget budget\{", text)), name
         assert not re.search(r"imeout_?ns\w* = \d", text, re.I), name
-    assert len(budgets) == 5 and all(b.endswith("timeout_ns") for _, b in budgets), budgets
+    assert len(budgets) == 9 and all(b.endswith("timeout_ns") for _, b in budgets), budgets
 
 
 @pytest.mark.parametrize("dtype,m,k,n,path,split", [
