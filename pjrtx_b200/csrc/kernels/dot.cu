@@ -1250,8 +1250,13 @@ double umma_pair_choose(const DotShape* shapes, int count, int sm_count, int* m_
 // Rows without a 16-byte pitch by residue (umma_shift.cuh) or through converters (kLoose). By residue costs a launch and a
 // longer epilogue, 4 us, and does not split k, but streams three times as fast. Measured at 16 rows, us, residues and
 // converters: 2048 x 1001 18.7 / 14.3, x 2001 18.7 / 17.6, x 3001 18.7 / 20.1, x 4001 18.8 / 20.4, x 8001 19 / 29; 8192 x 2001
-// 43 / 35, x 4001 43 / 48, x 8001 45 / 87; 256 x 16001 16.3 / 14.3.
-bool shift_pays(const DotShape& s) { return s.m <= 32 && s.n > 3000 && s.n * s.k >= 6000000; }
+// 43 / 35, x 4001 43 / 48, x 8001 45 / 87; 256 x 16001 16.3 / 14.3. Up to 26 tiles of 128 columns the converters' clusters of five
+// are one wave: 16384 x 3201 74.0 / 71.8, x 3401 73.8 / 85.2, 65536 x 3001 262 / 242, x 3401 263 / 298. Beyond 16 rows the 64 rows
+// that a short k's residues are padded to weigh more: 17 rows 64 x 93801 28.8 / 24.8, 96 x 200001 47.2 / 45.1, 128 x 46901 20.6 / 20.3,
+// 32 rows 64 x 93801 30.8 / 28.5, 128 x 46901 20.6 / 22.3 (16 rows 64 x 93801 18.6 / 22.4).
+bool shift_pays(const DotShape& s) {
+  return s.m <= 32 && s.n > (s.k <= 2048 ? 3000 : 26 * umma::kTileN) && s.n * s.k >= 6000000 && (s.m <= 16 || s.k >= 128);
+}
 
 DotScratch shift_plan(const DotShape& s, int sm_count) {
   DotScratch p;

@@ -527,6 +527,17 @@ def test_a_narrow_int8_projection_rides_along_with_a_wide_one(backend):
     assert st["rhs_s8"] == 1 and st["group"] == 3, st
 
 
+@pytest.mark.parametrize("m,k,n,residues", [
+    (16, 2048, 3001, 8), (32, 2048, 3001, 8), (16, 2056, 3001, 0), (16, 65536, 3327, 0), (16, 65536, 3329, 8), (32, 4096, 3329, 8),
+    (16, 64, 93801, 8), (17, 64, 93801, 0), (17, 120, 93801, 0), (17, 128, 93801, 8), (33, 2048, 32001, 0), (5, 256, 16001, 0),
+])
+def test_weight_rows_go_by_residue_where_it_is_shorter(backend, m, k, n, residues):
+    b = PlanBuilder()
+    b.set_outputs([b.dot_general(b.parameter(P.F16, [m, k]), b.parameter(P.F16, [k, n]), [1], [0])])
+    (st,) = backend.describe_kernels(b)["steps"]
+    assert st["path"] == 5 and st["shift"] == residues, st
+
+
 def test_error_word_codes_belong_to_one_kernel_each():
     """A caller drops its peers on code 21, so no local wait may raise it; the same for every other code."""
     kernels = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "pjrtx_b200", "csrc", "kernels")
