@@ -1295,10 +1295,14 @@ AttnDecodePlan attn_decode_plan(const AttnDecodeShape& s, int sm_count) {
       return p;
     }
   }
-  // The tensor-core kernel wherever it applies: since its rows come by tiled copies and its splits merge cooperatively it
+  // The tensor-core kernel wherever it applies but for one case below: since its rows come by tiled copies and its splits merge cooperatively it
   // is ahead at every size measured (8B shape, batch 1: 3.28 against 3.35 ms per step with 2.1 K keys, 3.36 against
   // 3.48 ms with 2.7 K; batch 2: 3.75 against 3.93 ms).
-  p.mma = mma_ok && (force && *force ? atoi(force) != 0 : true) ? 1 : 0;
+  // One query head per KV head over a second stage of keys that is not full (65 to 128) is as long on the CUDA cores, and with
+  // more pairs than fit once shorter there, us: 24 sequences of 8 KV heads, 128 keys 8.28 / 9.15, 32 of 80 keys 8.2 / 9.5, of 96
+  // 8.3 / 10.0, of 128 9.6 / 10.1, 64 of 96 12.3 / 14.3; 32 of 64 keys 8.2 / 7.9, of 144 11.5 / 10.2; 12 of 80 7.6 / 7.8.
+  const bool one_head_two_stages = rep == 1 && s.kv_len > kMmaStageKeys && s.kv_len <= 2 * kMmaStageKeys && 2 * tiles > sm_count;
+  p.mma = mma_ok && (force && *force ? atoi(force) != 0 : !one_head_two_stages) ? 1 : 0;
   if (p.mma) {
     // Two CTAs per SM are resident: one wave of them, no more (measured at 4K keys, batch 32: 32 / 64 / 128 / 256
     // (sequence, KV head) pairs run fastest with 9 / 4 / 2 / 1 splits — 25.5 / 36 / 57 / 84 us against 44 / 50 / 68 /

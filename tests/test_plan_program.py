@@ -335,8 +335,8 @@ def test_plan_fingerprint_is_stable_and_sensitive(backend):
 
 def test_decode_attention_kernel_choice_and_grid(backend, monkeypatch):
     """Planner rules of the decode attention step (device independent, 148 SMs assumed): 16-bit caches with 4 or 8
-    query heads per KV head, head size 64 / 128 and at least one 64-key stage go to the tensor-core kernel with one
-    wave of two CTAs per SM and no split shorter than 128 keys; a shorter buffer, f32 caches or another head ratio go to
+    query heads per KV head, or 1 or 2 of 128 elements, and at least one 64-key stage go to the tensor-core kernel with
+    one wave of two CTAs per SM and no split shorter than 128 keys; a shorter buffer, f32 caches or 1 or 2 heads of 64 go to
     the CUDA-core kernel, which keeps to one wave of one CTA per SM when there are fewer (sequence, KV head) pairs
     than SMs."""
     from pjrtx_b200 import PlanBuilder
@@ -368,7 +368,7 @@ def test_decode_attention_kernel_choice_and_grid(backend, monkeypatch):
     # one eighth of the 70B shape: 32 pairs -> 9 splits
     st = plan_of(P.BF16_CODE, 32, 8, 1, 128, 4352)
     assert st["mma"] == 1 and st["splits"] == 9
-    # a buffer shorter than a stage, f32 caches, two heads per KV head: CUDA-core kernel
+    # a buffer shorter than a stage, f32 caches, two heads of 64 per KV head: CUDA-core kernel
     assert plan_of(P.BF16_CODE, 2, 16, 4, 128, 40)["mma"] == 0
     assert plan_of(P.F32, 2, 8, 2, 64, 512)["mma"] == 0
     assert plan_of(P.F16, 2, 8, 4, 64, 512)["mma"] == 0
@@ -536,6 +536,20 @@ def test_weight_rows_go_by_residue_where_it_is_shorter(backend, m, k, n, residue
     b.set_outputs([b.dot_general(b.parameter(P.F16, [m, k]), b.parameter(P.F16, [k, n]), [1], [0])])
     (st,) = backend.describe_kernels(b)["steps"]
     assert st["path"] == 5 and st["shift"] == residues, st
+
+
+@pytest.mark.parametrize("batch,heads,kv_len,mma", [
+    (32, 8, 64, 1), (32, 8, 65, 0), (32, 8, 128, 0), (32, 8, 129, 1), (32, 16, 96, 1), (9, 8, 96, 1), (10, 8, 96, 0),
+])
+def test_one_query_head_over_two_short_stages_keeps_to_the_cuda_cores(backend, monkeypatch, batch, heads, kv_len, mma):
+    """Eight KV heads of 128: one query head each, 65 to 128 keys, more than 74 pairs of sequence and head."""
+    for name in ("MMA", "STAGED", "SPLITS"):
+        monkeypatch.delenv("PJRTX_B200_ATTENTION_" + name, raising=False)
+    b = PlanBuilder()
+    q, k, v = (b.parameter(P.F16, dims) for dims in ([batch, 1, heads, 128], [batch, kv_len, 8, 128], [batch, kv_len, 8, 128]))
+    b.set_outputs([b.custom_call("pjrtx.b200.scaled_dot_product_attention", [q, k, v, b.parameter(P.S32, [])], P.F16, [batch, 1, heads, 128])])
+    (st,) = backend.describe_kernels(b)["steps"]
+    assert st["mma"] == mma, st
 
 
 def test_error_word_codes_belong_to_one_kernel_each():
