@@ -535,42 +535,75 @@ __global__ void __launch_bounds__(threads_of(SRC), SRC == kLoose ? 1 : 2) umma_s
 
   if (warp == 4) {
     // ---- TMA producer ------------------------------------------------------------------------------------------
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    auto load_lhs = [&](const Tile& t, int kb, int stage) {
+      const uint32_t st = base + (uint32_t)stage * per_stage + w_bytes;
+#pragma unroll
+      for (int s = 0; s < SUB; s++)
+        tma_load_2d(st + (uint32_t)s * p.m_tile * 128u, &maps.lhs, kb * kDepth + s * kSubK, t.m_idx * p.m_tile, &full[stage]);
+    };
+    auto gave_up = [&](int i) {
+      atomicExch(p.error_flag, 11);
+      // Nothing more is requested; the copies in flight get a bounded time to land before the CTA leaves.
+      for (int b = 1; b <= p.stages; b++) {
+        const int j = i - b;  // the last unit requested into each stage
+        for (unsigned spin = 0; spin < (1u << 16) && !mbar_try_wait(&full[j % p.stages], (unsigned)(j / p.stages) & 1u); spin++) {
+        }
+      }
+    };
     int tile = cluster, kb = kb_begin, stage = 0;
     unsigned phase = 0;
-    Tile t = locate_tile(p, min(tile, p.tiles - 1));
-    for (int i = 0; i < count; i++) {
-      if (i >= p.stages && !__all_sync(0xffffffffu, mbar_wait(&empty[stage], phase ^ 1, budget))) {
-        if (leader) {
-          atomicExch(p.error_flag, 11);
-          // Nothing more is requested; the copies in flight get a bounded time to land before the CTA leaves.
-          for (int b = 1; b <= p.stages; b++) {
-            const int j = i - b;  // the last unit requested into each stage
-            for (unsigned spin = 0; spin < (1u << 16) && !mbar_try_wait(&full[j % p.stages], (unsigned)(j / p.stages) & 1u); spin++) {
+    if constexpr (SRC == kLoose) {
+      // Activations only, by one lane: beside sixteen converter warps the converged form of this loop costs the launch 4 to 8 %
+      // (us, converged and so: 5 x 65536 x 3001 260 / 237, 33 x 8192 x 32001 330 / 305, 64 x 2048 x 32001 95 / 88; 64 x 2048 x 1001
+      // 14.5 either way). Which part of it does was not found: waiting by one lane alone did not help.
+      if (lane == 0 && count > 0) {
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        Tile t = locate_tile(p, tile);
+        for (int i = 0; i < count; i++) {
+          if (i >= first) {
+            if (i >= p.stages && !mbar_wait(&empty[stage], phase ^ 1, budget)) {
+              gave_up(i);
+              break;
             }
+            mbar_expect_tx(&full[stage], per_stage);
+          }
+          load_lhs(t, kb, stage);
+          if (++kb == kb_end) {
+            kb = kb_begin;
+            tile += clusters;
+            if (tile < p.tiles) t = locate_tile(p, tile);
+          }
+          if (++stage == p.stages) {
+            stage = 0;
+            phase ^= 1;
           }
         }
-        break;
       }
-      if (leader) {
-        if (i >= first) {
-          mbar_expect_tx(&full[stage], per_stage);
-          load_rhs(t, kb, stage);
+    } else {
+      asm volatile("griddepcontrol.wait;" ::: "memory");
+      Tile t = locate_tile(p, min(tile, p.tiles - 1));
+      for (int i = 0; i < count; i++) {
+        if (i >= p.stages && !__all_sync(0xffffffffu, mbar_wait(&empty[stage], phase ^ 1, budget))) {
+          if (leader) gave_up(i);
+          break;
         }
-        const uint32_t st = base + (uint32_t)stage * per_stage + w_bytes;
-#pragma unroll
-        for (int s = 0; s < SUB; s++)
-          tma_load_2d(st + (uint32_t)s * p.m_tile * 128u, &maps.lhs, kb * kDepth + s * kSubK, t.m_idx * p.m_tile, &full[stage]);
-      }
-      __syncwarp();
-      if (++kb == kb_end) {
-        kb = kb_begin;
-        tile += clusters;
-        t = locate_tile(p, min(tile, p.tiles - 1));
-      }
-      if (++stage == p.stages) {
-        stage = 0;
-        phase ^= 1;
+        if (leader) {
+          if (i >= first) {
+            mbar_expect_tx(&full[stage], per_stage);
+            load_rhs(t, kb, stage);
+          }
+          load_lhs(t, kb, stage);
+        }
+        __syncwarp();
+        if (++kb == kb_end) {
+          kb = kb_begin;
+          tile += clusters;
+          t = locate_tile(p, min(tile, p.tiles - 1));
+        }
+        if (++stage == p.stages) {
+          stage = 0;
+          phase ^= 1;
+        }
       }
     }
     __syncwarp();
