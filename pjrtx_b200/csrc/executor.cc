@@ -654,9 +654,9 @@ void fuse_decode_attention(Plan* plan) {
 // over a [k, n] weight (the only quantised form the reference accepts: its mixed-type dot is rejected,
 // src/backend/mlx_metal/lowering_linalg.zig:14-53, and convert is api.cc:907-935). When the dequantised weight has no
 // other reader and the tensor-core stream can take the shape, the dot_general reads the bytes itself: its rhs becomes
-// w, the scale its third operand, and the dequantising instructions die. The kernel rebuilds, per element, exactly the
-// value the written program would have stored (f16 product rounded to nearest, then the conversion), so results are
-// those of the op-by-op program while the weights stay one byte wide in HBM.
+// w, the scale its third operand, and the dequantising instructions die. The kernel contracts the integers and scales the f32
+// sums: the rounding of every w * s that the written program performs is left out, and the weights stay one byte wide in
+// HBM.
 void fuse_dequant_dots(Plan* plan) {
   const size_t ni = plan->instructions.size(), nv = plan->values.size();
   std::vector<long> producer(nv, -1);

@@ -677,8 +677,8 @@ attn_decode_staged_kernel(DecodeArgs a, const T* __restrict__ q, const T* __rest
 // the same work is 32 warp-level MMAs per 16 keys.
 //
 // One CTA (4 warps) = one (sequence, KV head, key split). K and V rows stream through a ring of shared-memory stages
-// of 64 keys (cp.async, 16 bytes per request, rows XOR-swizzled in 16-byte units so that ldmatrix reads are
-// conflict-free); rows past the end of the split are zero-filled. Each warp owns 16 keys of a stage:
+// of 64 keys (tiled tensor-map copies issued by one thread, 128-byte swizzle so that ldmatrix reads are conflict-free); V rows
+// past the end of the split are cleared. Each warp owns 16 keys of a stage:
 //   S[16 x 16 keys] = Q[16 x HD] . K^T      mma.m16n8k16, Q fragments held in registers (rows >= REP are zero),
 //                                           K fragments by ldmatrix
 //   online softmax on the accumulator fragments (row statistics are shared by the four lanes of a quad)
@@ -1271,8 +1271,8 @@ AttnDecodePlan attn_decode_plan(const AttnDecodeShape& s, int sm_count) {
   const long long tiles = s.batch * s.kv_heads;
   const long long rep = s.heads / s.kv_heads;
   // Tensor-core kernel: 16-bit caches with four or eight query heads per KV head, one or two where heads are 128 wide, and
-  // 16-byte aligned rows; everything else (f32, one or two heads of 64) runs on the CUDA-core kernel. PJRTX_B200_ATTENTION_MMA=0 / 1 forces the choice wherever
-  // the tensor-core kernel applies.
+  // 16-byte aligned rows; everything else (f32, one or two heads of 64) runs on the CUDA-core kernel.
+  // PJRTX_B200_ATTENTION_MMA=0 / 1 forces the choice wherever the tensor-core kernel applies.
   const bool mma_ok = (s.dtype == kF16 || s.dtype == kBF16) && (((rep == 4 || rep == 8) && s.head_dim == 64) || s.head_dim == 128) &&
                       s.kv_len >= kMmaStageKeys &&  // the copies' box is a whole stage of keys
                       s.kv_row_stride % 8 == 0 && s.kv_head_stride % 8 == 0 && s.kv_batch_stride % 8 == 0;  // 16-byte pitches

@@ -1172,7 +1172,12 @@ bool umma_fits(int m_tile, int ksplit, bool several_tiles, int src, bool half) {
          (half ? umma::kSharedSmem : 227 * 1024);
 }
 
-// Tile height, split of k, CTAs per SM and ring size with the least modelled time, in nanoseconds. The weights arrive at the
+// Tile height, split of k, CTAs per SM and ring size with the least modelled time, in nanoseconds. The constants and the
+// points below were taken while a single thread issued copies and products; converged issue took 1.5 to 3 us off a decode launch and
+// more off int8 (umma_gemm.cuh), and they were kept for the choices they make: refitted to single launches of int8 they put one CTA
+// on an SM at small widths (14336 x 4096 alone 26.6 -> 22.6 us), and a whole step of 32 layers went from 4522 to 5530 us; refitted
+// above 64 rows (regret 2.6 -> 1.2 % over 1600 launches) they left pairs out at 708 x 512..1792, which that sweep did not cover.
+// The weights arrive at the
 // HBM rate or at the rate of the CTAs, 16 KiB per 250 ns with the whole ring, per 305 ns with half of it and per 400 ns where
 // two CTAs of the launch share an SM (32 x 14336 x 4096 by 32 CTAs: 64 us with the whole ring, 79 with half, the same for 16
 // to 128 rows); near the crossing the two add up softly. Tall tiles are bound by shared memory, the copies in and the tensor
@@ -1223,9 +1228,9 @@ UmmaChoice umma_choose(const DotShape* shapes, int count, int sm_count, int src)
   return best;
 }
 
-// The same model for CTA pairs (umma_pair.cuh), whose units take 300 ns and half a nanosecond per row. Measured, us, one SM
-// per tile and pairs: 128 x 4096 x 4096 20 / 31, 128 x 4096 x 28672 87 / 59, 256 x 14336 x 4096 52 / 81, 256 x 4096 x 28672
-// 84 / 68, 517 x 4096 x 4096 40 / 34.
+// The same model for CTA pairs (umma_pair.cuh), whose units took 300 ns and half a nanosecond per row by a single thread (now
+// 195 and 0.57, see above). Measured then, us, one SM per tile and pairs: 128 x 4096 x 4096 20 / 31, 128 x 4096 x 28672 87 / 59,
+// 256 x 14336 x 4096 52 / 81, 256 x 4096 x 28672 84 / 68, 517 x 4096 x 4096 40 / 34 (now 31).
 double umma_pair_choose(const DotShape* shapes, int count, int sm_count, int* m_tile) {
   const DotShape& s = shapes[0];
   const int64_t kblocks = (s.k + 63) / 64;
@@ -1311,7 +1316,7 @@ DotScratch umma_plan(const DotShape* shapes, int count, int sm_count, int kind) 
   const size_t ring_budget = (choice.half ? umma::kSharedSmem : 227 * 1024) - 1024 - umma::kBarrierBytes - sum;
   // 128-deep stages once every CTA gets a long run of them (fewer hand-overs); 64-deep otherwise, and whenever the ring
   // would hold fewer than four of the deep ones. Converted weights always come 128 deep: 64-deep stages double the
-  // hand-overs between copies, converters and the MMA lane (int8, 8B-width layers at 32 rows: 1.54 against 1.25 ms).
+  // hand-overs between copies, converters and the MMA warp (int8, 8B-width layers at 32 rows: 1.54 against 1.25 ms).
   const int64_t deep_units = (tiles + clusters - 1) / clusters * ((s.k + 127) / 128) / p.ksplit;
   p.sub = src != umma::kTile || (deep_units >= 16 && ring_budget / umma::stage_bytes(p.m_tile, 2, src) >= 4) ? 2 : 1;
   p.stages = (int)std::min<size_t>(12, ring_budget / umma::stage_bytes(p.m_tile, p.sub, src));  // two or more (umma_fits)

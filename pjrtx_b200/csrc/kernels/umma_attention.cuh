@@ -5,7 +5,8 @@
 // q is [batch, kv_heads, seq, rep, head_dim] (the operand layout of the recognised dot_general -> masked softmax ->
 // dot_general form), so the `seq * rep` query rows that share one KV head are one contiguous row-major matrix; row `x`
 // belongs to position x / rep. out has that layout too, or [batch, seq, kv_heads, rep, head_dim] where the program only reads
-// it transposed so (a launch of its own before: 26 us for 4 x 2048 positions of 32 heads, 4 us for 517). Scores and probabilities never leave the SM.
+// it transposed so (a launch of its own before: 26 us for 4 x 2048 positions of 32 heads, 4 us for 517). Scores and
+// probabilities never leave the SM.
 //
 // A CTA owns TILES (1 or 2) tiles of 128 query rows and walks the keys 0..(its last position) in blocks of 128:
 //   copy warp      q once, then K and V blocks into a ring of shared-memory slots (tiled tensor-map copies, 128-byte
@@ -27,8 +28,8 @@
 //
 // What bounds it: per block and tile 1024 cycles of tensor core and 1024 cycles of exponentials (128 x 128 at 16 per
 // cycle), which overlap between the two tiles. Measured for 4 x 2048 positions, 32 query heads of 128 over 8 KV heads: the
-// warp-level kernel before this one (mma.sync, 64 rows per CTA) 627 us, this one 256 us inside a full-depth prefill and 201 us
-// alone at full clock; 1 x 517 positions 24 and 14 us.
+// warp-level kernel before this one (mma.sync, 64 rows per CTA) 627 us, this one 260 us inside a full-depth prefill (the
+// transposed store included) and 204 us alone; 1 x 517 positions 24 and 13.5 us.
 // Two tiles per CTA (320 threads) get 168 registers and spill 56 to 60 bytes, one tile of 64 elements a row with two CTAs per
 // SM the same and 68 bytes; one of 128 has 180 and none. Reading the scores
 // twice in 32-column chunks to hold fewer of them was slower (248 / 275 us).

@@ -12,15 +12,12 @@
 // r's mbarrier, and sums what it received itself in rank order (run-to-run identical results). Nothing goes through
 // global memory and no CTA waits for another cluster. The host chooses m_tile and ksplit with a model of the HBM time,
 // the per-SM rate and the number of waves (umma_choose in dot.cu).
-// This replaced equal shares of 64-deep units per CTA with f32 partials in global memory and a fold by the CTA that
-// arrived last: there every launch paid its HBM time plus 14 to 21 us, 7 us of them the tail (partials out, arrival
-// counter, two dependent rounds of loads through one SM). What is left at the decode sizes is the launch itself (set-up,
-// first copies, sum, exit: 7 to 9 us) and, above it, HBM.
+// What bounds it at the decode sizes is the launch itself (set-up, first copies, sum, exit: 7 to 9 us) and, above it, HBM.
 //
-// Who issues: the copy warp and the MMA warp run their loops converged and let one elected thread issue (elect_one). With a
-// single thread in those loops every operand of an issued instruction went through a vector register: the MMA lane
-// needed 1380 cycles per 128-deep unit beside busy converters, of which the products take 370, and 570 per 64-deep unit
-// without them. Launches one after the other, us, before and now: 32 rows bf16 4096 x 4096 16.5 / 14.8, 4096 x 6144 18.6 /
+// Who issues: the copy warp and the MMA warp run their loops converged and let one elected thread issue (elect_one; the copy
+// warp of kLoose is the exception). With a single thread in those loops every operand of an issued instruction went through
+// a vector register: the MMA lane needed 1380 cycles per 128-deep unit beside busy converters, of which the products take 370,
+// and 570 per 64-deep unit without them. Launches one after the other, us, before and now: 32 rows bf16 4096 x 4096 16.5 / 14.8, 4096 x 6144 18.6 /
 // 16.9, 14336 x 4096 30.2 / 27.4, 2048 x 14336 20.5 / 18.5, 7168 x 2048 16.8 / 14.7, 4096 x 28672 43.3 / 42.8 (HBM).
 //
 // Roles of a CTA:
@@ -52,7 +49,7 @@
 //            (widen_byte_pair). 16 rows, us, before these and the issue above, and now: 4096 x 28672 40.9 / 33.3, 14336 x
 //            4096 30.8 / 26.1, 8192 x 57344 114 / 94.5, 4096 x 128256 119.5 / 102 (5.2 TB/s).
 //   kLoose   16-bit weights of any pitch and alignment (an odd vocabulary, say): converter warps read them with plain
-//            loads, one column per thread, and write them to TMEM, at 1.6 TB/s: the converters' ALU is 65 % busy and waits for
+//            loads, one column per thread, and write them to TMEM, at 1.7 TB/s: the converters' ALU is 65 % busy and waits for
 //            2-byte loads. Few rows of large weights go by residues instead (umma_shift.cuh).
 //
 // Programmatic dependent launch: weights are never written by earlier work of the stream (`early_rhs`), so their
@@ -172,7 +169,7 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity, const 
     }
   }
 }
-// x = innermost coordinate (always a multiple of 64 elements here, i.e. 128 bytes), y = outer coordinate.
+// x = innermost coordinate (a multiple of 64 elements here, of 8 in umma_shift.cuh: 16 bytes), y = outer coordinate.
 __device__ __forceinline__ void tma_load_2d(uint32_t smem_dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
   asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
                    smem_dst),
@@ -820,7 +817,7 @@ __global__ void __launch_bounds__(threads_of(SRC), SRC == kLoose ? 1 : 2) umma_s
             if (c0 + j < m_rows) store(c0 + j, __uint_as_float(r[j]));
         }
       }
-      // The accumulator is in registers / memory now: hand it back to the MMA lane.
+      // The accumulator is in registers / memory now: hand it back to the MMA warp.
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
       if (lane == 0) mbar_arrive(&acc_empty[buf]);

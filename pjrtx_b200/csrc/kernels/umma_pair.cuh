@@ -18,12 +18,10 @@
 // chip form a compact block and share both operands through L2.
 //
 // Both warps run converged and let an elected thread issue (elect_one in umma_gemm.cuh); by a single thread a 64-deep unit took
-// 300 ns and 0.5 ns per row, now 195 and 0.57: 517 rows, us, before and now, 14336 x 4096 85 / 71.5, 4096 x 28672 120 / 109, 4096 x
-// 4096 35.5 / 31; 2048 rows, 4096 x 28672 332 / 315 (1527 TFLOP/s).
-//
-// Measured before that, 8192 rows, bf16, one SM per tile and pairs: 4096 x 28672 2030 / 1340 us (1433 TFLOP/s), 14336 x 4096 880 / 648 us,
-// 4096 x 6144 429 / 310 us, 4096 x 4096 291 / 211 us. Inside a full-depth prefill, under the power cap and with the launch
-// ordered after its predecessor: 1382, 675, 325 and 220 us.
+// 300 ns and 0.5 ns per row, now 195 and 0.57. Measured, bf16, us, one SM per tile, pairs issued by a single thread, pairs now:
+// 517 rows, 14336 x 4096 - / 85 / 71.5, 4096 x 28672 - / 120 / 109, 4096 x 4096 40 / 35.5 / 31; 2048 rows, 4096 x 28672 - / 332 / 315
+// (1527 TFLOP/s); 8192 rows inside a full-depth prefill, under the power cap and ordered after the predecessor, 4096 x 28672 2030 /
+// 1382 / 1307, 14336 x 4096 880 / 675 / 662, 4096 x 6144 429 / 325 / 311, 4096 x 4096 291 / 220 / 212 (the first of each four alone).
 //
 // No copy is multicast. Waits are bounded by time as in umma_gemm.cuh. The launch is ordered after its predecessor; its
 // dependents are released after the tensor-memory allocation.
