@@ -1295,8 +1295,8 @@ AttnDecodePlan attn_decode_plan(const AttnDecodeShape& s, int sm_count) {
       return p;
     }
   }
-  // The tensor-core kernel wherever it applies but for one case below: since its rows come by tiled copies and its splits merge cooperatively it
-  // is ahead at every size measured (8B shape, batch 1: 3.28 against 3.35 ms per step with 2.1 K keys, 3.36 against
+  // The tensor-core kernel wherever it applies but for one case below: since its rows come by tiled copies and its splits
+  // merge cooperatively it is ahead at every other size measured (8B shape, batch 1: 3.28 against 3.35 ms per step with 2.1 K keys, 3.36 against
   // 3.48 ms with 2.7 K; batch 2: 3.75 against 3.93 ms).
   // One query head per KV head over a second stage of keys that is not full (65 to 128) is as long on the CUDA cores, and with
   // more pairs than fit once shorter there, us: 24 sequences of 8 KV heads, 128 keys 8.28 / 9.15, 32 of 80 keys 8.2 / 9.5, of 96
